@@ -17,7 +17,9 @@
  *     only scratch is per group.
  * Groups are whole nodes (the initial table is node-contiguous) or the whole
  * population.  Everything is HBM-light integer work: the passes are bound by
- * Philox arithmetic (about 140 integer instructions per key).
+ * Philox arithmetic (about 140 integer instructions per key).  The timers
+ * and the heterogeneity, whose definitions are FP64, have FP32 forms with
+ * the same bits (lpg_init_fast.cuh).
  */
 #include <cuda_runtime.h>
 
@@ -28,6 +30,7 @@
 
 #include "lpg.h"
 #include "lpg_init.h"
+#include "lpg_init_fast.cuh"
 
 int lpg_ops_fail(int code, const char* fmt, ...);
 
@@ -324,6 +327,77 @@ int select_k(Scratch& sc, cudaStream_t st, const lpg_columns& c, uint64_t seed, 
   return 0;
 }
 
+/* Timers and heterogeneity by the FP32 kernels where the parameters have an
+ * FP32 form (lpg_init_fast.cuh); the parts done are taken out of *parts.
+ * The line is the form's own range: a lognormal that hardly varies would
+ * put every draw beside the same whole day or FP32 step, all of them unsure
+ * (2e7 slots at sigma 0: 26 ms against 22 in FP64 alone).  Small tables
+ * take it too (16385 slots: 0.34 ms against 0.81). */
+int fill_fast(Scratch& sc, cudaStream_t st, const lpg_init_desc& d, const SlotArgs& A, const lpg_columns& c,
+              uint32_t* parts) {
+  if (d.capacity <= 0) return 0;
+  FiExact X{};
+  X.seed = d.seed;
+  X.capacity = d.capacity;
+  X.c = c;
+  const int grid = grid_for(d.capacity, FI_TILE), fix_grid = grid_for(d.capacity, FI_FIX_TILE);
+  if (*parts & LPG_INIT_TIMERS) {
+    const lpg_dist dist[3] = {d.dur_exp, d.dur_inf, d.t_to_paralysis};
+    FiTimers F{};
+    bool ok = true;
+    int rc = 0;
+    for (int b = 0; b < 3 && ok; ++b) {
+      std::vector<uint64_t> thr;
+      ok = fi_dist_of(dist[b], &F.d[b], &thr);
+      if (ok && !thr.empty()) {
+        uint64_t* p;
+        if ((rc = sc.upload(&p, thr))) return rc;
+        F.d[b].n_thr = (int32_t)thr.size();
+        F.d[b].thr = p;
+      }
+    }
+    if (ok) {
+      F.seed = d.seed;
+      F.capacity = d.capacity;
+      F.et = c.exposure_timer;
+      F.it = c.infection_timer;
+      F.pt = c.paralysis_timer;
+      k_init_timers_fast<<<grid, FI_THREADS, 0, st>>>(F);
+      X.k_exp = A.k_exp;
+      X.k_inf = A.k_inf;
+      X.k_par = A.k_par;
+      X.e1 = A.e1;
+      X.e2 = A.e2;
+      X.i1 = A.i1;
+      X.i2 = A.i2;
+      X.p1 = A.p1;
+      X.p2 = A.p2;
+      k_init_fix<false><<<fix_grid, FI_THREADS, 0, st>>>(X);
+      CKI(cudaGetLastError());
+      *parts &= ~(uint32_t)LPG_INIT_TIMERS;
+    }
+  }
+  if ((*parts & LPG_INIT_HETEROGENEITY) && A.het && A.sigma > 0.01 && A.sigma < 4.0 && A.scale < 1e6) {
+    static const FiTables* host = fi_tables(); /* constants, formed once */
+    FiTables* tab;
+    int rc = sc.alloc(&tab, 1);
+    if (rc) return rc;
+    CKI(cudaMemcpyAsync(tab, host, sizeof(FiTables), cudaMemcpyHostToDevice, st));
+    FiHet H{d.seed, d.capacity, fi_pair(A.mu), fi_pair(A.sigma), fi_pair(A.rho), fi_pair(A.srho), fi_pair(A.scale),
+            tab, c.acq_risk_multiplier, c.daily_infectivity};
+    k_init_het_fast<<<grid, FI_THREADS, 0, st>>>(H);
+    X.mu = A.mu;
+    X.sigma = A.sigma;
+    X.rho = A.rho;
+    X.srho = A.srho;
+    X.scale = A.scale;
+    k_init_fix<true><<<fix_grid, FI_THREADS, 0, st>>>(X);
+    CKI(cudaGetLastError());
+    *parts &= ~(uint32_t)LPG_INIT_HETEROGENEITY;
+  }
+  return 0;
+}
+
 }  // namespace
 
 extern "C" double lpg_init_mean_infectivity(uint64_t seed, double r0, lpg_dist dur_inf) {
@@ -429,8 +503,9 @@ extern "C" int lpg_init_columns(const lpg_init_desc* d, uint32_t parts, const lp
     A.km_len = d->km_len;
     A.km_max_year = d->km_max_year;
   }
-  const uint32_t slot_parts =
+  uint32_t slot_parts =
       parts & (LPG_INIT_BASE | LPG_INIT_TIMERS | LPG_INIT_HETEROGENEITY | LPG_INIT_AGES | LPG_INIT_DEATHS | LPG_INIT_RI);
+  if ((rc = fill_fast(sc, st, *d, A, c, &slot_parts))) return rc;
   if (slot_parts && d->capacity > 0) {
     k_init_slots<<<grid_for(d->capacity, kThreads * 8), kThreads, 0, st>>>(A, c, slot_parts);
     CKI(cudaGetLastError());
