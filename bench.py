@@ -1057,19 +1057,20 @@ def incidence_arm(args):
     tot = sum(ms for ms, _ in prof.values())
     kernels = {name: {"launches": n, "ms_per_eval": ms / K, "share": ms / tot if tot else None}
                for name, (ms, n) in prof.items()}
-    # the products run in double-float on the FP32 pipe: 12 FP32 instructions per term
-    # (Dekker product by FMA, two cross terms, Knuth TwoSum), T S G G terms per launch
+    # the products run by exact slicing on the tensor cores: 43 products of bf16 digit slices
+    # (diagonals 0 to 8 of eight slices each), T S G G terms a product and launch
     terms = float(T * S * G * G)
     top = max(prof, key=lambda n: prof[n][0])
     gemm = max(("k_inc_gemm_mix", "k_inc_gemm_flows"), key=lambda n: prof[n][0])
     ms_g = prof[gemm][0] / max(1, prof[gemm][1])
-    fp32_peak = 152 * 128 * 2.07e9 / 1e12  # lane-instructions/s at the maximum SM clock (nominal)
-    ach = 12.0 * terms / (ms_g / 1e3) / 1e12
-    roof = {"kernel": gemm, "top_kernel": top, "bound": "fp32", "achieved": ach, "peak": fp32_peak,
-            "unit": "T FP32 lane-instructions/s", "frac": ach / fp32_peak,
-            "peak_kind": "nominal GB300 FP32 issue rate, 152 SMs x 128 lanes x 2.07 GHz (not measured)",
-            "fp64_equivalent_tflops": 2.0 * terms / (ms_g / 1e3) / 1e12, "traffic": None,
-            "instructions_per_launch": 12.0 * terms}
+    flops = 43 * 2.0 * terms
+    ach = flops / (ms_g / 1e3) / 1e12
+    peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
+    bf16 = float(peaks.get("bf16_tflops", 1900.0))
+    roof = {"kernel": gemm, "top_kernel": top, "bound": "bf16 tensor", "achieved": ach, "peak": bf16,
+            "unit": "TFLOP/s of bf16 digit products", "frac": ach / bf16,
+            "peak_source": "measured" if "bf16_tflops" in peaks else "fallback",
+            "fp64_equivalent_tflops": 2.0 * terms / (ms_g / 1e3) / 1e12, "traffic": None, "flops_per_launch": flops}
     h2d_setup = sum(inp[k].nbytes for k in ("srisk", "beta", "pop", "doy", "year", "pops", "dist")) + target.nbytes
     cpu = None
     if not args.no_cpu:
@@ -1103,7 +1104,7 @@ def incidence_arm(args):
         "e2e": {"value": K / (t_setup + t_eval), "unit": "evaluations/s", "setup_ms": t_setup * 1e3,
                 "ms_per_eval": t_eval / K * 1e3, "h2d_bytes_per_step": h2d_setup / K + 8 * G,
                 "d2h_bytes_per_step": 8 * (8 + G)},
-        "gpu_launches": 7 * K,  # per evaluation: network, mix, forward, backward + seasonal, flows, network_grad
+        "gpu_launches": 8 * K,  # per evaluation: network, column maxima, slicing, mix, step, slicing, flows, network_grad
         "kernels": kernels,
         "roofline": roof,
         "cpu_baseline": cpu,

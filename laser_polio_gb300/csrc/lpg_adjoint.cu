@@ -22,23 +22,22 @@
  * curve the plan also forms the calibration loss
  * L = sum (log1p(lam) - log1p(target))^2 and its dL/dlam on the device.
  *
- * Layout in HBM: a plan keeps the aggregates resident — srisk, pop [T][G];
- * beta as [T][S][G] (strain-major per tick, so that the (t, s) rows of the
- * mixing product and every elementwise pass read G consecutive doubles);
- * u, exp(-r) and dL/du the same way; log(dist) and the network and its
- * gradients [G][G]; log(pops) [G].
+ * Layout in HBM: a plan keeps the aggregates resident — srisk and
+ * 1/max(pop, 1) [T][G]; beta as [T][S][G] (strain-major per tick, so that the
+ * (t, s) rows of the mixing product and every elementwise pass read G
+ * consecutive doubles); u and dL/du the same way; log(dist), log2(dist) and
+ * the flows and their gradients [G][G]; log(pops) [G].
  *
- * Arithmetic: double precision throughout, except inside the two
- * contractions, u = beta N per (t, s) row and dL/dN = beta^T dL/du, both
- * (T S) x G x G.  GB300 issues about two FP64 FMAs per clock per SM and 128
- * FP32 FMAs, so the products run in double-float: their operands are held
- * as FP32 pairs hi + lo (beta split once per plan, N and dL/du by the
- * kernels that produce them), each term hi*hi is formed exactly (Dekker's
- * product via FMA) with the cross terms, and the running sum is an FP32
- * pair kept by Knuth's TwoSum — about 2^-44 relative per dot product,
- * twelve FP32 operations per term and no FP64 work inside the products.
- * The FP32 pair cannot hold magnitudes below 2^-126, so products of
- * operands under about 1e-19 each lose relative (not absolute) accuracy.
+ * Arithmetic: double precision throughout, most of it without the FP64 unit.
+ * GB300 issues about two FP64 FMAs per clock per SM, 128 FP32 or integer
+ * operations, and 8192 bf16 tensor FMAs.
+ *   - The two contractions, u = beta N per (t, s) row and dL/dN = beta^T
+ *     dL/du, both (T S) x G x G, run on the tensor cores by exact slicing
+ *     (lpg_ozaki.cuh).  beta's slices are formed once per plan, N's and
+ *     dL/du's each evaluation.
+ *   - Contractions too small for that are summed in FP64 where their results
+ *     are used, with no launch of their own.
+ *   - exp and log1p run in 64-bit integer arithmetic (lpg_ixmath.cuh).
  * The sums use atomics, so results agree with a sequential FP64 evaluation
  * to rounding, not bit for bit.
  */
@@ -48,6 +47,8 @@
 #include <vector>
 
 #include "lpg.h"
+#include "lpg_ixmath.cuh"
+#include "lpg_ozaki.cuh"
 
 /* Per-host-thread error text of the standalone ops (lpg_ops.cu). */
 int lpg_ops_fail(int code, const char* fmt, ...);
@@ -56,11 +57,10 @@ namespace {
 
 constexpr double kTwoPi = 6.283185307179586476925286766559;
 #define INC_THREADS 256
-#define DF_BM 32      /* product tile rows */
-#define DF_BN 64      /* product tile columns */
-#define DF_BK 32      /* product tile depth */
-#define DF_THREADS 128 /* 4 x 4 outputs per thread */
-#define DF_MAX_SPLIT 8 /* depth slices of the flows product */
+#define INC_MAX_SPLIT 8 /* depth slices of a sliced product */
+#define INC_MAX_ROWS (65535 * 32)
+#define INC_SMALL_NODES 128
+#define INC_SMALL_TERMS 4000000 /* T S G^2 */
 
 enum { PH_NETWORK, PH_MIX, PH_FORWARD, PH_BACKWARD, PH_FLOWS, PH_NETWORK_GRAD, PH_COUNT };
 const char* const kPhaseNames[PH_COUNT] = {"k_inc_network", "k_inc_gemm_mix", "k_inc_forward",
@@ -70,309 +70,387 @@ struct IncScalars {
   double R, amp, peak;
 };
 
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+/* The sum over the CTA (whole warps, at most 32), in every thread.  An FP64
+ * addition holds the pipe for 16 cycles a warp, so only the first warp adds
+ * the warps' sums. */
 __device__ __forceinline__ double block_sum(double v, double* s_part) {
-  s_part[threadIdx.x] = v;
+  const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  v = warp_sum(v);
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) s_part[threadIdx.x] += s_part[threadIdx.x + o];
-    __syncthreads();
+  if (lane == 0) s_part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double r = lane < warps ? s_part[lane] : 0.0;
+    for (int o = 1; o < warps; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (lane == 0) s_part[0] = r;
   }
-  const double r = s_part[0];
   __syncthreads();
-  return r;
+  return s_part[0];
 }
 
-/* An FP64 value as an FP32 pair hi + lo. */
-__device__ __forceinline__ float2 df_split(double x) {
-  const float hi = __double2float_rn(x);
-  return make_float2(hi, __double2float_rn(x - (double)hi));
+#define INC_LOG2_NONE INT64_MIN /* log2 of 0 or infinity */
+
+/* log2 x with 52 fraction bits. */
+__device__ __forceinline__ int64_t inc_log2(double x) {
+  if (!(x > 0.0) || isinf(x)) return INC_LOG2_NONE;
+  int e;
+  const double m = frexp(x, &e); /* [1/2, 1): log2 m to 2^-53 absolute */
+  return ((int64_t)e << 52) + __double2ll_rn(log2(m) * 0x1p52);
 }
 
-__global__ void __launch_bounds__(INC_THREADS) k_inc_split(size_t n, const double* x, float2* y) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < n) y[idx] = df_split(x[idx]);
-}
-
-/* log(pops) [G] and log(dist) [G][G] (the diagonal is never read), once
- * per plan.  Zero gives -inf. */
+/* log(pops), log2(pops) [G]; log(dist), log2(dist) [G][G] (the diagonal is
+ * never read); 1/max(pop, 1) and log1p(target) [T][G]: once per plan. */
 __global__ void __launch_bounds__(INC_THREADS)
-    k_inc_logs(int G, const double* pops, const double* dist, double* logp, double* logd) {
+    k_inc_logs(int G, size_t TG, const double* pops, const double* dist, double* logp, double* logd, int64_t* lp2,
+               int64_t* ld2, const double* pop, double* rpop, double* target) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < (size_t)G * G) logd[idx] = log(dist[idx]);
-  if (idx < (size_t)G) logp[idx] = log(pops[idx]);
+  if (idx < (size_t)G * G) {
+    logd[idx] = log(dist[idx]);
+    ld2[idx] = inc_log2(dist[idx]);
+  }
+  if (idx < (size_t)G) {
+    logp[idx] = log(pops[idx]);
+    lp2[idx] = inc_log2(pops[idx]);
+  }
+  if (idx < TG) {
+    rpop[idx] = 1.0 / fmax(pop[idx], 1.0);
+    if (target) target[idx] = log1p(target[idx]);
+  }
+}
+
+/* a c 2^-56, rounded: a with 52 fraction bits times c with 56. */
+__device__ __forceinline__ int64_t inc_mul56(int64_t a, int64_t c) {
+  const int64_t hi = __mul64hi(a, c);
+  const uint64_t lo = (uint64_t)a * (uint64_t)c;
+  return (int64_t)((uint64_t)hi << 8 | lo >> 56) + (int64_t)(lo >> 55 & 1);
+}
+
+/* The gravity parameters of an evaluation: kP = k / P^c; a, b, c also with
+ * 56 fraction bits.  integer: every exponent stays within the fixed-point
+ * range (the host's check), so that the flows are formed in integers. */
+struct IncGravity {
+  double a, b, c, kP, max_frac;
+  int64_t a56, b56, c56;
+  int integer;
+};
+
+/* kP p^a */
+__device__ __forceinline__ double inc_row_scale(const IxTables* T, const IncGravity& V, double p, int64_t l2) {
+  if (!V.integer || (l2 == INC_LOG2_NONE && V.a != 0.0)) return V.kP * pow(p, V.a);
+  if (V.a == 0.0) return V.kP;
+  const int64_t E = inc_mul56(l2, V.a56);
+  return V.kP * ix_double(ix_exp2_frac(T, (uint64_t)E << 12), (int)(E >> 52));
 }
 
 /* Blocks [0, G): one network row i each — the scaled gravity flows
  * G[i,j] = k p_i^a p_j^b / d_ij^c / P^c (zero diagonal; non-finite
- * values are 0), formed as k p_i^a exp(b log p_j - c log d_ij) / P^c with
- * the 0^0 = 1 convention kept, their sum rs[i], and the normalised row
- * N[i,j] (scaled down to max_frac when rs[i] exceeds it; stored as FP32
- * pairs for the mixing product) with its FP64 sum.
- * Blocks [G, G + ceil(T/256)): the seasonal factor of each tick and its
- * derivatives with respect to amp and peak. */
+ * values are 0), formed as k p_i^a 2^(b log2 p_j - c log2 d_ij) / P^c with
+ * the 0^0 = 1 convention kept, their sum rs[i], the factor fac[i] that scales
+ * the row down to max_frac when rs[i] exceeds it (else 1), and the normalised
+ * row's sum; for the small sums also the normalised row N[i,j].
+ * Blocks [G, G + ceil(T/32)): the seasonal factor of each tick and its
+ * derivatives with respect to amp and peak.
+ * Bound by integer issue (about 110 instructions an element, one FP64
+ * addition); with the FP64 library's pow and exp 774 nodes took 94 us. */
+template <bool SMALL>
 __global__ void __launch_bounds__(INC_THREADS)
-    k_inc_network(int G, int T, const double* pops, const double* logp, const double* logd, double k, double a,
-                  double b, double c, double Pc, double max_frac, double* Gm, float2* N, double* rs, double* rsN,
-                  int* capped, const double* doy, const double* year, IncScalars sc, double* seas) {
-  __shared__ double s_part[INC_THREADS];
+    k_inc_network(int G, int T, const IxTables* __restrict__ tab, const double* pops, const double* logp,
+                  const double* logd, const int64_t* lp2, const int64_t* __restrict__ ld2, IncGravity V, double* Gm,
+                  double* N, double* rs, double* rsN, double* fac, const double* doy, const double* year,
+                  IncScalars sc, double* seas) {
+  __shared__ double s_part[INC_THREADS / 32], s_kpa;
   if ((int)blockIdx.x >= G) {
-    const int t = (blockIdx.x - G) * INC_THREADS + threadIdx.x;
-    if (t < T) {
+    /* a warp a block: the FP64 sine, cosine and divisions of 256 ticks on one SM would outlast the rows */
+    const int t = (blockIdx.x - G) * 32 + threadIdx.x;
+    if (threadIdx.x < 32 && t < T) {
       const double ang = kTwoPi * (doy[t] - sc.peak) / year[t];
-      const double ca = cos(ang);
+      double sa, ca;
+      sincos(ang, &sa, &ca);
       seas[t] = 1.0 + sc.amp * ca;
-      seas[T + t] = ca;                                      /* d seas / d amp */
-      seas[2 * T + t] = sc.amp * sin(ang) * kTwoPi / year[t]; /* d seas / d peak */
+      seas[T + t] = ca;                                 /* d seas / d amp */
+      seas[2 * T + t] = sc.amp * sa * kTwoPi / year[t]; /* d seas / d peak */
     }
     return;
   }
   const int i = blockIdx.x;
-  const double kpa = k * pow(pops[i], a) / Pc;
+  if (threadIdx.x == 0) s_kpa = inc_row_scale(tab, V, pops[i], lp2[i]);
+  __syncthreads();
+  const double kpa = s_kpa;
+  const uint64_t kb = (uint64_t)__double_as_longlong(kpa);
+  const int kx = (int)(kb >> 52 & 0x7ff);
+  const uint64_t km = ((kb & 0xfffffffffffffULL) | 1ULL << 52) << 11;
+  const bool integer = V.integer && kx > 0 && kx < 0x7ff;
   double sum = 0.0;
   for (int j = threadIdx.x; j < G; j += blockDim.x) {
     double v = 0.0;
     if (j != i) {
-      const double x = (b == 0.0 ? 0.0 : b * logp[j]) - (c == 0.0 ? 0.0 : c * logd[(size_t)i * G + j]);
-      v = kpa * exp(x);
-      if (!isfinite(v)) v = 0.0;
+      if (integer) {
+        const int64_t l = lp2[j], d = ld2[(size_t)i * G + j];
+        if ((l != INC_LOG2_NONE || V.b == 0.0) && (d != INC_LOG2_NONE || V.c == 0.0)) {
+          const int64_t E = (V.b == 0.0 ? 0 : inc_mul56(l, V.b56)) - (V.c == 0.0 ? 0 : inc_mul56(d, V.c56));
+          uint64_t m = __umul64hi(ix_exp2_frac(tab, (uint64_t)E << 12), km);
+          int n = (int)(E >> 52) + kx - 1022;
+          if (!(m >> 63)) {
+            m <<= 1;
+            n -= 1;
+          }
+          if (n >= -1022 && n <= 1022) v = __longlong_as_double(__double_as_longlong(ix_double(m, n)) | (long long)(kb & 1ULL << 63));
+        }
+      } else {
+        const double x = (V.b == 0.0 ? 0.0 : V.b * logp[j]) - (V.c == 0.0 ? 0.0 : V.c * logd[(size_t)i * G + j]);
+        v = kpa * exp(x);
+        if (!isfinite(v)) v = 0.0;
+      }
     }
     Gm[(size_t)i * G + j] = v;
     sum += v;
   }
   const double r = block_sum(sum, s_part);
-  const bool cap = r > max_frac;
-  double sumN = 0.0;
-  for (int j = threadIdx.x; j < G; j += blockDim.x) {
-    const double v = Gm[(size_t)i * G + j]; /* written by this thread above */
-    const double nv = cap ? v * (max_frac / r) : v;
-    N[(size_t)i * G + j] = df_split(nv);
-    sumN += nv;
+  const bool cap = r > V.max_frac;
+  const double f = cap ? V.max_frac / r : 1.0;
+  double rn = r;
+  if (SMALL || cap) {
+    double sumN = 0.0;
+    for (int j = threadIdx.x; j < G; j += blockDim.x) {
+      const double v = Gm[(size_t)i * G + j]; /* written by this thread above */
+      const double nv = cap ? v * f : v;
+      if (SMALL) N[(size_t)i * G + j] = nv;
+      sumN += nv;
+    }
+    rn = block_sum(sumN, s_part);
   }
-  const double rn = block_sum(sumN, s_part);
   if (threadIdx.x == 0) {
     rs[i] = r;
     rsN[i] = rn;
-    capped[i] = cap ? 1 : 0;
+    fac[i] = f;
   }
 }
 
-/* (sh, sl) += a * b for FP32 pairs a, b: the exact product of the high
- * parts (Dekker, by FMA) plus the cross terms, added by Knuth's TwoSum.
- * The _rn intrinsics are never contracted or reassociated. */
-__device__ __forceinline__ void df_fma(float& sh, float& sl, float2 a, float2 b) {
-  const float ph = __fmul_rn(a.x, b.x);
-  float pl = __fmaf_rn(a.x, b.x, -ph);
-  pl = __fmaf_rn(a.x, b.y, pl);
-  pl = __fmaf_rn(a.y, b.x, pl);
-  const float s = __fadd_rn(sh, ph);
-  const float bp = __fsub_rn(s, sh);
-  const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bp)), __fsub_rn(ph, bp));
-  sl = __fadd_rn(sl, __fadd_rn(err, pl));
-  sh = s;
+__device__ __forceinline__ double inc_exp_neg(const IxTables* tab, double x) {
+  return ix_below(x, 700.0) ? ix_exp_neg(tab, x) : exp(-x);
 }
 
-/* C_z[M][N] = sum over k in slice z of A(m, k) B[k][n], row-major, in
- * double-float, A and B given as FP32 pairs.  A(m, k) = A[m][k] (M x K) or, with TRANS_A, A[k][m]
- * (K x M).  blockIdx.z picks the depth slice [z kchunk, (z+1) kchunk) and
- * the output C + z M N.  32 x 64 tiles, 128 threads with 4 x 4 outputs
- * each (rows ty + 8i, columns tx + 16j). */
-template <bool TRANS_A>
-__global__ void __launch_bounds__(DF_THREADS)
-    k_inc_gemm(int M, int N, int K, int kchunk, const float2* __restrict__ A, const float2* __restrict__ B,
-               double* C) {
-  __shared__ float2 sA[DF_BK][DF_BM + 1]; /* [k][m] */
-  __shared__ float2 sB[DF_BK][DF_BN];     /* [k][n] */
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * DF_BM, n0 = blockIdx.x * DF_BN;
-  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  float sh[4][4], sl[4][4];
+__device__ __forceinline__ double inc_log1p(const IxTables* tab, double y) {
+  return ix_below(y, 0x1p60) && !ix_below(y, 0x1p-5) ? ix_log1p(tab, y) : log1p(y);
+}
+
+/* 1/d for d >= 1, to within an ulp: the hardware estimate, two Newton steps. */
+__device__ __forceinline__ double inc_recip(double d) {
+  if (!ix_below(d, 1e300) || ix_below(d, 1.0)) return 1.0 / d;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+  return __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+}
+
+struct IncStep {
+  int T, G, S, split; /* split: depth slices of the mixing product */
+  const double *srisk, *beta, *rpop, *seas, *r0s, *rsN, *ltarget, *g_in;
+  const double* u; /* the mixing product's slabs, or */
+  const double* N; /* the normalised network (small sums) */
+  double R;
+  double *lam, *loss; /* lam may be null */
+  double* gu; /* dL/du */
+  unsigned long long* max_gu;
+  double *g_r0s, *g_w;
+  int grad;
+};
+
+/* TC ticks of one node a thread: the mixing's diagonal term, the rates,
+ * lam, with a target the loss term and dL/dlam, and with grad the reverse
+ * pass of the same cells: dL/du, its column maxima, the r0s gradient, and
+ * w[t] = sum_n dL/dq / popc r0s, from which the last kernel forms the
+ * gradients of R, amp and peak.  Forward and reverse share the rates and
+ * exponentials in registers (they were two kernels and 2 T S G doubles
+ * between them).  Bound by FP64 issue: about 32 operations a cell, the
+ * exponentials and logarithms in integers (774 nodes, 365 ticks, 3 strains:
+ * 185 us before). */
+template <bool SMALL, int TC>
+__global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables* __restrict__ tab, IncStep A) {
+  __shared__ double s_loss[4];
+  const int n = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * TC, lane = threadIdx.x & 31;
+  const int T = A.T, G = A.G, S = A.S;
+  const size_t slab = (size_t)T * S * G;
+  const bool in = n < G;
+  const double keep = in ? 1.0 - A.rsN[n] : 0.0, r0 = in ? A.r0s[n] : 0.0;
+  double loss = 0.0, acc_r0 = 0.0;
+  unsigned long long mx = 0;
+  double w[TC];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TC; ++i) {
+    w[i] = 0.0;
+    const int t = t0 + i;
+    if (!in || t >= T) continue;
+    const size_t idx = (size_t)t * G + n;
+    const double st = A.seas[t], ip = A.rpop[idx];
+    const double q = st * A.R * r0 * ip;
+    double uu[LPG_MAX_STRAINS], ex[LPG_MAX_STRAINS], l = 0.0, mix[LPG_MAX_STRAINS] = {0.0, 0.0, 0.0, 0.0};
+    if (SMALL) {
+      const double* b = A.beta + (size_t)t * S * G;
+#pragma unroll 8
+      for (int j = 0; j < G; ++j) {
+        const double m = A.N[(size_t)j * G + n];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sh[i][j] = sl[i][j] = 0.f;
-  for (int k0 = kb; k0 < ke; k0 += DF_BK) {
-#pragma unroll
-    for (int r = 0; r < (DF_BK * DF_BM) / DF_THREADS; ++r) {
-      const int e = tid + r * DF_THREADS;
-      const int hi = e >> 5, lo = e & 31;
-      float2 v = make_float2(0.f, 0.f);
-      if (TRANS_A) { /* hi = k, lo = m: consecutive threads read consecutive m */
-        if (k0 + hi < ke && m0 + lo < M) v = A[(size_t)(k0 + hi) * M + m0 + lo];
-        sA[hi][lo] = v;
-      } else { /* hi = m, lo = k: consecutive threads read consecutive k */
-        if (m0 + hi < M && k0 + lo < ke) v = A[(size_t)(m0 + hi) * K + k0 + lo];
-        sA[lo][hi] = v;
+        for (int s = 0; s < LPG_MAX_STRAINS; ++s)
+          if (s < S) mix[s] = __fma_rn(b[s * G + j], m, mix[s]);
       }
     }
 #pragma unroll
-    for (int r = 0; r < (DF_BK * DF_BN) / DF_THREADS; ++r) {
-      const int e = tid + r * DF_THREADS;
-      const int hi = e >> 6, lo = e & 63;
-      float2 v = make_float2(0.f, 0.f);
-      if (k0 + hi < ke && n0 + lo < N) v = B[(size_t)(k0 + hi) * N + n0 + lo];
-      sB[hi][lo] = v;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int q = 0; q < DF_BK; ++q) {
-      float2 av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = sA[q][ty + 8 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = sB[q][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) df_fma(sh[i][j], sl[i][j], av[i], bv[j]);
-    }
-    /* renormalise each pair (Fast2Sum: |sh| >= |sl|) so that sl stays small */
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float t = __fadd_rn(sh[i][j], sl[i][j]);
-        sl[i][j] = __fsub_rn(sl[i][j], __fsub_rn(t, sh[i][j]));
-        sh[i][j] = t;
-      }
-    __syncthreads();
-  }
-  double* Cz = C + (size_t)blockIdx.z * M * N;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = m0 + ty + 8 * i;
-    if (row >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = n0 + tx + 16 * j;
-      if (col < N) Cz[(size_t)row * N + col] = (double)sh[i][j] + (double)sl[i][j];
-    }
-  }
-}
-
-/* Per (t, n), one tick per blockIdx.y: the mixing's diagonal term, the
- * rates, exp(-r) kept for the reverse pass, lam, and with a target the
- * loss term and dL/dlam. */
-__global__ void __launch_bounds__(INC_THREADS)
-    k_inc_forward(int T, int G, int S, const double* srisk, const double* beta, const double* pop,
-                  const double* seas, const double* r0s, const double* rsN, IncScalars sc, double* u, double* e,
-                  double* lam, const double* target, double* g, double* loss) {
-  __shared__ double s_part[INC_THREADS];
-  const int t = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t idx = (size_t)t * G + n;
-  double part = 0.0;
-  if (n < G) {
-    const double q = seas[t] * r0s[n] * sc.R / fmax(pop[idx], 1.0);
-    double l = 0.0;
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < LPG_MAX_STRAINS; ++s) {
+      uu[s] = ex[s] = 0.0;
+      if (s >= S) continue;
       const size_t k = ((size_t)t * S + s) * G + n;
-      const double uu = u[k] + beta[k] * (1.0 - rsN[n]);
-      u[k] = uu;
-      const double ex = exp(-(uu * q));
-      e[k] = ex;
-      l += 1.0 - ex;
+      double m;
+      if (SMALL) {
+        m = mix[s];
+      } else {
+        m = A.u[k];
+        for (int z = 1; z < A.split; ++z) m += A.u[z * slab + k];
+      }
+      uu[s] = __fma_rn(A.beta[k], keep, m);
+      ex[s] = inc_exp_neg(tab, uu[s] * q);
+      l += 1.0 - ex[s];
     }
-    const double lv = srisk[idx] * l;
-    lam[idx] = lv;
-    if (target) {
-      const double r = log1p(lv) - log1p(target[idx]);
-      g[idx] = 2.0 * r / (1.0 + lv);
-      part = r * r;
+    const double sr = A.srisk[idx], lv = sr * l;
+    if (A.lam) A.lam[idx] = lv;
+    double g = 0.0;
+    if (A.ltarget) {
+      const double r = inc_log1p(tab, lv) - A.ltarget[idx];
+      g = 2.0 * r * inc_recip(1.0 + lv);
+      loss = __fma_rn(r, r, loss);
     }
-  }
-  if (target) { /* uniform over the grid */
-    const double tot = block_sum(part, s_part);
-    if (threadIdx.x == 0) atomicAdd(loss, tot);
-  }
-}
-
-/* Per (t, n) of the reverse pass, one tick per blockIdx.y: dL/du (as FP32
- * pairs for the dL/dN product) and the contributions to dL/dseas[t],
- * dL/dr0s[n] and dL/dR (block sums for the per-tick and scalar ones). */
-__global__ void __launch_bounds__(INC_THREADS)
-    k_inc_backward(int T, int G, int S, const double* g, const double* srisk, const double* pop, const double* seas,
-                   const double* r0s, IncScalars sc, const double* u, const double* e, float2* gu, double* g_seas,
-                   double* g_r0s, double* g_R) {
-  __shared__ double s_part[INC_THREADS];
-  const int t = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t idx = (size_t)t * G + n;
-  double cR = 0.0, cS = 0.0;
-  if (n < G) {
-    const double st = seas[t];
-    const double popc = fmax(pop[idx], 1.0);
-    const double q = st * r0s[n] * sc.R / popc;
-    const double gs = g[idx] * srisk[idx];
+    if (!A.grad) continue;
+    if (A.g_in) g = A.g_in[idx];
+    const double gs = g * sr;
     double gq = 0.0;
-    for (int s = 0; s < S; ++s) {
+#pragma unroll
+    for (int s = 0; s < LPG_MAX_STRAINS; ++s) {
+      if (s >= S) continue;
       const size_t k = ((size_t)t * S + s) * G + n;
-      const double gr = gs * e[k];
-      gu[k] = df_split(gr * q);
-      gq += gr * u[k];
+      const double gr = gs * ex[s], gu = gr * q;
+      A.gu[k] = gu;
+      const unsigned long long b = oz_abs_bits(gu);
+      mx = b > mx ? b : mx;
+      gq = __fma_rn(gr, uu[s], gq);
     }
-    cS = gq * r0s[n] * sc.R / popc;
-    atomicAdd(&g_r0s[n], gq * st * sc.R / popc);
-    cR = gq * st * r0s[n] / popc;
+    const double gp = gq * ip;
+    w[i] = gp * r0;
+    acc_r0 = __fma_rn(gp * st, A.R, acc_r0);
   }
-  const double tS = block_sum(cS, s_part);
-  const double tR = block_sum(cR, s_part);
-  if (threadIdx.x == 0) {
-    atomicAdd(&g_seas[t], tS);
-    atomicAdd(g_R, tR);
+  if (A.grad) {
+    if (in) {
+      atomicAdd(&A.g_r0s[n], acc_r0);
+      if (!SMALL) atomicMax(&A.max_gu[n], mx);
+    }
+#pragma unroll
+    for (int i = 0; i < TC; ++i) {
+      const double v = warp_sum(w[i]);
+      if (lane == 0 && t0 + i < T) atomicAdd(&A.g_w[t0 + i], v);
+    }
   }
-}
-
-/* dL/damp and dL/dpeak from dL/dseas[t] (one CTA). */
-__global__ void __launch_bounds__(INC_THREADS)
-    k_inc_seasonal(int T, const double* seas, const double* g_seas, double* out) {
-  __shared__ double s_part[INC_THREADS];
-  double ga = 0.0, gp = 0.0;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    ga += g_seas[t] * seas[T + t];
-    gp += g_seas[t] * seas[2 * T + t];
-  }
-  ga = block_sum(ga, s_part);
-  gp = block_sum(gp, s_part);
-  if (threadIdx.x == 0) {
-    out[0] = ga;
-    out[1] = gp;
+  if (A.ltarget) { /* uniform over the grid */
+    loss = warp_sum(loss);
+    if (lane == 0) s_loss[threadIdx.x >> 5] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(A.loss, (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]));
   }
 }
 
-/* One row a per CTA: C[a][b] = the sum of the flows product's nsplit
- * depth slices, dL/dN[a][b] = C[a][b] - C[a][a] (zero on the diagonal),
- * then dL/dG through the row normalisation and the row's contributions to
- * dL/dk, dL/da, dL/db, dL/dc. */
-__global__ void __launch_bounds__(INC_THREADS)
-    k_inc_network_grad(int G, int nsplit, const double* C, const double* Gm, const double* rs, const int* capped,
-                       const double* logp, const double* logd, double k, double logP, double max_frac, double* gN,
-                       double* g_theta) {
-  __shared__ double s_part[INC_THREADS];
-  const int a = blockIdx.x;
-  const size_t GG = (size_t)G * G, row = (size_t)a * G;
-  double diag = 0.0;
-  for (int z = 0; z < nsplit; ++z) diag += C[z * GG + row + a];
-  double cpl = 0.0; /* the row's sum of dL/dN * G (the normalisation's coupling term) */
-  for (int b = threadIdx.x; b < G; b += blockDim.x) {
-    double cab = 0.0;
-    for (int z = 0; z < nsplit; ++z) cab += C[z * GG + row + b];
-    const double v = b == a ? 0.0 : cab - diag;
-    gN[row + b] = v;
-    cpl += v * Gm[row + b];
+/* The last block: dL/dR, dL/damp and dL/dpeak from w[t].  The others take
+ * rows a in turn — C[a][b] = the sum of the flows product's nsplit depth
+ * slices, or with SMALL the sum over (t, s) formed here, dL/dN[a][b] = C[a][b] - C[a][a] (zero on the diagonal), then dL/dG
+ * through the row normalisation and the contributions to dL/dk, dL/da, dL/db,
+ * dL/dc, kept per thread over the CTA's rows; dL/dN is written when asked
+ * for.  Bound by FP64 issue: five operations an element and two a row and
+ * thread (4000 nodes: 616 us with a reduction and two passes a row). */
+template <bool SMALL>
+__global__ void __launch_bounds__(INC_THREADS, SMALL ? 2 : 5)
+    k_inc_network_grad(int G, int T, int TS, int nsplit, const double* C, const double* beta, const double* gu, const double* Gm, const double* rs,
+                       const double* fac, const double* logp, const double* logd, double k, double logP,
+                       double* gN, double* g_theta, const double* seas, const double* g_w, double R, double* g_seas) {
+  __shared__ double s_part[INC_THREADS / 32];
+  const int rows = gridDim.x - 1;
+  if ((int)blockIdx.x == rows) {
+    double gR = 0.0, ga = 0.0, gp = 0.0;
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+      gR = __fma_rn(g_w[t], seas[t], gR);
+      ga = __fma_rn(g_w[t] * R, seas[T + t], ga);
+      gp = __fma_rn(g_w[t] * R, seas[2 * T + t], gp);
+    }
+    gR = block_sum(gR, s_part);
+    ga = block_sum(ga, s_part);
+    gp = block_sum(gp, s_part);
+    if (threadIdx.x == 0) {
+      g_seas[0] = gR;
+      g_seas[1] = ga;
+      g_seas[2] = gp;
+    }
+    return;
   }
-  const double coupling = block_sum(cpl, s_part);
-  const bool cap = capped[a] != 0;
-  const double ra = rs[a];
-  const double lpa = logp[a];
+  extern __shared__ double s_flow[]; /* the small sums: partial rows [slices][G] */
+  const size_t GG = (size_t)G * G;
+  auto nonzero = [](double x) { return ((uint64_t)__double_as_longlong(x) << 1) != 0; };
   double wk = 0.0, wa = 0.0, wb = 0.0, wc = 0.0;
-  for (int b = threadIdx.x; b < G; b += blockDim.x) {
-    if (b == a) continue;
-    const double gn = gN[row + b]; /* written by this thread above */
-    const double gg = cap ? (max_frac / ra) * (gn - coupling / ra) : gn;
-    const double w = gg * Gm[row + b];
-    if (w == 0.0) continue; /* a zero flow: its logs may be infinite */
-    wk += w;
-    wa += w * lpa;
-    wb += w * logp[b];
-    wc += w * (-logd[row + b] - logP);
+  for (int a = blockIdx.x; a < G; a += rows) {
+    const size_t row = (size_t)a * G;
+    if (SMALL) {
+      /* row a of beta^T dL/du: the depth cut over groups of threads, one column a thread */
+      const int width = (G + 31) / 32 * 32 < INC_THREADS ? (G + 31) / 32 * 32 : INC_THREADS;
+      const int slices = INC_THREADS / width, sl = threadIdx.x / width;
+      const int per = (TS + slices - 1) / slices, k1 = min(TS, (sl + 1) * per);
+      if (sl < slices)
+        for (int b = threadIdx.x % width; b < G; b += width) {
+          double c = 0.0;
+#pragma unroll 8
+          for (int k = sl * per; k < k1; ++k) c = __fma_rn(beta[(size_t)k * G + a], gu[(size_t)k * G + b], c);
+          s_flow[sl * G + b] = c;
+        }
+      __syncthreads();
+      for (int b = threadIdx.x; b < G; b += blockDim.x) {
+        double c = s_flow[b];
+        for (int q = 1; q < slices; ++q) c += s_flow[q * G + b];
+        s_flow[b] = c;
+      }
+      __syncthreads();
+    }
+    auto flow = [&](int b) { /* the depth slices' sum */
+      if (SMALL) return s_flow[b];
+      double c = C[row + b];
+      for (int z = 1; z < nsplit; ++z) c += C[z * GG + row + b];
+      return c;
+    };
+    const double diag = flow(a), f = fac[a];
+    const bool cap = f != 1.0;
+    double shift = 0.0; /* a capped row's coupling: sum of dL/dN G over the row, by its sum */
+    if (cap) {
+      double cpl = 0.0;
+      for (int b = threadIdx.x; b < G; b += blockDim.x)
+        cpl = __fma_rn(b == a ? 0.0 : flow(b) - diag, Gm[row + b], cpl);
+      shift = block_sum(cpl, s_part) / rs[a];
+    }
+    double wr = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < G; b += blockDim.x) {
+      double gn = b == a ? 0.0 : flow(b) - diag;
+      if (gN) gN[row + b] = gn;
+      if (cap) gn = f * (gn - shift);
+      const double w = b == a ? 0.0 : gn * Gm[row + b];
+      if (nonzero(w)) { /* not a zero flow, whose logs may be infinite */
+        wr += w;
+        wb = __fma_rn(w, logp[b], wb);
+        wc = __fma_rn(w, logd[row + b], wc);
+      }
+    }
+    if (nonzero(wr)) {
+      wk += wr;
+      wa = __fma_rn(wr, logp[a], wa);
+    }
+    if (SMALL) __syncthreads(); /* the row is read before the next one is summed */
   }
   wk = block_sum(wk, s_part);
   wa = block_sum(wa, s_part);
@@ -382,11 +460,13 @@ __global__ void __launch_bounds__(INC_THREADS)
     atomicAdd(&g_theta[0], wk / k);
     atomicAdd(&g_theta[1], wa);
     atomicAdd(&g_theta[2], wb);
-    atomicAdd(&g_theta[3], wc);
+    atomicAdd(&g_theta[3], -wc - wk * logP);
   }
 }
 
 }  // namespace
+
+enum { SC_LOSS = 0, SC_R = 1, SC_THETA = 4, SC_ERR = 8, SC_N = 16 };
 
 struct lpg_incidence_plan {
   int T = 0, G = 0, S = 0;
@@ -394,16 +474,26 @@ struct lpg_incidence_plan {
   cudaStream_t st = nullptr;
   bool own_stream = false;
   double P = 0.0, logP = 0.0;
+  double max_lp2 = 0.0, max_ld2 = 0.0; /* largest finite |log2 pops|, |log2 dist| */
+  bool small = false;                  /* the contractions summed in FP64 where they are used */
   /* resident inputs */
-  double *srisk = nullptr, *beta = nullptr, *pop = nullptr, *doy = nullptr, *year = nullptr, *pops = nullptr,
-         *logp = nullptr, *logd = nullptr, *target = nullptr;
+  double *srisk = nullptr, *beta = nullptr, *rpop = nullptr, *doy = nullptr, *year = nullptr, *pops = nullptr,
+         *logp = nullptr, *logd = nullptr, *target = nullptr; /* target: its log1p */
+  int64_t *lp2 = nullptr, *ld2 = nullptr;
+  IxTables* tab = nullptr;
   /* per evaluation */
-  double *r0s = nullptr, *seas = nullptr, *Gm = nullptr, *rs = nullptr, *rsN = nullptr, *u = nullptr,
-         *e = nullptr, *lam = nullptr, *g = nullptr, *gseas = nullptr, *gr0s = nullptr, *scal = nullptr,
-         *C = nullptr, *gN = nullptr;
-  float2 *beta_hl = nullptr, *N = nullptr, *gu = nullptr; /* the products' operands as FP32 pairs */
-  int* cap = nullptr;
-  double* h_scal = nullptr; /* pinned: [0] loss, [1] R, [2] amp, [3] peak, [4..7] k, a, b, c */
+  double *r0s = nullptr, *seas = nullptr, *Gm = nullptr, *rs = nullptr, *rsN = nullptr, *fac = nullptr,
+         *u = nullptr, *lam = nullptr, *g = nullptr, *C = nullptr, *gN = nullptr;
+  /* cleared each evaluation, one block: sums [SC_N], gr0s [G], w [T], column maxima of N and dL/du [G] */
+  double *sums = nullptr, *gr0s = nullptr, *gw = nullptr;
+  unsigned long long *max_n = nullptr, *max_gu = nullptr;
+  size_t clear_bytes = 0;
+  double *N = nullptr, *gu = nullptr;
+  /* the sliced products: digits, row and column maxima, tensor maps */
+  uint32_t *b_rows = nullptr, *b_cols = nullptr, *n_cols = nullptr, *gu_cols = nullptr;
+  unsigned long long *max_br = nullptr, *max_bc = nullptr;
+  CUtensorMap map_b{}, map_n{}, map_bt{}, map_gu{};
+  double* host = nullptr; /* pinned: sums and gr0s [SC_N + G], then r0s [G] */
   /* profiling */
   bool prof = false;
   cudaEvent_t ev[PH_COUNT + 1] = {};
@@ -433,33 +523,59 @@ int dalloc(T** p, size_t n) {
 }
 
 void plan_free(lpg_incidence_plan* p) {
-  void* ps[] = {p->srisk, p->beta, p->pop, p->doy, p->year,  p->pops, p->logp, p->logd, p->target,
-                p->r0s,   p->seas, p->Gm,  p->N,   p->rs,    p->rsN,  p->u,    p->e,    p->lam,
-                p->g,     p->gu,   p->gseas, p->gr0s, p->scal, p->C,   p->gN,   p->cap,  p->beta_hl};
+  void* ps[] = {p->srisk, p->beta, p->rpop, p->doy,  p->year,    p->pops,   p->logp,   p->logd,    p->target,
+                p->lp2,   p->ld2,  p->tab,  p->r0s,  p->seas,    p->Gm,     p->rs,     p->rsN,     p->fac,
+                p->u,     p->lam,  p->g,    p->C,    p->gN,      p->sums,   p->N,
+                p->gu,    p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc};
   for (void* q : ps)
     if (q) cudaFree(q);
-  if (p->h_scal) cudaFreeHost(p->h_scal);
+  if (p->host) cudaFreeHost(p->host);
   for (auto& ev : p->ev)
     if (ev) cudaEventDestroy(ev);
   if (p->own_stream && p->st) cudaStreamDestroy(p->st);
   delete p;
 }
 
+/* The shapes of the two sliced products and their depth slices. */
+void plan_products(const lpg_incidence_plan* p, OzArgs* mix, OzArgs* flows);
+
+int depth_pad(int k) { return (k + OZ_BK - 1) / OZ_BK * OZ_BK; }
+
 int plan_alloc(lpg_incidence_plan* p) {
-  const size_t T = p->T, G = p->G, TG = T * G, TSG = TG * p->S, GG = G * G;
+  const size_t T = p->T, G = p->G, TG = T * G, TSG = TG * p->S, GG = G * G, TS = T * p->S;
   int rc;
-  if ((rc = dalloc(&p->srisk, TG)) || (rc = dalloc(&p->beta, TSG)) || (rc = dalloc(&p->pop, TG)) ||
+  if ((rc = dalloc(&p->srisk, TG)) || (rc = dalloc(&p->beta, TSG)) || (rc = dalloc(&p->rpop, TG)) ||
       (rc = dalloc(&p->doy, T)) || (rc = dalloc(&p->year, T)) || (rc = dalloc(&p->pops, G)) ||
       (rc = dalloc(&p->logp, G)) || (rc = dalloc(&p->logd, GG)) || (rc = dalloc(&p->r0s, G)) ||
-      (rc = dalloc(&p->seas, 3 * T)) || (rc = dalloc(&p->Gm, GG)) || (rc = dalloc(&p->N, GG)) ||
-      (rc = dalloc(&p->beta_hl, TSG)) ||
-      (rc = dalloc(&p->rs, G)) || (rc = dalloc(&p->rsN, G)) || (rc = dalloc(&p->cap, G)) ||
-      (rc = dalloc(&p->u, TSG)) || (rc = dalloc(&p->e, TSG)) || (rc = dalloc(&p->lam, TG)) ||
-      (rc = dalloc(&p->g, TG)) || (rc = dalloc(&p->gu, TSG)) || (rc = dalloc(&p->gseas, T)) ||
-      (rc = dalloc(&p->gr0s, G)) || (rc = dalloc(&p->scal, 8)) || (rc = dalloc(&p->C, DF_MAX_SPLIT * GG)) ||
-      (rc = dalloc(&p->gN, GG)))
+      (rc = dalloc(&p->lp2, G)) || (rc = dalloc(&p->ld2, GG)) || (rc = dalloc(&p->tab, 1)) ||
+      (rc = dalloc(&p->seas, 3 * T)) || (rc = dalloc(&p->Gm, GG)) || (rc = dalloc(&p->rs, G)) ||
+      (rc = dalloc(&p->rsN, G)) || (rc = dalloc(&p->fac, G)) || (rc = dalloc(&p->lam, TG)) ||
+      (rc = dalloc(&p->g, TG)) || (rc = dalloc(&p->gN, GG)))
     return rc;
-  PCK(cudaMallocHost((void**)&p->h_scal, 8 * sizeof(double)));
+  const size_t clear = SC_N + G + T + 2 * G;
+  if ((rc = dalloc(&p->sums, clear))) return rc;
+  p->clear_bytes = clear * sizeof(double);
+  p->gr0s = p->sums + SC_N;
+  p->gw = p->gr0s + G;
+  p->max_n = reinterpret_cast<unsigned long long*>(p->gw + T);
+  p->max_gu = p->max_n + G;
+  if ((rc = dalloc(&p->gu, TSG))) return rc;
+  if (!p->small) {
+    const size_t kg = depth_pad(p->G), kt = depth_pad((int)TS), half = OZ_SLICES / 2; /* two digits a word */
+    OzArgs mix{}, flows{};
+    plan_products(p, &mix, &flows);
+    if ((rc = dalloc(&p->u, mix.split * TSG)) || (rc = dalloc(&p->C, flows.split * GG)) ||
+        (rc = dalloc(&p->b_rows, half * TS * kg)) ||
+        (rc = dalloc(&p->b_cols, half * G * kt)) || (rc = dalloc(&p->n_cols, half * G * kg)) ||
+        (rc = dalloc(&p->gu_cols, half * G * kt)) || (rc = dalloc(&p->max_br, TS)) || (rc = dalloc(&p->max_bc, G)))
+      return rc;
+    if (!oz_map(&p->map_b, p->b_rows, (int)TS, (int)kg, OZ_BM) || !oz_map(&p->map_n, p->n_cols, p->G, (int)kg, OZ_BN) ||
+        !oz_map(&p->map_bt, p->b_cols, p->G, (int)kt, OZ_BM) || !oz_map(&p->map_gu, p->gu_cols, p->G, (int)kt, OZ_BN))
+      return lpg_ops_fail(LPG_ERR_CUDA, "incidence plan: a tensor map was refused");
+  } else if ((rc = dalloc(&p->N, GG))) {
+    return rc;
+  }
+  PCK(cudaMallocHost((void**)&p->host, (SC_N + 2 * G) * sizeof(double)));
   for (auto& ev : p->ev) PCK(cudaEventCreate(&ev));
   return LPG_OK;
 }
@@ -470,45 +586,118 @@ inline void mark(lpg_incidence_plan* p, int ph, int n_launch) {
   p->launches[ph] += n_launch;
 }
 
-int plan_forward(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars sc, bool with_loss) {
-  const int T = p->T, G = p->G, S = p->S;
-  const double Pc = pow(p->P, prm->c);
-  mark(p, PH_NETWORK, 1);
-  k_inc_network<<<G + (T + INC_THREADS - 1) / INC_THREADS, INC_THREADS, 0, p->st>>>(
-      G, T, p->pops, p->logp, p->logd, prm->k, prm->a, prm->b, prm->c, Pc, prm->max_frac, p->Gm, p->N, p->rs,
-      p->rsN, p->cap, p->doy, p->year, sc, p->seas);
-  mark(p, PH_MIX, 1);
-  {
-    const dim3 grd((G + DF_BN - 1) / DF_BN, (T * S + DF_BM - 1) / DF_BM, 1);
-    k_inc_gemm<false><<<grd, DF_THREADS, 0, p->st>>>(T * S, G, G, G, p->beta_hl, p->N, p->u);
-  }
-  mark(p, PH_FORWARD, 1);
-  k_inc_forward<<<dim3((G + INC_THREADS - 1) / INC_THREADS, T), INC_THREADS, 0, p->st>>>(
-      T, G, S, p->srisk, p->beta, p->pop, p->seas, p->r0s, p->rsN, sc, p->u, p->e, p->lam,
-      with_loss ? p->target : nullptr, p->g, p->scal);
-  return plan_cuda(cudaGetLastError(), "forward launch");
+void plan_products(const lpg_incidence_plan* p, OzArgs* mix, OzArgs* flows) {
+  const int TS = p->T * p->S;
+  mix->M = TS;
+  mix->N = p->G;
+  mix->k_stages = depth_pad(p->G) / OZ_BK;
+  oz_plan(mix, p->nsm, INC_MAX_SPLIT);
+  mix->max_a = p->max_br;
+  mix->max_b = p->max_n;
+  mix->C = p->u;
+  mix->err = p->sums + SC_ERR;
+  flows->M = p->G;
+  flows->N = p->G;
+  flows->k_stages = depth_pad(TS) / OZ_BK;
+  oz_plan(flows, p->nsm, INC_MAX_SPLIT);
+  flows->max_a = p->max_bc;
+  flows->max_b = p->max_gu;
+  flows->C = p->C;
+  flows->err = p->sums + SC_ERR;
 }
 
-int plan_backward(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars sc) {
-  const int T = p->T, G = p->G, S = p->S;
-  mark(p, PH_BACKWARD, 2);
-  k_inc_backward<<<dim3((G + INC_THREADS - 1) / INC_THREADS, T), INC_THREADS, 0, p->st>>>(
-      T, G, S, p->g, p->srisk, p->pop, p->seas, p->r0s, sc, p->u, p->e, p->gu, p->gseas, p->gr0s, p->scal + 1);
-  k_inc_seasonal<<<1, INC_THREADS, 0, p->st>>>(T, p->seas, p->gseas, p->scal + 2);
-  mark(p, PH_FLOWS, 1);
-  /* depth slices so that the G x G output fills the SMs about four deep */
-  const int K = T * S, gx = (G + DF_BN - 1) / DF_BN, gy = (G + DF_BM - 1) / DF_BM;
-  const int ktiles = (K + DF_BK - 1) / DF_BK;
-  int split = (4 * p->nsm + gx * gy - 1) / (gx * gy);
-  split = split < 1 ? 1 : split > DF_MAX_SPLIT ? DF_MAX_SPLIT : split;
-  if (split > ktiles) split = ktiles;
-  const int kchunk = ((ktiles + split - 1) / split) * DF_BK;
-  const int nsplit = (K + kchunk - 1) / kchunk;
-  k_inc_gemm<true><<<dim3(gx, gy, nsplit), DF_THREADS, 0, p->st>>>(G, G, K, kchunk, p->beta_hl, p->gu, p->C);
-  mark(p, PH_NETWORK_GRAD, 1);
-  k_inc_network_grad<<<G, INC_THREADS, 0, p->st>>>(G, nsplit, p->C, p->Gm, p->rs, p->cap, p->logp, p->logd,
-                                                   prm->k, p->logP, prm->max_frac, p->gN, p->scal + 4);
-  return plan_cuda(cudaGetLastError(), "backward launch");
+/* x with 56 fraction bits, |x| < 64. */
+int64_t fixed56(double x) { return (int64_t)std::llrint(x * 72057594037927936.0); }
+
+template <bool SMALL>
+int launch_step(lpg_incidence_plan* p, const IncStep& A) {
+  /* one tick a thread, for latency, until that is 32 CTAs an SM; two beyond,
+   * which halves the atomics (774 nodes, 365 ticks: 45 and 47 us; 4000
+   * nodes, 90 ticks: 88 and 79 us; eight ticks a thread: 73 and 127) */
+  const int gx = (p->G + 127) / 128;
+  if ((int64_t)p->T * gx <= 32LL * p->nsm)
+    k_inc_step<SMALL, 1><<<dim3(gx, p->T), 128, 0, p->st>>>(p->tab, A);
+  else
+    k_inc_step<SMALL, 2><<<dim3(gx, (p->T + 1) / 2), 128, 0, p->st>>>(p->tab, A);
+  return plan_cuda(cudaGetLastError(), "step launch");
+}
+
+int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars sc, bool with_loss, const double* g_in,
+             bool want_lam, bool grad, bool want_network) {
+  const int T = p->T, G = p->G, S = p->S, TS = T * S;
+  IncGravity V{prm->a, prm->b, prm->c, prm->k / pow(p->P, prm->c), prm->max_frac, 0, 0, 0, 0};
+  auto small = [](double x) { return std::fabs(x) < 60.0; };
+  if (small(V.a) && small(V.b) && small(V.c) && std::fabs(V.a) * p->max_lp2 < 900.0 &&
+      std::fabs(V.b) * p->max_lp2 + std::fabs(V.c) * p->max_ld2 < 900.0) {
+    V.a56 = fixed56(V.a);
+    V.b56 = fixed56(V.b);
+    V.c56 = fixed56(V.c);
+    V.integer = 1;
+  }
+  OzArgs mix{}, flows{};
+  plan_products(p, &mix, &flows);
+  mark(p, PH_NETWORK, p->small ? 1 : 3);
+  const int nblk = G + (T + 31) / 32;
+  if (p->small) {
+    k_inc_network<true><<<nblk, INC_THREADS, 0, p->st>>>(G, T, p->tab, p->pops, p->logp, p->logd, p->lp2, p->ld2, V,
+                                                         p->Gm, p->N, p->rs, p->rsN, p->fac, p->doy, p->year, sc,
+                                                         p->seas);
+  } else {
+    k_inc_network<false><<<nblk, INC_THREADS, 0, p->st>>>(G, T, p->tab, p->pops, p->logp, p->logd, p->lp2, p->ld2, V,
+                                                          p->Gm, nullptr, p->rs, p->rsN, p->fac, p->doy, p->year, sc,
+                                                          p->seas);
+    k_oz_col_max<<<oz_col_grid(G, G), 256, 0, p->st>>>(G, G, p->Gm, p->fac, p->max_n);
+    k_oz_slice_cols<<<dim3((G + 31) / 32, depth_pad(G) / 32), 256, 0, p->st>>>(G, G, depth_pad(G), p->Gm, p->fac,
+                                                                              p->max_n, p->n_cols);
+  }
+  mark(p, PH_MIX, 1); /* with small sums part of the step's launch, counted here too */
+  if (!p->small) PCK(oz_gemm(p->map_b, p->map_n, mix, p->nsm, p->st));
+  mark(p, PH_FORWARD, 1);
+  IncStep A{};
+  A.T = T;
+  A.G = G;
+  A.S = S;
+  A.split = mix.split;
+  A.srisk = p->srisk;
+  A.beta = p->beta;
+  A.rpop = p->rpop;
+  A.seas = p->seas;
+  A.r0s = p->r0s;
+  A.rsN = p->rsN;
+  A.u = p->u;
+  A.N = p->N;
+  A.ltarget = with_loss ? p->target : nullptr;
+  A.g_in = g_in;
+  A.R = sc.R;
+  A.lam = want_lam ? p->lam : nullptr;
+  A.loss = p->sums + SC_LOSS;
+  A.gu = p->gu;
+  A.max_gu = p->max_gu;
+  A.g_r0s = p->gr0s;
+  A.g_w = p->gw;
+  A.grad = grad;
+  const int rc = p->small ? launch_step<true>(p, A) : launch_step<false>(p, A);
+  if (rc != LPG_OK || !grad) return rc;
+  mark(p, PH_BACKWARD, 1); /* its cells are part of the step's launch, counted here too; then the slicing */
+  double* gN = want_network ? p->gN : nullptr;
+  if (p->small) {
+    mark(p, PH_FLOWS, 1); /* part of the next launch */
+    mark(p, PH_NETWORK_GRAD, 1);
+    const int smem = (int)sizeof(double) * (G > INC_THREADS ? G : INC_THREADS);
+    k_inc_network_grad<true><<<G + 1, INC_THREADS, smem, p->st>>>(
+        G, T, TS, 1, nullptr, p->beta, p->gu, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
+        p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
+  } else {
+    const int kt = depth_pad(TS);
+    k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->gu, nullptr, p->max_gu, p->gu_cols);
+    mark(p, PH_FLOWS, 1);
+    PCK(oz_gemm(p->map_bt, p->map_gu, flows, p->nsm, p->st));
+    mark(p, PH_NETWORK_GRAD, 1);
+    k_inc_network_grad<false><<<(G < 8 * p->nsm ? G : 8 * p->nsm) + 1, INC_THREADS, 0, p->st>>>(
+        G, T, TS, flows.split, p->C, nullptr, nullptr, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
+        p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
+  }
+  return plan_cuda(cudaGetLastError(), "gradient launch");
 }
 
 }  // namespace
@@ -520,9 +709,9 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
   const int T = in->T, G = in->G, S = in->S;
   if (T <= 0 || G <= 0 || S <= 0 || S > LPG_MAX_STRAINS)
     return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: bad sizes T=%d G=%d S=%d", T, G, S);
-  if ((int64_t)T * S > 65535LL * DF_BM || T > 65535)
+  if ((int64_t)T * S > INC_MAX_ROWS || T > 65535)
     return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: T=%d or T*S = %lld too large (T <= 65535, T*S <= %d)", T,
-                        (long long)T * S, 65535 * DF_BM);
+                        (long long)T * S, INC_MAX_ROWS);
   if (!in->srisk || !in->beta || !in->pop || !in->doy || !in->year || !in->pops || !in->dist)
     return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: null input array");
   double P = 0.0;
@@ -540,6 +729,24 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
   p->S = S;
   p->P = P;
   p->logP = log(P);
+  auto widest = [](double x, double* m) {
+    const double l = x > 0.0 && std::isfinite(x) ? std::fabs(std::log2(x)) : 0.0;
+    if (l > *m) *m = l;
+  };
+  for (int i = 0; i < G; ++i) widest(in->pops[i], &p->max_lp2);
+  double dlo = HUGE_VAL, dhi = 0.0;
+  for (size_t i = 0; i < (size_t)G * G; ++i)
+    if (in->dist[i] > 0.0 && std::isfinite(in->dist[i])) {
+      dlo = in->dist[i] < dlo ? in->dist[i] : dlo;
+      dhi = in->dist[i] > dhi ? in->dist[i] : dhi;
+    }
+  widest(dlo, &p->max_ld2);
+  widest(dhi, &p->max_ld2);
+  /* the FP64 sums are one chain of G terms a thread; the sliced products take
+   * about 60 us with their operands' slicing, whatever their size (181
+   * ticks, 100 nodes, 2 strains: 71 us in three kernels against 91 in eight;
+   * 21 ticks, 333 nodes, 3 strains: 131 against about 100) */
+  p->small = G <= INC_SMALL_NODES && (int64_t)T * S * G * G <= INC_SMALL_TERMS;
   int rc = LPG_OK;
   int dev = 0;
   rc = plan_cuda(cudaGetDevice(&dev), "device");
@@ -565,25 +772,39 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
       double* dst;
       const double* src;
       size_t n;
-    } up[] = {{p->srisk, in->srisk, TG},       {p->beta, bt.data(), TG * S},        {p->pop, in->pop, TG},
+    } up[] = {{p->srisk, in->srisk, TG},       {p->beta, bt.data(), TG * S},        {p->rpop, in->pop, TG},
               {p->doy, in->doy, (size_t)T},    {p->year, in->year, (size_t)T},      {p->pops, in->pops, (size_t)G},
               {d_dist, in->dist, GG}};
     for (auto& c : up) {
       rc = plan_cuda(cudaMemcpyAsync(c.dst, c.src, sizeof(double) * c.n, cudaMemcpyHostToDevice, p->st), "upload");
       if (rc != LPG_OK) break;
     }
-    if (rc == LPG_OK) {
-      k_inc_logs<<<(unsigned)((GG + INC_THREADS - 1) / INC_THREADS), INC_THREADS, 0, p->st>>>(G, p->pops, d_dist,
-                                                                                             p->logp, p->logd);
-      k_inc_split<<<(unsigned)((TG * S + INC_THREADS - 1) / INC_THREADS), INC_THREADS, 0, p->st>>>(TG * S, p->beta,
-                                                                                                 p->beta_hl);
-      rc = plan_cuda(cudaGetLastError(), "log launch");
-    }
     if (rc == LPG_OK && target) {
       rc = dalloc(&p->target, TG);
       if (rc == LPG_OK)
         rc = plan_cuda(cudaMemcpyAsync(p->target, target, sizeof(double) * TG, cudaMemcpyHostToDevice, p->st),
                        "upload target");
+    }
+    IxTables tab;
+    if (rc == LPG_OK) {
+      ix_fill_tables(&tab);
+      rc = plan_cuda(cudaMemcpyAsync(p->tab, &tab, sizeof tab, cudaMemcpyHostToDevice, p->st), "upload tables");
+    }
+    if (rc == LPG_OK) {
+      const size_t cells = GG > TG ? GG : TG;
+      k_inc_logs<<<(unsigned)((cells + INC_THREADS - 1) / INC_THREADS), INC_THREADS, 0, p->st>>>(
+          G, TG, p->pops, d_dist, p->logp, p->logd, p->lp2, p->ld2, p->rpop, p->rpop, p->target);
+      const int TS = T * S;
+      if (!p->small) {
+        const int kg = depth_pad(G), kt = depth_pad(TS);
+        rc = plan_cuda(cudaMemsetAsync(p->max_bc, 0, sizeof(unsigned long long) * G, p->st), "clear maxima");
+        k_oz_row_max<<<(TS + 7) / 8, 256, 0, p->st>>>(TS, G, p->beta, p->max_br);
+        k_oz_slice_rows<<<dim3(TS, (kg / 2 + 255) / 256), 256, 0, p->st>>>(TS, G, kg, p->beta, p->max_br, p->b_rows);
+        k_oz_col_max<<<oz_col_grid(TS, G), 256, 0, p->st>>>(TS, G, p->beta, nullptr, p->max_bc);
+        k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->beta, nullptr, p->max_bc,
+                                                                        p->b_cols);
+      }
+      if (rc == LPG_OK) rc = plan_cuda(cudaGetLastError(), "log launch");
     }
     if (rc == LPG_OK) rc = plan_cuda(cudaStreamSynchronize(p->st), "upload sync");
   }
@@ -606,24 +827,21 @@ extern "C" int lpg_incidence_plan_eval(lpg_incidence_plan* p, const lpg_incidenc
   const size_t TG = (size_t)T * G, GG = (size_t)G * G;
   const IncScalars sc{prm->R, prm->amp, prm->peak};
   const bool with_loss = p->target != nullptr && (!g_lam || loss_out);
-  PCK(cudaMemcpyAsync(p->r0s, prm->r0s, sizeof(double) * G, cudaMemcpyHostToDevice, p->st));
-  PCK(cudaMemsetAsync(p->scal, 0, sizeof(double) * 8, p->st));
-  int rc = plan_forward(p, prm, sc, with_loss);
+  double* h_r0s = p->host + SC_N + G;
+  for (int i = 0; i < G; ++i) h_r0s[i] = prm->r0s[i];
+  PCK(cudaMemcpyAsync(p->r0s, h_r0s, sizeof(double) * G, cudaMemcpyHostToDevice, p->st));
+  PCK(cudaMemsetAsync(p->sums, 0, p->clear_bytes, p->st));
+  if (grad && g_lam) PCK(cudaMemcpyAsync(p->g, g_lam, sizeof(double) * TG, cudaMemcpyHostToDevice, p->st));
+  const bool want_network = grad && grad->network;
+  const int rc = plan_run(p, prm, sc, with_loss, grad && g_lam ? p->g : nullptr, lam_out != nullptr, grad != nullptr,
+                          want_network);
   if (rc != LPG_OK) return rc;
-  if (grad) {
-    if (g_lam) PCK(cudaMemcpyAsync(p->g, g_lam, sizeof(double) * TG, cudaMemcpyHostToDevice, p->st));
-    PCK(cudaMemsetAsync(p->gseas, 0, sizeof(double) * T, p->st));
-    PCK(cudaMemsetAsync(p->gr0s, 0, sizeof(double) * G, p->st));
-    rc = plan_backward(p, prm, sc);
-    if (rc != LPG_OK) return rc;
-  }
   if (p->prof) PCK(cudaEventRecord(p->ev[PH_COUNT], p->st));
-  PCK(cudaMemcpyAsync(p->h_scal, p->scal, sizeof(double) * 8, cudaMemcpyDeviceToHost, p->st));
+  PCK(cudaMemcpyAsync(p->host, p->sums, sizeof(double) * (SC_N + (grad ? G : 0)), cudaMemcpyDeviceToHost, p->st));
   if (lam_out) PCK(cudaMemcpyAsync(lam_out, p->lam, sizeof(double) * TG, cudaMemcpyDeviceToHost, p->st));
-  if (grad && grad->r0s) PCK(cudaMemcpyAsync(grad->r0s, p->gr0s, sizeof(double) * G, cudaMemcpyDeviceToHost, p->st));
-  if (grad && grad->network)
-    PCK(cudaMemcpyAsync(grad->network, p->gN, sizeof(double) * GG, cudaMemcpyDeviceToHost, p->st));
+  if (want_network) PCK(cudaMemcpyAsync(grad->network, p->gN, sizeof(double) * GG, cudaMemcpyDeviceToHost, p->st));
   PCK(cudaStreamSynchronize(p->st));
+  if (p->host[SC_ERR] != 0.0) return lpg_ops_fail(LPG_ERR_TIMEOUT, "incidence plan: a product's wait ran out");
   if (p->prof) {
     const int last = grad ? PH_COUNT : PH_BACKWARD;
     for (int ph = 0; ph < last; ++ph) {
@@ -633,15 +851,17 @@ extern "C" int lpg_incidence_plan_eval(lpg_incidence_plan* p, const lpg_incidenc
       p->ms[ph] += ms;
     }
   }
-  if (loss_out) *loss_out = p->h_scal[0];
+  if (loss_out) *loss_out = p->host[SC_LOSS];
   if (grad) {
-    grad->R = p->h_scal[1];
-    grad->amp = p->h_scal[2];
-    grad->peak = p->h_scal[3];
-    grad->k = p->h_scal[4];
-    grad->a = p->h_scal[5];
-    grad->b = p->h_scal[6];
-    grad->c = p->h_scal[7];
+    if (grad->r0s)
+      for (int i = 0; i < G; ++i) grad->r0s[i] = p->host[SC_N + i];
+    grad->R = p->host[SC_R];
+    grad->amp = p->host[SC_R + 1];
+    grad->peak = p->host[SC_R + 2];
+    grad->k = p->host[SC_THETA];
+    grad->a = p->host[SC_THETA + 1];
+    grad->b = p->host[SC_THETA + 2];
+    grad->c = p->host[SC_THETA + 3];
   }
   return LPG_OK;
 }
