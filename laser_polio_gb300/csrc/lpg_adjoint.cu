@@ -785,11 +785,9 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
         rc = plan_cuda(cudaMemcpyAsync(p->target, target, sizeof(double) * TG, cudaMemcpyHostToDevice, p->st),
                        "upload target");
     }
-    IxTables tab;
-    if (rc == LPG_OK) {
-      ix_fill_tables(&tab);
-      rc = plan_cuda(cudaMemcpyAsync(p->tab, &tab, sizeof tab, cudaMemcpyHostToDevice, p->st), "upload tables");
-    }
+    if (rc == LPG_OK)
+      rc = plan_cuda(cudaMemcpyAsync(p->tab, ix_tables(), sizeof(IxTables), cudaMemcpyHostToDevice, p->st),
+                     "upload tables");
     if (rc == LPG_OK) {
       const size_t cells = GG > TG ? GG : TG;
       k_inc_logs<<<(unsigned)((cells + INC_THREADS - 1) / INC_THREADS), INC_THREADS, 0, p->st>>>(

@@ -8,7 +8,7 @@
  * fractions with 63 or 64 bits, good to about 2^-60, and round to a double
  * once: they are as accurate as the FP64 library's and several times
  * cheaper.  Methods: table reductions (Tang) and short Taylor series.
- * Tables are formed on the host in long double (ix_fill_tables).
+ * Tables are formed on the host in long double (ix_tables).
  */
 #ifndef LPG_IXMATH_CUH
 #define LPG_IXMATH_CUH
@@ -154,13 +154,19 @@ __device__ __forceinline__ double ix_log1p(const IxTables* T, double y) {
   return ix_double(sum << lz, 6 - lz);
 }
 
-inline void ix_fill_tables(IxTables* T) {
-  for (int j = 0; j < IX_EXP_N; ++j) T->exp2_t[j] = (uint64_t)rintl(exp2l(j / 128.0L) * 9223372036854775808.0L);
-  for (int j = 0; j < IX_LOG_N; ++j) {
-    const long double c = rintl(1024.0L / (1.0L + (j + 0.5L) / 128.0L)) / 1024.0L;
-    T->log_c[j] = (uint64_t)(c * 9223372036854775808.0L);
-    T->log_v[j] = (uint64_t)(-logl(c) * 9223372036854775808.0L);
-  }
+/* The tables, formed once (0.1 ms where long double is done in software). */
+inline const IxTables* ix_tables() {
+  static const IxTables tables = [] {
+    IxTables T;
+    for (int j = 0; j < IX_EXP_N; ++j) T.exp2_t[j] = (uint64_t)rintl(exp2l(j / 128.0L) * 9223372036854775808.0L);
+    for (int j = 0; j < IX_LOG_N; ++j) {
+      const long double c = rintl(1024.0L / (1.0L + (j + 0.5L) / 128.0L)) / 1024.0L;
+      T.log_c[j] = (uint64_t)(c * 9223372036854775808.0L);
+      T.log_v[j] = (uint64_t)(-logl(c) * 9223372036854775808.0L);
+    }
+    return T;
+  }();
+  return &tables;
 }
 
 #endif /* LPG_IXMATH_CUH */

@@ -58,25 +58,23 @@ def count_SEIRP(node_id, disease_state, strain, potentially_paralyzed, paralyzed
         raise ValueError("count_SEIRP: a column is shorter than n_people")
     device = cols[1].device
     with torch.cuda.device(device):
-        outs = [torch.empty(int(n_nodes), dtype=torch.int32, device=device) for _ in range(4)]
-        ebs = torch.empty((int(n_nodes), int(n_strains)), dtype=torch.int32, device=device)
-        ibs = torch.empty_like(ebs)
-        potp = torch.empty(int(n_nodes), dtype=torch.int32, device=device)
-        par = torch.empty_like(potp)
-        bad = torch.zeros(1, dtype=torch.int64, device=device)
+        G, ns = int(n_nodes), int(n_strains)
+        # one allocation for the eight results: the host side is most of a small call
+        S, E, I, R, potp, par, ebs, ibs = torch.empty(G * (6 + 2 * ns), dtype=torch.int32, device=device).split(
+            [G] * 6 + [G * ns] * 2)
+        bad = torch.empty(1, dtype=torch.int64, device=device) if n_invalid is not None else None
         lib = _lib.load()
         stream = torch.cuda.current_stream(device).cuda_stream
-        S, E, I, R = outs
-        rc = lib.lpg_count_seirp(*[c.data_ptr() for c in cols], int(n_nodes), int(n_strains), n_people,
+        rc = lib.lpg_count_seirp(*[c.data_ptr() for c in cols], G, ns, n_people,
                                  S.data_ptr(), E.data_ptr(), I.data_ptr(), R.data_ptr(), ebs.data_ptr(),
-                                 ibs.data_ptr(), potp.data_ptr(), par.data_ptr(), bad.data_ptr(),
-                                 C.c_void_p(stream))
+                                 ibs.data_ptr(), potp.data_ptr(), par.data_ptr(),
+                                 bad.data_ptr() if bad is not None else None, C.c_void_p(stream))
         if rc != 0:
             msg = lib.lpg_op_last_error().decode()
             if rc == -1:
                 raise ValueError(msg)
             raise _lib.LpgError(rc, msg)
-    res = (S, E, I, R, ebs, ibs, potp, par)
+    res = (S, E, I, R, ebs.view(G, ns), ibs.view(G, ns), potp, par)
     if n_invalid is not None:
         n_invalid.append(int(bad.item()))
     if host:
