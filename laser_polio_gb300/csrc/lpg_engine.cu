@@ -58,8 +58,9 @@ struct Staging {
 
 struct SimHost {
   lpg_sim_desc d;
-  std::vector<double> birth_rate, p_ri, p_ipv, strain_scal, net, rowsum, r0s, seas;
-  std::vector<uint64_t> netq_t;
+  std::vector<double> birth_rate, p_ri, p_ipv, strain_scal, r0s, seas;
+  uint64_t* netq_t = nullptr; /* device: the network in two parts, transposed */
+  double* rowsum = nullptr;   /* device */
   std::vector<float> p_sia;
   std::vector<int64_t> km;
   std::vector<lpg_seed_event> seeds;
@@ -80,6 +81,15 @@ struct lpg_handle {
   std::vector<DevRep> hreps;
   DevWorld W{};
   std::vector<void*> allocs;
+  /* small buffers are carved from slabs: one allocation, and for uploads one
+   * copy, for many */
+  struct Slab {
+    uint8_t* dev = nullptr;
+    std::vector<uint8_t> host; /* upload slabs: the bytes to copy */
+    size_t used = 0, sent = 0;
+  };
+  Slab plain;
+  std::vector<Slab> uploads;
   bool started = false;
   std::string err;
   bool use_graphs = true;
@@ -127,28 +137,125 @@ static int fail(lpg_handle* h, int code, const char* fmt, ...) {
                                        __FILE__, __LINE__);                                            \
   } while (0)
 
+constexpr size_t kSlabBytes = 1 << 20, kSlabItem = 1 << 17;
+static size_t pad256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+static int dalloc_bytes(lpg_handle* h, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) return fail(h, LPG_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  h->allocs.push_back(*p);
+  return 0;
+}
+
 template <typename T>
 static int dalloc(lpg_handle* h, T** p, size_t n) {
-  size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-  cudaError_t e = cudaMalloc((void**)p, bytes);
-  if (e != cudaSuccess) return fail(h, LPG_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-  h->allocs.push_back((void*)*p);
+  const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+  if (bytes > kSlabItem) return dalloc_bytes(h, (void**)p, bytes);
+  if (!h->plain.dev || h->plain.used + bytes > kSlabBytes) {
+    h->plain.used = 0;
+    const int rc = dalloc_bytes(h, (void**)&h->plain.dev, kSlabBytes);
+    if (rc) {
+      h->plain.dev = nullptr;
+      return rc;
+    }
+  }
+  *p = (T*)(h->plain.dev + h->plain.used);
+  h->plain.used += pad256(bytes);
   return 0;
 }
 
+/* A device copy of v; small ones arrive with the next flush_uploads. */
 template <typename T>
 static int dupload(lpg_handle* h, T** p, const std::vector<T>& v) {
-  int rc = dalloc(h, p, v.size());
-  if (rc) return rc;
-  if (!v.empty()) CK(cudaMemcpyAsync(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
+  const size_t bytes = v.size() * sizeof(T);
+  if (bytes > kSlabItem) {
+    int rc = dalloc(h, p, v.size());
+    if (rc) return rc;
+    CK(cudaMemcpyAsync(*p, v.data(), bytes, cudaMemcpyHostToDevice, h->stream));
+    return 0;
+  }
+  if (h->uploads.empty() || h->uploads.back().used + bytes > kSlabBytes) {
+    lpg_handle::Slab s;
+    const int rc = dalloc_bytes(h, (void**)&s.dev, kSlabBytes);
+    if (rc) return rc;
+    s.host.resize(kSlabBytes);
+    h->uploads.push_back(std::move(s));
+  }
+  lpg_handle::Slab& s = h->uploads.back();
+  *p = (T*)(s.dev + s.used);
+  if (bytes) memcpy(s.host.data() + s.used, v.data(), bytes);
+  s.used += pad256(std::max<size_t>(bytes, 1));
   return 0;
 }
 
+static int flush_uploads(lpg_handle* h) {
+  for (auto& s : h->uploads) {
+    if (s.used > s.sent)
+      CK(cudaMemcpyAsync(s.dev + s.sent, s.host.data() + s.sent, std::min(s.used, kSlabBytes) - s.sent,
+                         cudaMemcpyHostToDevice, h->stream));
+    s.sent = s.used;
+  }
+  return 0;
+}
+
+/* Buffers carved from one allocation: freeing a handle's 30-odd large ones
+ * one by one took more than twice as long. */
+struct Carve {
+  std::vector<std::pair<void**, size_t>> items;
+  size_t total = 0;
+  template <typename T>
+  void add(T** p, size_t n) {
+    items.emplace_back((void**)p, total);
+    total += pad256(std::max<size_t>(n, 1) * sizeof(T));
+  }
+  int commit(lpg_handle* h) {
+    uint8_t* base = nullptr;
+    const int rc = dalloc_bytes(h, (void**)&base, std::max<size_t>(total, 256));
+    if (rc) return rc;
+    for (auto& it : items) *it.first = base + it.second;
+    return 0;
+  }
+};
+
+/* Frees an allocation of its own; a part of a slab stays until the end. */
 static void dfree_one(lpg_handle* h, void* p) {
   if (!p) return;
-  cudaFree(p);
   auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
-  if (it != h->allocs.end()) h->allocs.erase(it);
+  if (it == h->allocs.end()) return;
+  cudaFree(p);
+  h->allocs.erase(it);
+}
+
+/* The network in the two fixed-point parts of lpg_net_split, transposed:
+ * q[2 (j n + i)], 32 x 32 tiles turned in shared memory. */
+__global__ void __launch_bounds__(256) k_net_split(int n, const double* __restrict__ net, ulonglong2* __restrict__ q) {
+  __shared__ double s[32][33];
+  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = ty; r < 32; r += 8)
+    if (i0 + r < n && j0 + tx < n) s[r][tx] = net[(size_t)(i0 + r) * n + j0 + tx];
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8)
+    if (j0 + r < n && i0 + tx < n) {
+      uint64_t hi, lo;
+      lpg_net_split(s[tx][r], &hi, &lo);
+      q[(size_t)(j0 + r) * n + i0 + tx] = make_ulonglong2(hi, lo);
+    }
+}
+
+/* Row sums in column order (the order decides the last bit): a warp takes
+ * 32 rows, a lane adds its own. */
+__global__ void __launch_bounds__(32) k_net_rowsum(int n, const double* __restrict__ net, double* __restrict__ sum) {
+  __shared__ double s[32][33];
+  const int i0 = blockIdx.x * 32, lane = threadIdx.x;
+  double acc = 0.0;
+  for (int j0 = 0; j0 < n; j0 += 32) {
+    __syncwarp();
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) s[r][lane] = i0 + r < n && j0 + lane < n ? net[(size_t)(i0 + r) * n + j0 + lane] : 0.0;
+    __syncwarp();
+    for (int j = 0; j < 32 && j0 + j < n; ++j) acc = acc + s[lane][j];
+  }
+  if (i0 + lane < n) sum[i0 + lane] = acc;
 }
 
 __global__ void k_fill_f32(float* p, int64_t n, float v) {
@@ -280,7 +387,13 @@ __global__ void k_scatter(DevWorld W, ScatterArgs a) {
     scatter_one(W, a, i);
 }
 
-/* Columns of one simulation (rep) back in reference slot order.  Timers of
+template <typename T>
+__device__ __forceinline__ void put(T* col, uint32_t i, T v) {
+  if (col) col[i] = v;
+}
+
+/* Columns of one simulation (rep) back in reference slot order, those that
+ * are asked for.  Timers of
  * agents in E or I are brought up to the step of tick tc (the last that has
  * run) when the simulation steps disease states (ds_on); RI timers of the
  * alive, not chronically-missed agents to the RI ticks up to tc when RI
@@ -302,23 +415,23 @@ __global__ void k_gather(DevWorld W, Staging s, int32_t chunk_base, int32_t used
     int8_t et = W.et[pos], it = W.it[pos], pt = W.pt[pos];
     if (ds_on && (ds == 1 || ds == 2)) /* the count-downs up to the step of tick tc */
       ev_advance(ds, st, et, it, pt, tc - W.evt[pos] + 1 + ev_pure(ds, st, et, it, pt, pp));
-    s.ds[i] = ds;
-    s.strain[i] = st;
-    s.et[i] = et;
-    s.it[i] = it;
-    s.pt[i] = pt;
-    s.pp[i] = pp;
-    s.par[i] = W.par[pos];
-    s.ipv[i] = W.ipv[pos];
-    s.cm[i] = cm;
-    s.node[i] = (int16_t)(meta.x - node_base);
+    put(s.ds, i, ds);
+    put(s.strain, i, st);
+    put(s.et, i, et);
+    put(s.it, i, it);
+    put(s.pt, i, pt);
+    put(s.pp, i, pp);
+    put(s.par, i, W.par[pos]);
+    put(s.ipv, i, W.ipv[pos]);
+    put(s.cm, i, cm);
+    put(s.node, i, (int16_t)(meta.x - node_base));
     int16_t ri = W.ri[pos];
     if (ri_on && ds >= 0 && cm != 1) ri = ri_now(rp, ri, i, W.dob[pos], tc);
-    s.ri[i] = ri;
-    s.risk[i] = W.risk[pos];
-    s.inf[i] = W.inf[pos];
-    s.dob[i] = W.dob[pos];
-    s.dod[i] = W.dod[pos];
+    put(s.ri, i, ri);
+    put(s.risk, i, W.risk[pos]);
+    put(s.inf, i, W.inf[pos]);
+    put(s.dob, i, W.dob[pos]);
+    put(s.dod, i, W.dod[pos]);
   }
 }
 
@@ -399,6 +512,12 @@ static int validate_desc(const lpg_sim_desc& d, int r, std::string* msg) {
   const size_t n = (size_t)d.n_nodes;
   auto check = [&](const double* a, size_t k, double lo, double hi, const char* name) -> int {
     if (!a) return 0;
+    /* all at once first, without branches (a NaN fails both comparisons) */
+    const double top = hi < 1.7976931348623157e308 ? hi : 1.7976931348623157e308;
+    const double low = lo > -1.7976931348623157e308 ? lo : -1.7976931348623157e308;
+    unsigned ok = 1;
+    for (size_t i = 0; i < k; ++i) ok &= (unsigned)(a[i] >= low) & (unsigned)(a[i] <= top);
+    if (ok) return 0;
     for (size_t i = 0; i < k; ++i)
       if (!std::isfinite(a[i]) || a[i] < lo || a[i] > hi)
         return bad(LPG_ERR_ARG, "sim %d: %s[%zu] = %g is not finite or outside [%g, %g]", r, name, i, a[i], lo, hi);
@@ -478,23 +597,8 @@ extern "C" int lpg_create(const lpg_sim_desc* sims, int32_t n_sims, int32_t devi
     s.p_ri = vec(d.vx_prob_ri, n, 0.0);
     s.p_ipv = vec(d.vx_prob_ipv, n, 0.0);
     s.strain_scal = vec(d.strain_r0_scalars, (size_t)d.n_strains, 1.0);
-    s.net = vec(d.network, n * n, 0.0);
     s.r0s = vec(d.r0_scalars, n, 1.0);
     s.seas = vec(d.seasonality, (size_t)d.nt, 1.0);
-    s.netq_t.assign(2 * n * n, 0);
-    for (size_t i = 0; i < n; ++i)
-      for (size_t j = 0; j < n; ++j) {
-        uint64_t hi, lo;
-        lpg_net_split(s.net[i * n + j], &hi, &lo);
-        s.netq_t[2 * (j * n + i)] = hi;
-        s.netq_t[2 * (j * n + i) + 1] = lo;
-      }
-    s.rowsum.assign(n, 0.0);
-    for (size_t i = 0; i < n; ++i) {
-      double acc = 0.0;
-      for (size_t j = 0; j < n; ++j) acc = acc + s.net[i * n + j];
-      s.rowsum[i] = acc;
-    }
     s.p_sia.assign(n, 0.0f);
     if (d.vx_prob_sia) std::copy(d.vx_prob_sia, d.vx_prob_sia + n, s.p_sia.begin());
     s.km.assign(d.km_cumdeaths, d.km_cumdeaths + d.km_len);
@@ -515,6 +619,30 @@ extern "C" int lpg_create(const lpg_sim_desc* sims, int32_t n_sims, int32_t devi
   CK(cudaSetDevice(device));
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   CK(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device));
+  /* the networks go to the device from where they are and are split there */
+  size_t largest = 0;
+  for (int r = 0; r < n_sims; ++r) {
+    SimHost& s = h->sims[r];
+    const size_t n = (size_t)s.d.n_nodes;
+    largest = std::max(largest, n * n);
+    if (dalloc(h, &s.netq_t, 2 * n * n) || dalloc(h, &s.rowsum, n)) return LPG_ERR_NOMEM;
+  }
+  double* net = nullptr;
+  if (dalloc(h, &net, largest)) return LPG_ERR_NOMEM;
+  for (int r = 0; r < n_sims; ++r) {
+    SimHost& s = h->sims[r];
+    const int n = s.d.n_nodes;
+    if (s.d.network)
+      CK(cudaMemcpyAsync(net, s.d.network, sizeof(double) * n * n, cudaMemcpyHostToDevice, h->stream));
+    else
+      CK(cudaMemsetAsync(net, 0, sizeof(double) * n * n, h->stream));
+    const int tiles = (n + 31) / 32;
+    k_net_split<<<dim3(tiles, tiles), 256, 0, h->stream>>>(n, net, reinterpret_cast<ulonglong2*>(s.netq_t));
+    k_net_rowsum<<<tiles, 32, 0, h->stream>>>(n, net, s.rowsum);
+    CK(cudaGetLastError());
+  }
+  CK(cudaStreamSynchronize(h->stream)); /* the caller's arrays are read */
+  dfree_one(h, net);
   return LPG_OK;
 }
 
@@ -529,7 +657,7 @@ static int alloc_staging(lpg_handle* h, Staging& s, int64_t cap) {
     total += (esz[k] * n + 255) & ~(size_t)255;
   }
   uint8_t* base = nullptr;
-  if (dalloc(h, &base, total)) return LPG_ERR_NOMEM;
+  if (dalloc_bytes(h, (void**)&base, total)) return LPG_ERR_NOMEM;
   s.base = base;
   s.ds = reinterpret_cast<int8_t*>(base + off[0]);
   s.strain = reinterpret_cast<int8_t*>(base + off[1]);
@@ -688,69 +816,91 @@ extern "C" int lpg_start(lpg_handle* h) {
   W.wait_spin = h->test_wait_spin > 0 ? h->test_wait_spin : LPG_MBAR_SPIN;
   W.test_bar_skip = h->test_bar_skip;
   const int64_t P = (int64_t)chunk_total * LPG_CHUNK;
-  int rc = 0;
-  rc |= dalloc(h, &W.ds, P);
-  rc |= dalloc(h, &W.strain, P);
-  rc |= dalloc(h, &W.et, P);
-  rc |= dalloc(h, &W.it, P);
-  rc |= dalloc(h, &W.pt, P);
-  rc |= dalloc(h, &W.pp, P);
-  rc |= dalloc(h, &W.par, P);
-  rc |= dalloc(h, &W.ipv, P);
-  rc |= dalloc(h, &W.cm, P);
-  rc |= dalloc(h, &W.ri, P);
-  rc |= dalloc(h, &W.risk, P);
-  rc |= dalloc(h, &W.inf, P);
-  rc |= dalloc(h, &W.dob, P);
-  rc |= dalloc(h, &W.dod, P);
-  rc |= dalloc(h, &W.evt, P);
-  rc |= dalloc(h, &W.rdt, P);
-  rc |= dalloc(h, &W.ref, P);
-  rc |= dalloc(h, &W.cmeta, chunk_total);
-  rc |= dalloc(h, &W.qcnt, 2048);
-  rc |= dalloc(h, &W.qfirst, 2048);
-  rc |= dalloc(h, &W.due, (size_t)chunk_total * LPG_NSUB);
-  rc |= dalloc(h, &W.due_n, 1);
-  rc |= dalloc(h, &W.evq, (size_t)chunk_total * LPG_CHUNK);
-  rc |= dalloc(h, &W.chunk_w, chunk_total);
-  rc |= dalloc(h, &W.sub_w, (size_t)chunk_total * LPG_NSUB);
-  rc |= dalloc(h, &W.sub_dod, (size_t)chunk_total * LPG_NSUB);
-  rc |= dalloc(h, &W.sub_evt, (size_t)chunk_total * LPG_NSUB);
-  rc |= dalloc(h, &W.sub_rdt, (size_t)chunk_total * LPG_NSUB);
-  rc |= dalloc(h, &W.cpref, chunk_total);
-  rc |= dalloc(h, &W.node_chunks[0], chunk_total);
-  rc |= dalloc(h, &W.node_chunks[1], chunk_total);
-  rc |= dalloc(h, &W.node_chunk_start[0], csr_total);
-  rc |= dalloc(h, &W.node_chunk_start[1], csr_total);
-  rc |= dalloc(h, &W.node_rep, G);
-  rc |= dalloc(h, &W.node_count, G);
-  rc |= dalloc(h, &W.ev, (size_t)EV_N * G);
-  rc |= dalloc(h, &W.tot, (size_t)TT_N * G);
-  rc |= dalloc(h, &W.sw, G);
-  rc |= dalloc(h, &W.bb, (size_t)LPG_MAX_STRAINS * G);
-  rc |= dalloc(h, &W.nb_end, G);
-  rc |= dalloc(h, &W.nb_li0, G);
-  rc |= dalloc(h, &W.prob, (size_t)LPG_MAX_STRAINS * G);
-  rc |= dalloc(h, &W.inck, (size_t)LPG_MAX_STRAINS * G);
-  rc |= dalloc(h, &W.size, G);
-  rc |= dalloc(h, &W.uniq, G);
-  rc |= dalloc(h, &W.ksel, G);
-  rc |= dalloc(h, &W.tgt_off, G + 1);
-  {
-    uint8_t* si = nullptr;
-    rc |= dalloc(h, &si, (size_t)G * sizeof(SelInfo));
-    W.sel_info = si;
-  }
+  Carve carve;
+  carve.add(&W.ds, P);
+  carve.add(&W.strain, P);
+  carve.add(&W.et, P);
+  carve.add(&W.it, P);
+  carve.add(&W.pt, P);
+  carve.add(&W.pp, P);
+  carve.add(&W.par, P);
+  carve.add(&W.ipv, P);
+  carve.add(&W.cm, P);
+  carve.add(&W.ri, P);
+  carve.add(&W.risk, P);
+  carve.add(&W.inf, P);
+  carve.add(&W.dob, P);
+  carve.add(&W.dod, P);
+  carve.add(&W.evt, P);
+  carve.add(&W.rdt, P);
+  carve.add(&W.ref, P);
+  carve.add(&W.cmeta, chunk_total);
+  carve.add(&W.qcnt, 2048);
+  carve.add(&W.qfirst, 2048);
+  carve.add(&W.due, (size_t)chunk_total * LPG_NSUB);
+  carve.add(&W.due_n, 1);
+  carve.add(&W.evq, (size_t)chunk_total * LPG_CHUNK);
+  carve.add(&W.chunk_w, chunk_total);
+  carve.add(&W.sub_w, (size_t)chunk_total * LPG_NSUB);
+  carve.add(&W.sub_dod, (size_t)chunk_total * LPG_NSUB);
+  carve.add(&W.sub_evt, (size_t)chunk_total * LPG_NSUB);
+  carve.add(&W.sub_rdt, (size_t)chunk_total * LPG_NSUB);
+  carve.add(&W.cpref, chunk_total);
+  carve.add(&W.node_chunks[0], chunk_total);
+  carve.add(&W.node_chunks[1], chunk_total);
+  carve.add(&W.node_chunk_start[0], csr_total);
+  carve.add(&W.node_chunk_start[1], csr_total);
+  carve.add(&W.node_rep, G);
+  carve.add(&W.node_count, G);
+  carve.add(&W.ev, (size_t)EV_N * G);
+  carve.add(&W.tot, (size_t)TT_N * G);
+  carve.add(&W.sw, G);
+  carve.add(&W.bb, (size_t)LPG_MAX_STRAINS * G);
+  carve.add(&W.nb_end, G);
+  carve.add(&W.nb_li0, G);
+  carve.add(&W.prob, (size_t)LPG_MAX_STRAINS * G);
+  carve.add(&W.inck, (size_t)LPG_MAX_STRAINS * G);
+  carve.add(&W.size, G);
+  carve.add(&W.uniq, G);
+  carve.add(&W.ksel, G);
+  carve.add(&W.tgt_off, G + 1);
+  uint8_t* sel_info = nullptr;
+  carve.add(&sel_info, (size_t)G * sizeof(SelInfo));
   /* selection targets (at most the susceptibles) and the E/I queue slabs
    * (at most one entry per position) share this buffer */
   int64_t hits = (int64_t)chunk_total * LPG_CHUNK;
   W.hits_cap = hits;
-  rc |= dalloc(h, &W.hits, hits);
-  rc |= dalloc(h, &W.ctr, LPG_NUM_COUNTERS);
-  rc |= dalloc(h, &W.end_done, 1);
-  rc |= dalloc(h, &W.grid_bar, 1);
-  rc |= dalloc(h, &W.reps, R);
-  if (rc) return LPG_ERR_NOMEM;
+  carve.add(&W.hits, hits);
+  carve.add(&W.ctr, LPG_NUM_COUNTERS);
+  carve.add(&W.end_done, 1);
+  carve.add(&W.grid_bar, 1);
+  carve.add(&W.reps, R);
+  for (int r = 0; r < R; ++r) { /* results, and the unborn pools: reference slots [count, capacity) */
+    const lpg_sim_desc& d = h->sims[r].d;
+    DevRep& rp = hr[r];
+    int64_t off = 0;
+    for (int k = 0; k < RS_N; ++k) {
+      rp.res_off[k] = off;
+      off += (int64_t)d.nt * d.n_nodes * (res_wide[k] ? d.n_strains : 1);
+    }
+    h->sims[r].res_elems = off;
+    carve.add(&rp.res, off);
+    if (h->sims[r].record) carve.add(&rp.rec, (size_t)d.nt * d.n_nodes * (3 + d.n_strains));
+    const int64_t np = d.capacity - d.count;
+    carve.add(&rp.pl_et, np);
+    carve.add(&rp.pl_it, np);
+    carve.add(&rp.pl_pt, np);
+    carve.add(&rp.pl_strain, np);
+    carve.add(&rp.pl_pp, np);
+    carve.add(&rp.pl_par, np);
+    carve.add(&rp.pl_ipv, np);
+    carve.add(&rp.pl_cm, np);
+    carve.add(&rp.pl_ri, np);
+    carve.add(&rp.pl_risk, np);
+    carve.add(&rp.pl_inf, np);
+  }
+  if (carve.commit(h)) return LPG_ERR_NOMEM;
+  W.sel_info = sel_info;
   CK(cudaMemsetAsync(W.ds, 0xff, P, st));
   CK(cudaMemsetAsync(W.ref, 0xff, P * 4, st));
   CK(cudaMemsetAsync(W.qcnt, 0, 4 * 2048, st));
@@ -815,15 +965,8 @@ extern "C" int lpg_start(lpg_handle* h) {
     rp.p_ipv = dp;
     if (dupload(h, &dp, s.strain_scal)) return LPG_ERR_NOMEM;
     rp.strain_scal = dp;
-    if (dupload(h, &dp, s.net)) return LPG_ERR_NOMEM;
-    rp.net = dp;
-    {
-      uint64_t* qp;
-      if (dupload(h, &qp, s.netq_t)) return LPG_ERR_NOMEM;
-      rp.netq_t = qp;
-    }
-    if (dupload(h, &dp, s.rowsum)) return LPG_ERR_NOMEM;
-    rp.rowsum = dp;
+    rp.netq_t = s.netq_t;
+    rp.rowsum = s.rowsum;
     if (dupload(h, &dp, s.r0s)) return LPG_ERR_NOMEM;
     rp.r0s = dp;
     if (dupload(h, &dp, s.seas)) return LPG_ERR_NOMEM;
@@ -912,37 +1055,15 @@ extern "C" int lpg_start(lpg_handle* h) {
     if (dupload(h, &dd_, hseed)) return LPG_ERR_NOMEM;
     rp.seeds = dd_;
     /* results */
-    int64_t off = 0;
-    for (int k = 0; k < RS_N; ++k) {
-      rp.res_off[k] = off;
-      off += (int64_t)d.nt * n * (res_wide[k] ? d.n_strains : 1);
-    }
-    s.res_elems = off;
-    if (dalloc(h, &rp.res, off)) return LPG_ERR_NOMEM;
-    CK(cudaMemsetAsync(rp.res, 0, sizeof(int32_t) * off, st));
+    CK(cudaMemsetAsync(rp.res, 0, sizeof(int32_t) * s.res_elems, st));
     CK(cudaMemcpyAsync(rp.res + rp.res_off[RS_POP], s.pop0.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
     if (!s.Rpre.empty())
       CK(cudaMemcpyAsync(rp.res + rp.res_off[RS_R], s.Rpre.data(), sizeof(int32_t) * s.Rpre.size(), cudaMemcpyHostToDevice, st));
     if (s.record) {
       const size_t nrec = (size_t)d.nt * n * (3 + d.n_strains);
-      if (dalloc(h, &rp.rec, nrec)) return LPG_ERR_NOMEM;
       CK(cudaMemsetAsync(rp.rec, 0, sizeof(double) * nrec, st));
     }
-    /* unborn pool: reference slots [count, capacity) */
-    const int64_t np = std::max<int64_t>(d.capacity - d.count, 1);
-    rc = 0;
-    rc |= dalloc(h, &rp.pl_et, np);
-    rc |= dalloc(h, &rp.pl_it, np);
-    rc |= dalloc(h, &rp.pl_pt, np);
-    rc |= dalloc(h, &rp.pl_strain, np);
-    rc |= dalloc(h, &rp.pl_pp, np);
-    rc |= dalloc(h, &rp.pl_par, np);
-    rc |= dalloc(h, &rp.pl_ipv, np);
-    rc |= dalloc(h, &rp.pl_cm, np);
-    rc |= dalloc(h, &rp.pl_ri, np);
-    rc |= dalloc(h, &rp.pl_risk, np);
-    rc |= dalloc(h, &rp.pl_inf, np);
-    if (rc) return LPG_ERR_NOMEM;
+    /* unborn pool */
     const int64_t pc = d.capacity - d.count;
     if (pc > 0) {
       Staging& g = s.stg;
@@ -972,6 +1093,7 @@ extern "C" int lpg_start(lpg_handle* h) {
     }
     h_start[rp.csr_base + n] = csr_start[r][n];
   }
+  if (flush_uploads(h)) return LPG_ERR_CUDA;
   CK(cudaMemcpyAsync(W.node_rep, h_node_rep.data(), sizeof(int32_t) * G, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(W.node_count, h_node_count.data(), sizeof(int64_t) * G, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(W.cmeta, h_meta.data(), sizeof(int4) * chunk_total, cudaMemcpyHostToDevice, st));
@@ -1000,6 +1122,7 @@ extern "C" int lpg_start(lpg_handle* h) {
       if (dupload(h, &d_rank, rank)) return LPG_ERR_NOMEM;
       CK(cudaStreamSynchronize(st));
     }
+    if (flush_uploads(h)) return LPG_ERR_CUDA;
     ScatterArgs a{s.stg, s.d.count, d_nc0, d_first, d_rank};
     if (s.d.count > 0) {
       if (a.rank) k_scatter<<<2048, 256, 0, st>>>(W, a);
@@ -1312,6 +1435,44 @@ extern "C" int lpg_read_aggregates(lpg_handle* h, int32_t sim, double* srisk, do
   return LPG_OK;
 }
 
+static Staging staging_of(const lpg_columns* c) {
+  Staging s;
+  s.ds = c->disease_state;
+  s.strain = c->strain;
+  s.et = c->exposure_timer;
+  s.it = c->infection_timer;
+  s.pt = c->paralysis_timer;
+  s.pp = c->potentially_paralyzed;
+  s.par = c->paralyzed;
+  s.ipv = c->ipv_protected;
+  s.cm = c->chronically_missed;
+  s.node = c->node_id;
+  s.ri = c->ri_timer;
+  s.risk = c->acq_risk_multiplier;
+  s.inf = c->daily_infectivity;
+  s.dob = c->date_of_birth;
+  s.dod = c->date_of_death;
+  return s;
+}
+
+/* Every column given lies in this device's own memory, aligned to its element. */
+static bool on_device(const lpg_columns* c, int device) {
+  const Staging s = staging_of(c);
+  const std::pair<const void*, size_t> ps[] = {{s.ds, 1}, {s.strain, 1}, {s.et, 1}, {s.it, 1}, {s.pt, 1},
+                                               {s.pp, 1}, {s.par, 1}, {s.ipv, 1}, {s.cm, 1}, {s.node, 2},
+                                               {s.ri, 2}, {s.risk, 4}, {s.inf, 4}, {s.dob, 4}, {s.dod, 4}};
+  for (const auto& p : ps) {
+    if (!p.first) continue;
+    cudaPointerAttributes at;
+    if ((uintptr_t)p.first % p.second || cudaPointerGetAttributes(&at, p.first) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+  }
+  return true;
+}
+
 extern "C" int lpg_read_columns(lpg_handle* h, int32_t sim, const lpg_columns* c) {
   if (!h || !c || sim < 0 || sim >= (int)h->sims.size()) return LPG_ERR_ARG;
   if (!h->started) return fail(h, LPG_ERR_STATE, "no columns before lpg_start");
@@ -1319,6 +1480,16 @@ extern "C" int lpg_read_columns(lpg_handle* h, int32_t sim, const lpg_columns* c
   CK(cudaStreamSynchronize(h->stream));
   DevRep r;
   CK(cudaMemcpy(&r, h->W.reps + sim, sizeof(DevRep), cudaMemcpyDeviceToHost));
+  /* columns that are all on this device are written where they are; host
+   * ones go through a staging copy */
+  if (on_device(c, h->device)) {
+    const Staging to = staging_of(c);
+    k_gather<<<2048, 256, 0, h->stream>>>(h->W, to, r.chunk_base, r.used_chunks, r.node_base, r.t - 1,
+                                          (r.comps & LPG_COMP_DS) ? 1 : 0, sim);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(h->stream));
+    return LPG_OK;
+  }
   Staging s;
   int rc = alloc_staging(h, s, std::max<int64_t>(r.count, 1));
   if (rc) return rc;
@@ -1358,11 +1529,17 @@ extern "C" int lpg_check_invariants(lpg_handle* h) {
   int32_t *tot, *subd, *sube, *subr;
   uint64_t *sw, *bb, *cw, *subw;
   int* bad;
-  if (dalloc(h, &tot, (size_t)TT_N * G) || dalloc(h, &sw, G) || dalloc(h, &bb, (size_t)LPG_MAX_STRAINS * G) ||
-      dalloc(h, &cw, W.total_chunks) || dalloc(h, &subw, (size_t)W.total_chunks * LPG_NSUB) ||
-      dalloc(h, &subd, (size_t)W.total_chunks * LPG_NSUB) || dalloc(h, &sube, (size_t)W.total_chunks * LPG_NSUB) ||
-      dalloc(h, &subr, (size_t)W.total_chunks * LPG_NSUB) || dalloc(h, &bad, 1))
-    return LPG_ERR_NOMEM;
+  Carve carve;
+  carve.add(&tot, (size_t)TT_N * G);
+  carve.add(&sw, G);
+  carve.add(&bb, (size_t)LPG_MAX_STRAINS * G);
+  carve.add(&cw, W.total_chunks);
+  carve.add(&subw, (size_t)W.total_chunks * LPG_NSUB);
+  carve.add(&subd, (size_t)W.total_chunks * LPG_NSUB);
+  carve.add(&sube, (size_t)W.total_chunks * LPG_NSUB);
+  carve.add(&subr, (size_t)W.total_chunks * LPG_NSUB);
+  carve.add(&bad, 1);
+  if (carve.commit(h)) return LPG_ERR_NOMEM;
   cudaStream_t st = h->stream;
   CK(cudaMemsetAsync(tot, 0, sizeof(int32_t) * TT_N * G, st));
   CK(cudaMemsetAsync(sw, 0, sizeof(uint64_t) * G, st));
@@ -1381,8 +1558,7 @@ extern "C" int lpg_check_invariants(lpg_handle* h) {
   int hb = 0;
   CK(cudaMemcpyAsync(&hb, bad, 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  void* ps[] = {tot, sw, bb, cw, subw, subd, sube, subr, bad};
-  for (void* p : ps) dfree_one(h, p);
+  dfree_one(h, tot); /* the first of the carved buffers: the allocation */
   if (hb) return fail(h, LPG_ERR_INTERNAL, "running totals differ from a recount (mask 0x%x)", hb);
   return LPG_OK;
 }

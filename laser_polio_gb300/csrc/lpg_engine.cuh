@@ -114,7 +114,6 @@ typedef struct {
   const double* p_ri;
   const double* p_ipv;
   const double* strain_scal;
-  const double* net;   /* network[i][j], row-major */
   const uint64_t* netq_t; /* transposed, in two fixed-point parts: netq_t[j][i][0..1] = network[i][j] (lpg_net_split) */
   const double* rowsum;
   const double* r0s;
