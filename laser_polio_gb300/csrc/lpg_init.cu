@@ -8,13 +8,14 @@
  *     the capacity (lpg_init.h holds the arithmetic, shared with the oracle);
  *   - the choices without replacement (chronically missed, immune and
  *     initially infected agents) take, in each group, the k agents with the
- *     smallest counter-based 64-bit keys: a radix select on the keys' high
- *     32 bits in four 8-bit passes (a privatised shared-memory histogram per
- *     CTA tile, one thread per group to pick the digit), then one marking
- *     pass; the few agents whose high key bits equal the threshold are
- *     ordered by (full key, slot) on one thread per group.  The keys are
- *     recomputed from Philox in every pass instead of being stored, so the
- *     only scratch is per group.
+ *     smallest counter-based 64-bit keys, ties by slot.  Keys are uniform, so
+ *     the k-th smallest of n lies within a few sqrt(k (n - k) / n) / n of k / n:
+ *     one pass over the agents forms each key once, keeps a bit for the keys
+ *     below that window, counts them, and lists the few inside it; a CTA per
+ *     group picks the missing ones from its list; a last pass over the bits
+ *     marks.  Were the window to miss (it is 7 standard deviations either
+ *     side), the choice is made again with a wider one.  Scratch: a bit an
+ *     agent and 16 bytes a listed key.
  * Groups are whole nodes (the initial table is node-contiguous) or the whole
  * population.  Everything is HBM-light integer work: the passes are bound by
  * Philox arithmetic (about 140 integer instructions per key).  The timers
@@ -36,8 +37,7 @@ int lpg_ops_fail(int code, const char* fmt, ...);
 
 namespace {
 
-constexpr int kTile = 8192;  /* slots per CTA tile of the histogram passes */
-constexpr int kEqCap = 256;  /* keys per group whose high 32 bits may equal the threshold */
+constexpr int kTile = 8192; /* slots per CTA tile of the selection's pass */
 constexpr int kThreads = 256;
 
 struct SlotArgs {
@@ -64,125 +64,175 @@ __device__ __forceinline__ int32_t group_of(const int64_t* start, int32_t n, int
   return a;
 }
 
+/* The parts that fill constants and node ids, 16 slots a thread and step:
+ * one node search and 16-byte stores where the columns allow them. */
+__device__ __forceinline__ void fill_base(const SlotArgs& A, const lpg_columns& c, int64_t i0, bool wide) {
+  if (wide && i0 + 16 <= A.capacity && (i0 + 16 <= A.count || i0 >= A.count)) {
+    const bool live = i0 < A.count;
+    const uint4 zero = make_uint4(0, 0, 0, 0), ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+    *reinterpret_cast<uint4*>(c.disease_state + i0) = live ? zero : ones;
+    *reinterpret_cast<uint4*>(c.strain + i0) = zero;
+    *reinterpret_cast<uint4*>(c.potentially_paralyzed + i0) = ones;
+    *reinterpret_cast<uint4*>(c.paralyzed + i0) = zero;
+    *reinterpret_cast<uint4*>(c.ipv_protected + i0) = zero;
+    *reinterpret_cast<uint4*>(c.chronically_missed + i0) = zero;
+    uint32_t w[8];
+    if (!live) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = ~0u;
+    } else {
+      int32_t g = group_of(A.node_start, A.n_nodes, i0);
+      if (A.node_start[g + 1] >= i0 + 16) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = (uint32_t)g * 0x10001u;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t lo = (uint32_t)group_of(A.node_start, A.n_nodes, i0 + 2 * j);
+          w[j] = lo | (uint32_t)group_of(A.node_start, A.n_nodes, i0 + 2 * j + 1) << 16;
+        }
+      }
+    }
+    uint4* d = reinterpret_cast<uint4*>(c.node_id + i0);
+    d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    return;
+  }
+  for (int64_t i = i0; i < i0 + 16 && i < A.capacity; ++i) {
+    const bool live = i < A.count;
+    c.disease_state[i] = live ? 0 : -1;
+    c.node_id[i] = live ? (int16_t)group_of(A.node_start, A.n_nodes, i) : (int16_t)-1;
+    c.strain[i] = 0;
+    c.potentially_paralyzed[i] = -1;
+    c.paralyzed[i] = 0;
+    c.ipv_protected[i] = 0;
+    c.chronically_missed[i] = 0;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) k_init_base(SlotArgs A, lpg_columns c, bool wide) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x * 16;
+  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16; i0 < A.capacity; i0 += stride)
+    fill_base(A, c, i0, wide);
+}
+
 __global__ void __launch_bounds__(kThreads) k_init_slots(SlotArgs A, lpg_columns c, uint32_t parts) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.capacity; i += stride) {
-    const bool live = i < A.count;
-    if (parts & LPG_INIT_BASE) {
-      c.disease_state[i] = live ? 0 : -1;
-      c.node_id[i] = live ? (int16_t)group_of(A.node_start, A.n_nodes, i) : (int16_t)-1;
-      c.strain[i] = 0;
-      c.potentially_paralyzed[i] = -1;
-      c.paralyzed[i] = 0;
-      c.ipv_protected[i] = 0;
-      c.chronically_missed[i] = 0;
-    }
     if (parts & LPG_INIT_TIMERS)
       lpg_init_timers(A.seed, (uint64_t)i, A.k_exp, A.e1, A.e2, A.k_inf, A.i1, A.i2, A.k_par, A.p1, A.p2,
                       &c.exposure_timer[i], &c.infection_timer[i], &c.paralysis_timer[i]);
     if (parts & LPG_INIT_HETEROGENEITY)
       lpg_init_het(A.seed, (uint64_t)i, A.het, A.mu, A.sigma, A.rho, A.srho, A.scale, &c.acq_risk_multiplier[i],
                    &c.daily_infectivity[i]);
+  }
+}
+
+/* Dates of birth and death and RI dates.  Bound by Philox (a block each);
+ * with searches of seven steps in global memory and FP64 scaling 2.3e8 slots
+ * took 11.3 ms. */
+__global__ void __launch_bounds__(kThreads) k_init_dates(SlotArgs A, lpg_columns c, uint32_t parts) {
+  __shared__ FiDates D;
+  fi_dates_load(D, parts & LPG_INIT_AGES ? A.age_cum : nullptr, A.age_lo, A.age_hi, A.n_bins,
+                parts & LPG_INIT_DEATHS ? A.km : nullptr, A.km_len, A.km_max_year);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.capacity; i += stride) {
+    const bool live = i < A.count;
     int32_t dob = -1;
     if (parts & LPG_INIT_AGES) {
-      dob = live ? -lpg_init_age(A.seed, (uint64_t)i, A.n_bins, A.age_cum, A.age_lo, A.age_hi) : -1;
+      dob = live ? -fi_age(D, A.seed, (uint64_t)i) : -1;
       c.date_of_birth[i] = dob;
-    } else if (parts & (LPG_INIT_DEATHS | LPG_INIT_RI)) {
+    } else {
       dob = c.date_of_birth[i];
     }
     if (parts & LPG_INIT_DEATHS) {
       int32_t dod = 0;
       if (live) {
         const int64_t age = -(int64_t)dob;
-        const double u0 = lpg_u01(A.seed, LPG_P_INIT_KM, 0, (uint64_t)i, 0, 0);
-        const double u1 = lpg_u01(A.seed, LPG_P_INIT_KM, 0, (uint64_t)i, 0, 1);
-        dod = (int32_t)(lpg_km_age_at_death(A.km, A.km_len, A.km_max_year, age, u0, u1) - age);
+        uint64_t w[4] = {(uint64_t)i, 0, (uint64_t)LPG_P_INIT_KM << 32, 0};
+        lpg_philox4x64_10(w, A.seed, LPG_KEY_TAG);
+        dod = (int32_t)(fi_age_at_death(D, age, w[0] >> 11, w[1] >> 11) - age);
       }
       c.date_of_death[i] = dod;
     }
-    if (parts & LPG_INIT_RI) c.ri_timer[i] = live ? lpg_init_ri(A.seed, (uint64_t)i, dob) : (int16_t)-1;
+    if (parts & LPG_INIT_RI) c.ri_timer[i] = live ? fi_ri(A.seed, (uint64_t)i, dob) : (int16_t)-1;
   }
 }
 
 /* --- selection of k agents per group by their smallest keys ------------- */
+struct SelGroup {
+  int64_t start;     /* first agent; the next group's start ends it */
+  int64_t k;         /* <= 0: none, >= size: all */
+  uint64_t lo, hi;   /* keys below lo are taken, keys in [lo, hi] listed */
+  int64_t list, cap; /* the group's part of the list */
+};
+struct SelKey {
+  uint64_t key;
+  int64_t slot;
+};
 struct Sel {
   uint64_t seed;
   uint32_t purpose;
   int32_t n_groups;
-  const int64_t* start; /* [n_groups + 1] */
-  const int64_t* k;     /* [n_groups] */
-  uint32_t* prefix;     /* [n_groups] high key bits fixed so far */
-  int64_t* krem;        /* [n_groups] agents still to take among those matching the prefix */
-  uint32_t* hist;       /* [n_groups][256] */
-  uint32_t* eq_n;       /* [n_groups] */
-  int64_t* eq;          /* [n_groups][kEqCap] */
-  int* err;
+  const SelGroup* g;          /* [n_groups + 1] */
+  unsigned long long* below;  /* [n_groups] */
+  unsigned long long* listed; /* [n_groups] */
+  SelKey* list;
+  uint32_t* bits; /* one per agent */
+  int* err;       /* a window that missed */
 };
 
-__device__ __forceinline__ bool sel_active(const Sel& S, int32_t g) {
-  const int64_t n = S.start[g + 1] - S.start[g];
-  return S.k[g] > 0 && S.k[g] < n;
-}
-
-__device__ __forceinline__ uint32_t key_hi(const Sel& S, int64_t i) {
-  return (uint32_t)(lpg_raw(S.seed, S.purpose, 0, (uint64_t)i, 0, 0) >> 32);
-}
-
-__global__ void k_rsel_init(Sel S) {
-  for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < S.n_groups; g += gridDim.x * blockDim.x) {
-    S.prefix[g] = 0;
-    S.krem[g] = S.k[g];
-    S.eq_n[g] = 0;
-    for (int d = 0; d < 256; ++d) S.hist[(int64_t)g * 256 + d] = 0;
+__device__ __forceinline__ int32_t sel_group(const Sel& S, int64_t slot) {
+  int32_t a = 0, b = S.n_groups - 1;
+  while (a < b) {
+    const int32_t m = (a + b + 1) >> 1;
+    if (S.g[m].start <= slot) a = m; else b = m - 1;
   }
+  return a;
 }
 
-__global__ void __launch_bounds__(kThreads) k_rsel_hist(Sel S, int pass, int64_t count) {
-  __shared__ uint32_t h[256];
-  const int shift = 24 - 8 * pass;
+/* Bound by Philox (the 64-bit products: 2.1 ms for 2.2e8 blocks).  2.2e8
+ * agents in 774 nodes chosen and marked in 3.3 ms; four passes for the keys'
+ * digits and a marking one, a Philox block an agent each, took 14.6. */
+__global__ void __launch_bounds__(kThreads) k_rsel_pass(Sel S, int64_t count) {
+  const int lane = threadIdx.x & 31;
   for (int64_t t0 = (int64_t)blockIdx.x * kTile; t0 < count; t0 += (int64_t)gridDim.x * kTile) {
     const int64_t t1 = t0 + kTile < count ? t0 + kTile : count;
-    const int32_t g0 = group_of(S.start, S.n_groups, t0), g1 = group_of(S.start, S.n_groups, t1 - 1);
-    const bool priv = g0 == g1;
-    if (priv && !sel_active(S, g0)) continue; /* uniform over the CTA */
-    if (priv) {
-      for (int d = threadIdx.x; d < 256; d += blockDim.x) h[d] = 0;
-      __syncthreads();
-    }
-    for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
-      const int32_t g = priv ? g0 : group_of(S.start, S.n_groups, i);
-      if (!priv && !sel_active(S, g)) continue;
-      const uint32_t key = key_hi(S, i);
-      if (pass > 0 && (key >> (shift + 8)) != S.prefix[g]) continue;
-      const uint32_t d = (key >> shift) & 255u;
-      if (priv) atomicAdd(&h[d], 1u); else atomicAdd(&S.hist[(int64_t)g * 256 + d], 1u);
-    }
-    if (priv) {
-      __syncthreads();
-      for (int d = threadIdx.x; d < 256; d += blockDim.x)
-        if (h[d]) atomicAdd(&S.hist[(int64_t)g0 * 256 + d], h[d]);
-      __syncthreads();
-    }
-  }
-}
-
-/* the digit holding the krem-th smallest key of each group */
-__global__ void k_rsel_scan(Sel S) {
-  for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < S.n_groups; g += gridDim.x * blockDim.x) {
-    if (!sel_active(S, g)) continue;
-    uint32_t* h = S.hist + (int64_t)g * 256;
-    int64_t below = 0;
-    int digit = 255;
-    for (int d = 0; d < 256; ++d) {
-      if (below + (int64_t)h[d] >= S.krem[g]) {
-        digit = d;
-        break;
+    const int32_t g0 = sel_group(S, t0);
+    const bool one = S.g[g0 + 1].start >= t1; /* the tile lies in one group */
+    const SelGroup G0 = S.g[g0];
+    const int64_t n0 = S.g[g0 + 1].start - G0.start;
+    uint32_t below = 0;
+    for (int64_t i0 = t0 + (threadIdx.x & ~31); i0 < t1; i0 += blockDim.x) {
+      const int64_t i = i0 + lane;
+      bool take = false, inside = false;
+      int32_t g = g0;
+      uint64_t key = 0;
+      if (i < t1) {
+        if (!one) g = sel_group(S, i);
+        const int64_t k = one ? G0.k : S.g[g].k, n = one ? n0 : S.g[g + 1].start - S.g[g].start;
+        if (k >= n) {
+          take = true;
+        } else if (k > 0) {
+          key = lpg_raw(S.seed, S.purpose, 0, (uint64_t)i, 0, 0);
+          const uint64_t lo = one ? G0.lo : S.g[g].lo, hi = one ? G0.hi : S.g[g].hi;
+          take = key < lo;
+          inside = !take && key <= hi;
+          if (take && !one) atomicAdd(&S.below[g], 1ULL);
+        }
       }
-      below += h[d];
+      const uint32_t word = __ballot_sync(0xffffffffu, take);
+      if (lane == 0) {
+        S.bits[i0 >> 5] = word; /* tiles start at multiples of 32 */
+        below += __popc(word);
+      }
+      if (inside) {
+        const unsigned long long at = atomicAdd(&S.listed[g], 1ULL);
+        const SelGroup& G = S.g[g];
+        if ((int64_t)at < G.cap) S.list[G.list + at] = SelKey{key, i};
+      }
     }
-    S.prefix[g] = (S.prefix[g] << 8) | (uint32_t)digit;
-    S.krem[g] -= below;
-    for (int d = 0; d < 256; ++d) h[d] = 0;
+    if (one && lane == 0 && below && G0.k < n0) atomicAdd(&S.below[g0], (unsigned long long)below);
   }
 }
 
@@ -192,49 +242,83 @@ __device__ __forceinline__ void sel_apply(const lpg_columns& c, int action, int6
   else c.disease_state[i] = 2;
 }
 
-__global__ void __launch_bounds__(kThreads) k_rsel_mark(Sel S, lpg_columns c, int action, int64_t count) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-    const int32_t g = group_of(S.start, S.n_groups, i);
-    const int64_t n = S.start[g + 1] - S.start[g], k = S.k[g];
-    if (k <= 0) continue;
-    if (k >= n) {
-      sel_apply(c, action, i);
-      continue;
+/* One group a CTA: the need smallest (key, slot) of its list, by byte digits
+ * from the window's highest varying one. */
+__global__ void __launch_bounds__(kThreads) k_rsel_pick(Sel S) {
+  __shared__ uint32_t h[256];
+  __shared__ uint64_t s_prefix;
+  __shared__ int64_t s_need, s_slot;
+  __shared__ uint32_t s_same;
+  const int32_t g = blockIdx.x;
+  const SelGroup G = S.g[g];
+  const int64_t n = S.g[g + 1].start - G.start;
+  if (G.k <= 0 || G.k >= n) return;
+  const int64_t m = (int64_t)S.listed[g], need = G.k - (int64_t)S.below[g];
+  if (need < 0 || need > m || m > G.cap) {
+    if (threadIdx.x == 0) atomicOr(S.err, 1);
+    return;
+  }
+  if (need == 0) return;
+  const SelKey* L = S.list + G.list;
+  if (threadIdx.x == 0) {
+    s_prefix = 0;
+    s_need = need;
+    s_same = 0xffffffffu;
+  }
+  int shift = 64 - __clzll((long long)(G.hi - G.lo));
+  shift = shift > 8 ? shift - 8 : 0;
+  uint64_t fixed = 0; /* digits fixed so far: keys (less lo) that match s_prefix in the bits of `fixed` */
+  __syncthreads();
+  for (;;) {
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t prefix = s_prefix;
+    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) {
+      const uint64_t v = L[q].key - G.lo;
+      if ((v & fixed) == prefix) atomicAdd(&h[(v >> shift) & 255u], 1u);
     }
-    const uint32_t key = key_hi(S, i);
-    if (key < S.prefix[g]) {
-      sel_apply(c, action, i);
-    } else if (key == S.prefix[g]) {
-      const uint32_t q = atomicAdd(&S.eq_n[g], 1u);
-      if (q < (uint32_t)kEqCap) S.eq[(int64_t)g * kEqCap + q] = i;
-      else atomicOr(S.err, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int64_t want = s_need;
+      int d = 0;
+      while (d < 255 && want > (int64_t)h[d]) want -= h[d++];
+      s_need = want;
+      s_prefix = prefix | (uint64_t)d << shift;
+      s_same = h[d];
     }
+    __syncthreads();
+    fixed |= 255ULL << shift;
+    if (s_same == 1 || shift == 0) break;
+    shift = shift > 8 ? shift - 8 : 0;
+  }
+  /* the threshold's digits are s_prefix; of the s_same keys that share them
+   * the s_need smallest are taken: all, unless whole keys are equal, when the
+   * slots decide */
+  const uint64_t prefix = s_prefix;
+  if ((uint64_t)s_need < s_same) {
+    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) {
+      if (((L[q].key - G.lo) & fixed) != prefix) continue;
+      int64_t rank = 0;
+      for (int64_t p = 0; p < m; ++p)
+        rank += ((L[p].key - G.lo) & fixed) == prefix && L[p].slot < L[q].slot ? 1 : 0;
+      if (rank == s_need - 1) s_slot = L[q].slot;
+    }
+  } else if (threadIdx.x == 0) {
+    s_slot = INT64_MAX;
+  }
+  __syncthreads();
+  for (int64_t q = threadIdx.x; q < m; q += blockDim.x) {
+    const uint64_t v = (L[q].key - G.lo) & fixed;
+    if (v < prefix || (v == prefix && L[q].slot <= s_slot)) atomicOr(&S.bits[L[q].slot >> 5], 1u << (L[q].slot & 31));
   }
 }
 
-/* among the agents whose high key bits equal the threshold, the krem first
- * by (full key, slot) */
-__global__ void k_rsel_ties(Sel S, lpg_columns c, int action) {
-  for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < S.n_groups; g += gridDim.x * blockDim.x) {
-    if (!sel_active(S, g)) continue;
-    const int n = (int)(S.eq_n[g] < (uint32_t)kEqCap ? S.eq_n[g] : (uint32_t)kEqCap);
-    int64_t* e = S.eq + (int64_t)g * kEqCap;
-    for (int a = 1; a < n; ++a) { /* insertion sort by (key, slot) */
-      const int64_t v = e[a];
-      const uint64_t kv = lpg_raw(S.seed, S.purpose, 0, (uint64_t)v, 0, 0);
-      int b = a - 1;
-      while (b >= 0) {
-        const uint64_t kb = lpg_raw(S.seed, S.purpose, 0, (uint64_t)e[b], 0, 0);
-        if (kb < kv || (kb == kv && e[b] < v)) break;
-        e[b + 1] = e[b];
-        --b;
-      }
-      e[b + 1] = v;
-    }
-    const int64_t take = S.krem[g] < n ? S.krem[g] : n;
-    for (int64_t j = 0; j < take; ++j) sel_apply(c, action, e[j]);
-  }
+__global__ void __launch_bounds__(kThreads) k_rsel_mark(const uint32_t* __restrict__ bits, lpg_columns c, int action, int64_t count) {
+  const int64_t words = (count + 31) / 32, stride = (int64_t)gridDim.x * (kThreads / 32);
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int64_t w = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); w < words; w += stride)
+    if (bits[w] >> lane & 1u) sel_apply(c, action, w * 32 + lane);
 }
 
 #define CKI(x)                                                                              \
@@ -285,45 +369,53 @@ int grid_for(int64_t n, int per_block) {
 int select_k(Scratch& sc, cudaStream_t st, const lpg_columns& c, uint64_t seed, uint32_t purpose, int action,
              const std::vector<int64_t>& start, const std::vector<int64_t>& k, int64_t count) {
   const int32_t G = (int32_t)k.size();
+  bool any = false;
+  for (int32_t g = 0; g < G; ++g) any = any || (k[g] > 0 && start[g + 1] > start[g]);
+  if (!any) return 0;
   Sel S{};
   S.seed = seed;
   S.purpose = purpose;
   S.n_groups = G;
-  int64_t *d_start, *d_k, *krem, *eq;
-  uint32_t *prefix, *hist, *eq_n;
-  int* err;
-  int rc = sc.upload(&d_start, start);
-  if (!rc) rc = sc.upload(&d_k, k);
-  if (!rc) rc = sc.alloc(&prefix, (size_t)G);
-  if (!rc) rc = sc.alloc(&krem, (size_t)G);
-  if (!rc) rc = sc.alloc(&hist, (size_t)G * 256);
-  if (!rc) rc = sc.alloc(&eq_n, (size_t)G);
-  if (!rc) rc = sc.alloc(&eq, (size_t)G * kEqCap);
-  if (!rc) rc = sc.alloc(&err, 1);
+  std::vector<SelGroup> groups(G + 1);
+  const size_t words = (size_t)(count + 31) / 32;
+  unsigned long long* counters;
+  int rc = sc.alloc(&S.bits, words);
+  if (!rc) rc = sc.alloc(&counters, 2 * (size_t)G + 1);
   if (rc) return rc;
-  S.start = d_start;
-  S.k = d_k;
-  S.prefix = prefix;
-  S.krem = krem;
-  S.hist = hist;
-  S.eq_n = eq_n;
-  S.eq = eq;
-  S.err = err;
-  CKI(cudaMemsetAsync(err, 0, sizeof(int), st));
-  const int gb = (G + 255) / 256;
-  k_rsel_init<<<gb, 256, 0, st>>>(S);
-  const int tiles = grid_for(count, kTile);
-  for (int pass = 0; pass < 4; ++pass) {
-    k_rsel_hist<<<tiles, kThreads, 0, st>>>(S, pass, count);
-    k_rsel_scan<<<gb, 256, 0, st>>>(S);
+  S.below = counters;
+  S.listed = counters + G;
+  S.err = reinterpret_cast<int*>(counters + 2 * (size_t)G);
+  for (double wide = 7.0;; wide *= 8.0) {
+    int64_t total = 0;
+    for (int32_t g = 0; g < G; ++g) {
+      SelGroup& q = groups[g];
+      const int64_t n = start[g + 1] - start[g];
+      q = SelGroup{start[g], k[g], 0, ~0ULL, total, 0};
+      if (k[g] <= 0 || k[g] >= n) continue;
+      const double dn = (double)n, dk = (double)k[g], sd = std::sqrt(dk * (dn - dk) / dn) + 1.0;
+      const double lo = (dk - wide * sd) / dn, hi = (dk + wide * sd) / dn;
+      if (lo > 0.0) q.lo = (uint64_t)(lo * 18446744073709551616.0);
+      if (hi < 1.0) q.hi = (uint64_t)(hi * 18446744073709551616.0);
+      const double cap = (2.0 * wide + 8.0) * sd + 64.0;
+      q.cap = cap < dn ? (int64_t)cap : n;
+      total += q.cap;
+    }
+    groups[G] = SelGroup{start[G], 0, 0, 0, total, 0};
+    SelGroup* d_groups;
+    if ((rc = sc.upload(&d_groups, groups)) || (rc = sc.alloc(&S.list, (size_t)total))) return rc;
+    S.g = d_groups;
+    CKI(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (2 * (size_t)G + 1), st));
+    k_rsel_pass<<<grid_for(count, kTile), kThreads, 0, st>>>(S, count);
+    k_rsel_pick<<<G, kThreads, 0, st>>>(S);
+    CKI(cudaGetLastError());
+    int h_err = 0;
+    CKI(cudaMemcpyAsync(&h_err, S.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CKI(cudaStreamSynchronize(st));
+    if (!h_err) break;
+    if (wide > 1e12) return lpg_ops_fail(LPG_ERR_INTERNAL, "init: a selection window cannot miss every key");
   }
-  k_rsel_mark<<<grid_for(count, kThreads * 4), kThreads, 0, st>>>(S, c, action, count);
-  k_rsel_ties<<<gb, 256, 0, st>>>(S, c, action);
+  k_rsel_mark<<<grid_for(count, kThreads * 4), kThreads, 0, st>>>(S.bits, c, action, count);
   CKI(cudaGetLastError());
-  int h_err = 0;
-  CKI(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CKI(cudaStreamSynchronize(st));
-  if (h_err) return lpg_ops_fail(LPG_ERR_INTERNAL, "init: more than %d keys tie at a selection threshold", kEqCap);
   return 0;
 }
 
@@ -506,6 +598,21 @@ extern "C" int lpg_init_columns(const lpg_init_desc* d, uint32_t parts, const lp
   uint32_t slot_parts =
       parts & (LPG_INIT_BASE | LPG_INIT_TIMERS | LPG_INIT_HETEROGENEITY | LPG_INIT_AGES | LPG_INIT_DEATHS | LPG_INIT_RI);
   if ((rc = fill_fast(sc, st, *d, A, c, &slot_parts))) return rc;
+  if ((slot_parts & LPG_INIT_BASE) && d->capacity > 0) {
+    const void* ps[] = {c.disease_state, c.node_id, c.strain, c.potentially_paralyzed, c.paralyzed, c.ipv_protected,
+                        c.chronically_missed};
+    bool wide = true;
+    for (const void* q : ps) wide = wide && ((uintptr_t)q & 15u) == 0;
+    k_init_base<<<grid_for(d->capacity, kThreads * 16), kThreads, 0, st>>>(A, c, wide);
+    CKI(cudaGetLastError());
+    slot_parts &= ~(uint32_t)LPG_INIT_BASE;
+  }
+  const uint32_t dates = slot_parts & (LPG_INIT_AGES | LPG_INIT_DEATHS | LPG_INIT_RI);
+  if (dates && d->capacity > 0) {
+    k_init_dates<<<grid_for(d->capacity, kThreads * 8), kThreads, 0, st>>>(A, c, dates);
+    CKI(cudaGetLastError());
+    slot_parts &= ~dates;
+  }
   if (slot_parts && d->capacity > 0) {
     k_init_slots<<<grid_for(d->capacity, kThreads * 8), kThreads, 0, st>>>(A, c, slot_parts);
     CKI(cudaGetLastError());

@@ -503,6 +503,129 @@ __global__ void __launch_bounds__(FI_THREADS) k_init_het_fast(FiHet A) {
   }
 }
 
+/* --- dates: the FP64 definitions' integers by integer arithmetic ------------- */
+/* floor(u * span) as FP64 gives it, u = m 2^-53 and 0 <= span < 2^31: the
+ * exact product's floor, unless the product lies so close below a whole
+ * number (2^-21) that its rounding to 53 bits may reach it. */
+__device__ __forceinline__ int64_t fi_scaled_floor(uint64_t m, int64_t span) {
+  const uint64_t a = m << 11, lo = a * (uint64_t)span;
+  if ((lo >> 43) == 0x1fffff || (uint64_t)span >> 31)
+    return (int64_t)floor((double)m * 0x1.0p-53 * (double)span);
+  return (int64_t)__umul64hi(a, (uint64_t)span);
+}
+
+/* The date tables of a CTA, in shared memory where they fit (FI_TABLE
+ * entries), with guides: the first entry that a draw of the bucket can
+ * reach, so that a search is one or two steps and not seven. */
+#define FI_TABLE 256
+#define FI_GUIDE 256
+struct FiDates {
+  const int64_t *cum, *km;
+  const int32_t *lo, *hi;
+  int32_t n_bins, km_len, km_max_year;
+  int64_t s_cum[FI_TABLE], s_km[FI_TABLE];
+  int32_t s_lo[FI_TABLE], s_hi[FI_TABLE];
+  uint16_t age_guide[FI_GUIDE], km_guide[FI_GUIDE];
+  float km_scale; /* buckets per death */
+};
+
+__device__ __forceinline__ int32_t fi_first_above(const int64_t* cum, int32_t n, int64_t v) {
+  int32_t a = 0, b = n;
+  while (a < b) {
+    const int32_t m = (a + b) >> 1;
+    if (cum[m] > v) b = m; else a = m + 1;
+  }
+  return a;
+}
+
+/* All threads of the CTA; the guides hold for tables of fewer than 65536
+ * entries (start at entry 0 otherwise). */
+__device__ __forceinline__ void fi_dates_load(FiDates& D, const int64_t* cum, const int32_t* lo, const int32_t* hi,
+                                              int32_t n_bins, const int64_t* km, int32_t km_len, int32_t km_max_year) {
+  const bool ages = cum != nullptr, deaths = km != nullptr;
+  if (threadIdx.x == 0) {
+    D.n_bins = n_bins;
+    D.km_len = km_len;
+    D.km_max_year = km_max_year;
+    D.cum = n_bins <= FI_TABLE ? D.s_cum : cum;
+    D.lo = n_bins <= FI_TABLE ? D.s_lo : lo;
+    D.hi = n_bins <= FI_TABLE ? D.s_hi : hi;
+    D.km = km_len <= FI_TABLE ? D.s_km : km;
+  }
+  if (ages && n_bins <= FI_TABLE)
+    for (int q = threadIdx.x; q < n_bins; q += blockDim.x) {
+      D.s_cum[q] = cum[q];
+      D.s_lo[q] = lo[q];
+      D.s_hi[q] = hi[q];
+    }
+  if (deaths && km_len <= FI_TABLE)
+    for (int q = threadIdx.x; q < km_len; q += blockDim.x) D.s_km[q] = km[q];
+  __syncthreads();
+  const int32_t top = km_max_year < km_len - 1 ? km_max_year : km_len - 1;
+  for (int b = threadIdx.x; b < FI_GUIDE; b += blockDim.x) {
+    if (ages) {
+      /* bucket b: the uniform's top 8 bits */
+      const uint64_t v = lpg_scale_target((uint64_t)b << 45, (uint64_t)cum[n_bins - 1]);
+      D.age_guide[b] = n_bins < 65536 ? (uint16_t)fi_first_above(D.cum, n_bins - 1, (int64_t)v) : 0;
+    }
+    if (deaths) {
+      /* bucket b: draws from (b - 1) / 256 of the total on, a bucket's slack for the FP32 scaling */
+      const int64_t total = top >= 0 ? km[top] : 0;
+      const int64_t from = b > 0 && total > 0 ? (int64_t)((double)total * (b - 1) / FI_GUIDE) : INT64_MIN;
+      D.km_guide[b] = top >= 0 && km_len < 65536 ? (uint16_t)fi_first_above(D.km, top + 1, from) : 0;
+      if (b == 0) D.km_scale = total > 0 ? (float)FI_GUIDE / (float)total : 0.0f;
+    }
+  }
+  __syncthreads();
+}
+
+/* lpg_init_age */
+__device__ __forceinline__ int32_t fi_age(const FiDates& D, uint64_t seed, uint64_t slot) {
+  uint64_t w[4] = {slot, 0, (uint64_t)LPG_P_INIT_AGE << 32, 0};
+  lpg_philox4x64_10(w, seed, LPG_KEY_TAG);
+  const uint64_t m = w[0] >> 11;
+  const int64_t v = (int64_t)lpg_scale_target(m, (uint64_t)D.cum[D.n_bins - 1]);
+  int32_t a = D.age_guide[m >> 45]; /* first bin with cum > v */
+  while (a < D.n_bins - 1 && D.cum[a] <= v) ++a;
+  const int32_t age = D.lo[a] + (int32_t)fi_scaled_floor(w[1] >> 11, D.hi[a] - D.lo[a]);
+  return age < 1 ? 1 : age;
+}
+
+/* lpg_km_age_at_death from the 53-bit integers of its uniforms */
+__device__ __forceinline__ int32_t fi_age_at_death(const FiDates& D, int64_t age_days, uint64_t m0, uint64_t m1) {
+  const int32_t top = D.km_max_year < D.km_len - 1 ? D.km_max_year : D.km_len - 1;
+  int64_t years = age_days >> 30 ? age_days / 365 : (int64_t)((int32_t)age_days / 365);
+  if (years > top) years = top;
+  const int64_t lower = years > 0 ? D.km[years - 1] : 0;
+  const int64_t total = D.km[top];
+  const int64_t span = total - lower > 0 ? total - lower : 0;
+  int64_t y = top;
+  if (span > 0) {
+    const int64_t draw = lower + fi_scaled_floor(m0, span);
+    const float at = (float)draw * D.km_scale;
+    int32_t a = D.km_guide[at <= 0.0f ? 0 : at < (float)(FI_GUIDE - 1) ? (int)at : FI_GUIDE - 1];
+    while (a <= top && D.km[a] <= draw) ++a; /* first index with cum > draw, top + 1 if none */
+    y = a > years ? a : years;
+    if (y > top) y = top;
+  }
+  const int64_t day_lo = y == years ? age_days : y * 365;
+  int64_t day_hi = (y + 1) * 365;
+  if (day_hi < day_lo + 1) day_hi = day_lo + 1;
+  return (int32_t)(day_lo + fi_scaled_floor(m1, day_hi - day_lo));
+}
+
+/* lpg_init_ri: dob + (42 + 56 u) truncated.  The FP64 sum is within 2^-20 of
+ * the exact one; a fraction that close to a whole day is left to FP64. */
+__device__ __forceinline__ int16_t fi_ri(uint64_t seed, uint64_t slot, int32_t dob) {
+  const uint64_t m = lpg_u53(seed, LPG_P_INIT_RI, 0, slot, 0, 0);
+  const uint64_t days = 56 * m; /* 53 fraction bits */
+  const uint32_t f = (uint32_t)(days >> 21) /* 32 fraction bits */;
+  const int64_t v = (int64_t)dob + 42 + (int64_t)(days >> 53);
+  if (f < 0x2000u || f > 0xffffdfffu || v > 0x7ffffff0) return lpg_init_ri(seed, slot, dob);
+  const int32_t d = (int32_t)(v < 0 ? v + 1 : v); /* towards zero, never whole */
+  return (int16_t)(uint16_t)(uint32_t)d;
+}
+
 /* --- the slots left to FP64 -------------------------------------------------- */
 struct FiExact {
   uint64_t seed;

@@ -22,13 +22,15 @@ TIMERS = [
 HET = [(4.0, 0.8), (float(np.exp(0.64) - 1.0), -0.9), (0.0, 0.5), (1e-3, 1.0), (1e8, 0.3)]
 
 
-def _both(capacity, parts, fields):
+def _both(capacity, parts, fields, pops=None):
     from oracle_backend import oracle_fill
 
     out = []
     for fill in (dinit.fill, oracle_fill):
-        people = LaserFrame(capacity=capacity, initial_count=capacity)
-        spec = dinit.InitSpec(7, np.array([capacity]), capacity, capacity)
+        node_pop = np.array([capacity]) if pops is None else np.asarray(pops)
+        count = int(node_pop.sum())
+        people = LaserFrame(capacity=capacity, initial_count=count)
+        spec = dinit.InitSpec(7, node_pop, count, capacity)
         for k, v in fields.items():
             setattr(spec, k, v)
         fill(people, spec, parts)
@@ -50,3 +52,33 @@ def test_gpu_timers_equal_the_fp64_definition(exp, inf, par, capacity):
 def test_gpu_heterogeneity_equals_the_fp64_definition(var, corr, capacity):
     _both(capacity, _abi.INIT_HETEROGENEITY, {"risk_mult_var": var, "corr_risk_inf": corr, "r0": 14.0,
                                               "dur_inf": (GAMMA, 4.51, 5.32), "heterogeneity": 1})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pops", [[1], [31, 0, 1, 32, 33], [8191, 1, 8193], [40_000, 7, 0, 60_001], [300] * 200])
+def test_gpu_choices_and_node_ids(pops):
+    """Tiles of 8192 agents, words of 32, windows that cover a whole small
+    node; none, one, all but one and all of a node."""
+    n = np.asarray(pops)
+    cap = int(n.sum()) + 21
+    rng = np.random.default_rng(len(pops))
+    for k in (np.zeros_like(n), np.minimum(n, 1), np.maximum(n - 1, 0), n, rng.integers(0, n + 1)):
+        _both(cap, _abi.INIT_BASE | _abi.INIT_IMMUNITY, {"immune_k": k}, pops)
+    for k in (0, 1, int(n.sum()) // 3, int(n.sum())):
+        _both(cap, _abi.INIT_BASE | _abi.INIT_MISSED, {"missed_k": k}, pops)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bins,deaths", [(1, 1), (17, 101), (256, 256), (257, 400)])
+def test_gpu_dates(bins, deaths):
+    """Tables within and beyond shared memory's 256 entries, empty bins and
+    years, totals of more than 2^31 deaths."""
+    rng = np.random.default_rng(bins)
+    lo = np.cumsum(rng.integers(1, 90, bins)).astype(np.int32)
+    w = rng.integers(0, 3, bins).astype(np.int64)
+    w[-1] = 1
+    fields = {"age_lo": lo, "age_hi": lo + rng.integers(1, 400, bins).astype(np.int32), "age_weight": w,
+              "km_max_year": 300}
+    for scale in (1, 10**8):
+        fields["km"] = np.cumsum(rng.integers(0, 2, deaths) * scale).astype(np.int64)
+        _both(50_021, _abi.INIT_BASE | _abi.INIT_AGES | _abi.INIT_DEATHS | _abi.INIT_RI, fields, [30_000, 20_000])
