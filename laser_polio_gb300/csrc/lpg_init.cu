@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "lpg.h"
@@ -327,31 +328,88 @@ __global__ void __launch_bounds__(kThreads) k_rsel_mark(const uint32_t* __restri
     if (e_ != cudaSuccess) return lpg_ops_fail(LPG_ERR_CUDA, "init: %s", cudaGetErrorString(e_)); \
   } while (0)
 
-/* Device scratch freed on the stream when it goes out of scope. */
+/* A thread's workspace on a device, kept for its next call: a small table's
+ * initialisation is five calls of some 50 us of kernels each, and an
+ * allocation with its free costs 0.2 ms (the stream-ordered pool, which gives
+ * its memory back at every synchronisation, the same).  4 MB at most a thread
+ * and device, freed when the thread ends.  A call has its stream finish
+ * before it returns, so the next one may use any stream. */
+constexpr size_t kWorkBytes = 4 << 20, kTableBytes = 1 << 18;
+struct Workspace {
+  int device;
+  uint8_t* dev;
+  std::vector<uint8_t> host; /* the tables, as they go up */
+};
+struct Workspaces {
+  std::vector<Workspace> all;
+  ~Workspaces() {
+    for (auto& w : all) cudaFree(w.dev);
+  }
+  Workspace* get() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    for (auto& w : all)
+      if (w.device == device) return &w;
+    Workspace w{device, nullptr, std::vector<uint8_t>(kTableBytes)};
+    if (cudaMalloc((void**)&w.dev, kWorkBytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    all.push_back(std::move(w));
+    return &all.back();
+  }
+};
+thread_local Workspaces t_workspaces;
+
+/* A call's device scratch: tables first, which go up with one copy
+ * (ready()), then buffers, in the thread's workspace as far as it reaches and
+ * allocated beyond. */
 struct Scratch {
   cudaStream_t st;
   std::vector<void*> ptrs;
-  explicit Scratch(cudaStream_t s) : st(s) {}
+  Workspace* w;
+  size_t used = 0, sent = 0, taken = kTableBytes;
+  explicit Scratch(cudaStream_t s) : st(s), w(t_workspaces.get()) {}
   ~Scratch() {
-    for (void* p : ptrs) cudaFreeAsync(p, st);
+    cudaStreamSynchronize(st);
+    for (void* p : ptrs) cudaFree(p);
   }
   template <class T>
   int alloc(T** out, size_t n) {
-    void* p = nullptr;
-    if (cudaMallocAsync(&p, (n ? n : 1) * sizeof(T), st) != cudaSuccess) {
-      cudaGetLastError();
-      return lpg_ops_fail(LPG_ERR_NOMEM, "init: device scratch of %zu bytes", n * sizeof(T));
+    const size_t bytes = (n ? n : 1) * sizeof(T), room = (bytes + 255) & ~(size_t)255;
+    if (w && taken + room <= kWorkBytes) {
+      *out = (T*)(w->dev + taken);
+      taken += room;
+      return 0;
     }
-    ptrs.push_back(p);
-    *out = (T*)p;
+    if (cudaMalloc((void**)out, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return lpg_ops_fail(LPG_ERR_NOMEM, "init: device scratch of %zu bytes", bytes);
+    }
+    ptrs.push_back(*out);
     return 0;
   }
   template <class T>
   int upload(T** out, const std::vector<T>& v) {
-    int rc = alloc(out, v.size());
-    if (rc) return rc;
-    if (cudaMemcpyAsync(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st) != cudaSuccess)
+    const size_t bytes = v.size() * sizeof(T), room = (bytes + 255) & ~(size_t)255;
+    if (!w || used + room > kTableBytes) {
+      const int rc = alloc(out, v.size());
+      if (rc) return rc;
+      if (cudaMemcpyAsync(*out, v.data(), bytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
+        return lpg_ops_fail(LPG_ERR_CUDA, "init: upload");
+      return 0;
+    }
+    *out = (T*)(w->dev + used);
+    if (bytes) memcpy(w->host.data() + used, v.data(), bytes);
+    used += room;
+    return 0;
+  }
+  /* before a kernel that reads what was uploaded */
+  int ready() {
+    if (used > sent &&
+        cudaMemcpyAsync(w->dev + sent, w->host.data() + sent, used - sent, cudaMemcpyHostToDevice, st) != cudaSuccess)
       return lpg_ops_fail(LPG_ERR_CUDA, "init: upload");
+    sent = used;
     return 0;
   }
 };
@@ -378,10 +436,10 @@ int select_k(Scratch& sc, cudaStream_t st, const lpg_columns& c, uint64_t seed, 
   S.n_groups = G;
   std::vector<SelGroup> groups(G + 1);
   const size_t words = (size_t)(count + 31) / 32;
-  unsigned long long* counters;
-  int rc = sc.alloc(&S.bits, words);
-  if (!rc) rc = sc.alloc(&counters, 2 * (size_t)G + 1);
+  unsigned long long* counters; /* then the bits */
+  int rc = sc.alloc(&counters, 2 * (size_t)G + 2 + (words + 1) / 2);
   if (rc) return rc;
+  S.bits = reinterpret_cast<uint32_t*>(counters + 2 * (size_t)G + 2);
   S.below = counters;
   S.listed = counters + G;
   S.err = reinterpret_cast<int*>(counters + 2 * (size_t)G);
@@ -402,7 +460,7 @@ int select_k(Scratch& sc, cudaStream_t st, const lpg_columns& c, uint64_t seed, 
     }
     groups[G] = SelGroup{start[G], 0, 0, 0, total, 0};
     SelGroup* d_groups;
-    if ((rc = sc.upload(&d_groups, groups)) || (rc = sc.alloc(&S.list, (size_t)total))) return rc;
+    if ((rc = sc.upload(&d_groups, groups)) || (rc = sc.alloc(&S.list, (size_t)total)) || (rc = sc.ready())) return rc;
     S.g = d_groups;
     CKI(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (2 * (size_t)G + 1), st));
     k_rsel_pass<<<grid_for(count, kTile), kThreads, 0, st>>>(S, count);
@@ -449,6 +507,7 @@ int fill_fast(Scratch& sc, cudaStream_t st, const lpg_init_desc& d, const SlotAr
       }
     }
     if (ok) {
+      if ((rc = sc.ready())) return rc;
       F.seed = d.seed;
       F.capacity = d.capacity;
       F.et = c.exposure_timer;
@@ -472,9 +531,9 @@ int fill_fast(Scratch& sc, cudaStream_t st, const lpg_init_desc& d, const SlotAr
   if ((*parts & LPG_INIT_HETEROGENEITY) && A.het && A.sigma > 0.01 && A.sigma < 4.0 && A.scale < 1e6) {
     static const FiTables* host = fi_tables(); /* constants, formed once */
     FiTables* tab;
-    int rc = sc.alloc(&tab, 1);
+    int rc = sc.upload(&tab, std::vector<FiTables>(1, *host));
+    if (!rc) rc = sc.ready();
     if (rc) return rc;
-    CKI(cudaMemcpyAsync(tab, host, sizeof(FiTables), cudaMemcpyHostToDevice, st));
     FiHet H{d.seed, d.capacity, fi_pair(A.mu), fi_pair(A.sigma), fi_pair(A.rho), fi_pair(A.srho), fi_pair(A.scale),
             tab, c.acq_risk_multiplier, c.daily_infectivity};
     k_init_het_fast<<<grid, FI_THREADS, 0, st>>>(H);
@@ -540,9 +599,11 @@ extern "C" int lpg_init_columns(const lpg_init_desc* d, uint32_t parts, const lp
   A.count = d->count;
   A.capacity = d->capacity;
   A.n_nodes = n;
-  int64_t* d_start;
-  if ((rc = sc.upload(&d_start, start))) return rc;
-  A.node_start = d_start;
+  if (parts & LPG_INIT_BASE) {
+    int64_t* d_start;
+    if ((rc = sc.upload(&d_start, start))) return rc;
+    A.node_start = d_start;
+  }
   A.k_exp = d->dur_exp.kind;
   A.e1 = d->dur_exp.p1;
   A.e2 = d->dur_exp.p2;
@@ -603,17 +664,20 @@ extern "C" int lpg_init_columns(const lpg_init_desc* d, uint32_t parts, const lp
                         c.chronically_missed};
     bool wide = true;
     for (const void* q : ps) wide = wide && ((uintptr_t)q & 15u) == 0;
+    if ((rc = sc.ready())) return rc;
     k_init_base<<<grid_for(d->capacity, kThreads * 16), kThreads, 0, st>>>(A, c, wide);
     CKI(cudaGetLastError());
     slot_parts &= ~(uint32_t)LPG_INIT_BASE;
   }
   const uint32_t dates = slot_parts & (LPG_INIT_AGES | LPG_INIT_DEATHS | LPG_INIT_RI);
   if (dates && d->capacity > 0) {
+    if ((rc = sc.ready())) return rc;
     k_init_dates<<<grid_for(d->capacity, kThreads * 8), kThreads, 0, st>>>(A, c, dates);
     CKI(cudaGetLastError());
     slot_parts &= ~dates;
   }
   if (slot_parts && d->capacity > 0) {
+    if ((rc = sc.ready())) return rc;
     k_init_slots<<<grid_for(d->capacity, kThreads * 8), kThreads, 0, st>>>(A, c, slot_parts);
     CKI(cudaGetLastError());
   }

@@ -38,6 +38,7 @@ PART_COLUMNS = {
     _abi.INIT_RI: ("date_of_birth", "ri_timer"),
 }
 COLUMN_DTYPES = {name: dtype for name, _, dtype in _abi.COLUMN_FIELDS}
+COLUMN_POINTERS = {name: ptr for name, ptr, _ in _abi.COLUMN_FIELDS}
 
 
 def part_columns(parts: int):
@@ -203,7 +204,7 @@ def fill(people, spec: InitSpec, parts: int) -> None:
             tensors[name] = torch.empty(spec.capacity, dtype=tdt, device="cuda")
     cols = _abi.lpg_columns()
     for name, t in tensors.items():
-        setattr(cols, name, C.cast(C.c_void_p(t.data_ptr()), dict((n, p) for n, p, _ in _abi.COLUMN_FIELDS)[name]))
+        setattr(cols, name, C.cast(C.c_void_p(t.data_ptr()), COLUMN_POINTERS[name]))
     desc, _keep = spec.desc()
     lib = _lib.load()
     stream = torch.cuda.current_stream().cuda_stream
