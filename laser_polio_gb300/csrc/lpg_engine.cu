@@ -732,6 +732,9 @@ extern "C" int lpg_bind_columns(lpg_handle* h, int32_t sim, const lpg_columns* c
 
 static int launch_tick(lpg_handle* h, uint8_t need, int* n_launched);
 
+/* k_sel_round0's dynamic shared memory: the target offsets, while they fit. */
+static size_t sel_smem(int G) { return G < LPG_SEL_NODES ? sizeof(int64_t) * ((size_t)G + 1) : 0; }
+
 extern "C" int lpg_start(lpg_handle* h) {
   if (!h) return LPG_ERR_ARG;
   if (h->started) return LPG_OK;
@@ -834,6 +837,7 @@ extern "C" int lpg_start(lpg_handle* h) {
   carve.add(&W.evt, P);
   carve.add(&W.rdt, P);
   carve.add(&W.ref, P);
+  carve.add(&W.sel_done, 1);
   carve.add(&W.cmeta, chunk_total);
   carve.add(&W.qcnt, 2048);
   carve.add(&W.qfirst, 2048);
@@ -912,6 +916,7 @@ extern "C" int lpg_start(lpg_handle* h) {
   CK(cudaMemsetAsync(W.bb, 0, sizeof(uint64_t) * LPG_MAX_STRAINS * G, st));
   CK(cudaMemsetAsync(W.size, 0, sizeof(int64_t) * G, st));
   CK(cudaMemsetAsync(W.uniq, 0, sizeof(int64_t) * G, st));
+  CK(cudaMemsetAsync(W.sel_done, 0, sizeof(int32_t), st));
   CK(cudaMemsetAsync(W.ctr, 0, sizeof(unsigned long long) * LPG_NUM_COUNTERS, st));
   CK(cudaMemsetAsync(W.end_done, 0, 4, st));
   CK(cudaMemsetAsync(W.grid_bar, 0, 8, st));
@@ -1171,7 +1176,8 @@ extern "C" int lpg_start(lpg_handle* h) {
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, R > 1 && R <= LPG_DUE_FLAT ? k_due<true> : k_due<false>, 256, 0));
   h->due_blocks = std::max(1, occ) * h->sm_count;
   occ = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sel_round0, 256, 0));
+  CK(cudaFuncSetAttribute(k_sel_round0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem(LPG_SEL_NODES - 1)));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sel_round0, 256, sel_smem(G)));
   if (occ < 1) return fail(h, LPG_ERR_CUDA, "k_sel_round0 does not fit on an SM");
   h->round0_max = occ * h->sm_count;
   h->select_blocks = h->round0_max;
@@ -1237,7 +1243,8 @@ static int launch_one(lpg_handle* h, int k, bool timed) {
     case 9: {
       /* cooperative: its CTAs meet at a grid barrier, so all must be resident */
       void* args[] = {&W};
-      CK(cudaLaunchCooperativeKernel((const void*)k_sel_round0, dim3(h->select_blocks), dim3(256), args, 0, st));
+      CK(cudaLaunchCooperativeKernel((const void*)k_sel_round0, dim3(h->select_blocks), dim3(256), args,
+                                     sel_smem(G), st));
       break;
     }
     case 10: CK(launch_pdl(k_sel_rounds, dim3(h->rounds_blocks), dim3(256), 0, st, W)); break;

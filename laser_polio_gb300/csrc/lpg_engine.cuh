@@ -209,6 +209,7 @@ typedef struct {
   int64_t* tgt_off; /* [G + 1] */
   void* sel_info;     /* [G] SelInfo: per-node selection record of the tick */
   uint32_t* hits; /* selection targets */
+  int32_t* sel_done; /* rounds of the tick's selection that k_sel_round0 made */
   int64_t hits_cap;
   uint64_t* evq;     /* event queues of the sweeps: one slab per sweep CTA */
   uint32_t* qcnt;    /* [2][1024] entries per slab (k_sweep_due, k_sweep_rs) */

@@ -36,14 +36,17 @@
 
 #define FULLMASK 0xffffffffu
 #define LPG_NONE 0xffffffffu
-/* State byte of an agent claimed by a round-0 target of this tick while the
+/* State byte of an agent claimed by a target of k_sel_round0 while the
  * round is still running: the round's other targets locate on the frozen
  * CDF, so they still count it as susceptible; k_sel_round0 makes it exposed
  * (1) after its grid barrier.  No other kernel sees it. */
 #define LPG_DS_CLAIMED 0x40u
-/* a state byte that carries selection weight: susceptible, or claimed in the
- * running round 0 */
-__device__ __forceinline__ bool sel_open(uint32_t b) { return (b & ~LPG_DS_CLAIMED & 0xffu) == 0; }
+/* 0x80 in every byte of w that is a state carrying selection weight:
+ * susceptible, or claimed in the running round of the grid. */
+__device__ __forceinline__ uint32_t sel_open4(uint32_t w) {
+  const uint32_t x = w & ~(LPG_DS_CLAIMED * 0x01010101u);
+  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
+}
 
 /* Programmatic dependent launch: the tick's kernels are launched so that
  * the next one's CTAs may be scheduled while this one finishes.  Every tick
@@ -61,6 +64,12 @@ __device__ __forceinline__ void pdl_begin() {
 /* ------------------------------------------------------------------------ */
 /* fixed-point weights (identical definitions in the oracle)                */
 __device__ __forceinline__ uint64_t fix_risk(float r) { return lpg_fix_risk_f32(r); }
+/* The same in one 32-bit conversion (a quarter of the 64-bit one's cost on
+ * the selection's scans), which saturates at all ones: that stands for a
+ * risk from 256 on (no product below 2^32 rounds to it), whose weight is
+ * fix_risk's. */
+#define LPG_W32_BIG 0xffffffffu
+__device__ __forceinline__ uint32_t sel_w32(float r) { return __float2uint_rn(r * 16777216.0f); }
 __device__ __forceinline__ uint64_t fix_beta(float inf, double scal) {
   double d = ((double)inf * scal) * 0x1.0p40;
   if (!(d > 0.0)) return 0;
@@ -1743,7 +1752,8 @@ __global__ void __launch_bounds__(1024) k_seed(DevWorld W) {
 /* ------------------------------------------------------------------------ */
 /* Per-node record of one selection step, written once per tick so that a
  * target needs one load to find everything about its node. */
-#define LPG_SEL_OFFS 2048 /* target offsets kept in shared memory when G < this */
+#define LPG_SEL_OFFS 2048 /* chunk prefixes of a node that k_sel_rounds keeps in shared memory */
+#define LPG_SEL_NODES 8192 /* k_sel_round0 keeps its target offsets in shared memory when G < this */
 #define LPG_NODE_TX_THREADS 64
 /* six CTAs of the node step per SM (at most 170 registers a thread): one
  * wave covers 912 nodes, so a 774-node tick needs no second wave */
@@ -1785,27 +1795,6 @@ __device__ __forceinline__ uint64_t strain_threshold(double c) {
   if (!(x > 0.0)) return 0;
   if (x >= 0x1.0p53) return (uint64_t)1 << 53;
   return (uint64_t)ceil(x);
-}
-
-/* Cumulative relative FOI that the strain draw compares against
- * (model.py:1127-1135), formed with the same operations in the same order. */
-__device__ __forceinline__ void sel_strain_cum(const DevWorld& W, const DevRep* rp, int g, uint64_t* thr) {
-  double p[LPG_MAX_STRAINS], q[LPG_MAX_STRAINS];
-  double totalp = 0.0;
-  const int ns = rp->ns;
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-    p[k] = k < ns ? W.prob[(int64_t)k * W.G + g] : 0.0;
-    if (k < ns) totalp = totalp + p[k];
-  }
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) q[k] = p[k] / totalp; /* independent divisions */
-  double c = 0.0;
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-    if (k < ns) c = c + q[k];
-    thr[k] = strain_threshold(c);
-  }
 }
 
 /* Node-local inclusive prefix of the chunk weights of a chunk list (n
@@ -2046,7 +2035,7 @@ __global__ void __launch_bounds__(LPG_NODE_TX_THREADS, LPG_NODE_TX_MIN_BLOCKS) k
 #pragma unroll
   for (int k = 0; k < LPG_MAX_STRAINS; ++k)
     if (k < ns) total_p = total_p + p[k];
-  /* strain thresholds of the selection (sel_strain_cum's values), the
+  /* strain thresholds of the selection, the
    * divisions on their own lanes */
   const double qk = pk / total_p;
   uint64_t thr[LPG_MAX_STRAINS];
@@ -2176,7 +2165,7 @@ __global__ void __launch_bounds__(128) k_node_tx_lanes(DevWorld W) {
       total_p = total_p + pk;
     }
   }
-  /* strain thresholds of the selection (sel_strain_cum's values) */
+  /* strain thresholds of the selection */
   uint64_t thr[LPG_MAX_STRAINS];
   {
     double c = 0.0;
@@ -2237,269 +2226,21 @@ __global__ void __launch_bounds__(128) k_node_tx_lanes(DevWorld W) {
 
 /* ------------------------------------------------------------------------ */
 
-/* Slot of target v inside chunk cid (v < the chunk's remaining weight):
- * sub-block by its 16 totals, slot by the 128 state bytes and risks.
- * LPG_NONE if the weights are inconsistent (an internal error). */
-__device__ __forceinline__ uint32_t locate_in_chunk(const DevWorld& W, int64_t cid, uint64_t v) {
-  uint64_t swv[LPG_NSUB];
-#pragma unroll
-  for (int k = 0; k < LPG_NSUB; ++k) swv[k] = __ldcg(&W.sub_w[cid * LPG_NSUB + k]);
-  int sb = LPG_NSUB;
-#pragma unroll
-  for (int k = 0; k < LPG_NSUB; ++k) {
-    if (sb == LPG_NSUB) {
-      if (swv[k] > v) sb = k;
-      else v -= swv[k];
-    }
-  }
-  uint32_t hit = LPG_NONE;
-  if (sb < LPG_NSUB) {
-    const int64_t p0 = cid * LPG_CHUNK + (int64_t)sb * LPG_SUB;
-    uint4 sv[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) sv[k] = __ldcg(reinterpret_cast<const uint4*>(W.ds + p0) + k);
-    for (int grp = 0; grp < 4 && hit == LPG_NONE; ++grp) {
-      float4 rv[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) rv[k] = reinterpret_cast<const float4*>(W.risk + p0 + grp * 32)[k];
-      const uint32_t* sw32 = reinterpret_cast<const uint32_t*>(&sv[grp * 2]);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        if (hit != LPG_NONE) break;
-        const uint32_t sbyte = (sw32[k >> 2] >> (8 * (k & 3))) & 0xffu;
-        if (!sel_open(sbyte)) continue;
-        const uint64_t w = fix_risk(reinterpret_cast<const float*>(rv)[k]);
-        if (w > v) hit = (uint32_t)(p0 + grp * 32 + k);
-        else v -= w;
-      }
-    }
-  }
-  return hit;
-}
-
-/* Locate target v (< the node's remaining susceptible weight) in the node's
- * frozen CDF.  cp holds n chunk prefixes of the node's chunk list ls (n
- * entries); the node's own prefix of entry j is cp[j] - base.  First chunk
- * whose prefix exceeds v (searchsorted side='right', model.py:1118), then
- * the slot inside it. */
-__device__ __forceinline__ uint32_t locate(const DevWorld& W, const int32_t* ls, const uint64_t* cp, int32_t n,
-                                           uint64_t v, uint64_t base) {
-  int32_t lo = 0, hi = n - 1;
-  while (lo < hi) {
-    int32_t mid = (lo + hi) >> 1;
-    if (cp[mid] - base > v) hi = mid; else lo = mid + 1;
-  }
-  if (lo > 0) v -= cp[lo - 1] - base;
-  return locate_in_chunk(W, ls[lo], v);
-}
-
-/* A team of T lanes (T a power of two <= 32, aligned in its warp) that
- * locates one target together. */
-struct Team {
-  unsigned mask; /* the team's lanes */
-  int T, l, lane0;
+/* The agent a target falls on. */
+struct Located {
+  uint32_t hit;  /* its slot; LPG_NONE: the weights are inconsistent (an internal error), and the rest is not set */
+  uint32_t word; /* the slot's state word (4 state bytes) as read: the claim's first guess */
+  uint32_t ref;  /* its reference index */
+  int8_t et;     /* its E duration */
+  uint64_t w;    /* its weight */
 };
-__device__ __forceinline__ Team make_team(int T) {
-  Team t;
-  const int lane = threadIdx.x & 31;
-  t.T = T;
-  t.l = lane & (T - 1);
-  t.lane0 = lane & ~(T - 1);
-  t.mask = T == 32 ? FULLMASK : (((1u << T) - 1u) << t.lane0);
-  return t;
-}
-__device__ __forceinline__ unsigned team_ballot(const Team& tm, bool p) {
-  return tm.T == 32 ? __ballot_sync(tm.mask, p) : (__ballot_sync(tm.mask, p) >> tm.lane0) & ((1u << tm.T) - 1u);
-}
-__device__ __forceinline__ uint64_t team_incl_scan(const Team& tm, uint64_t x) {
-  for (int o = 1; o < tm.T; o <<= 1) {
-    const uint64_t y = __shfl_up_sync(tm.mask, x, o, tm.T);
-    if (tm.l >= o) x += y;
-  }
-  return x;
-}
-
-/* Probe l of a (T+1)-ary search of [lo, lo + m): lo + (l + 1) m / (T + 1).
- * In 32 bits: m is below 2^21 (chunks of a node, or nodes of a batch) and
- * l + 1 at most 32; with T a constant the division is a multiply. */
-template <int T>
-__device__ __forceinline__ int32_t team_probe(int32_t lo, int32_t m, int l) {
-  return lo + (int32_t)(((uint32_t)(l + 1) * (uint32_t)m) / (uint32_t)(T + 1));
-}
-
-/* locate() by a team of T lanes: the same answer, with a (T+1)-ary search
- * of the chunk prefix and, for T >= 4, the sub-block totals and the 128
- * slots split over the lanes (each lane a contiguous run; a team scan finds
- * the lane that holds the target).  Every lane of the team returns the hit.
- * All 32 lanes of the warp call it together (teams without a target pass
- * active = false) so that the warp reconverges between the stages: teams
- * that diverged in the search would otherwise run the later stages one team
- * at a time.  Each probe of the search requests the chunk id beside the
- * prefix, and the team keeps the values at the bounds (the prefix below lo,
- * the chunk at hi), so that the chunk and the target's offset in it are
- * known when the search ends, without further loads.  word_out / risk_out
- * (when given) receive the hit slot's state word (4 state bytes) and risk as
- * read.  T is a template constant, so that every loop below has its exact
- * trip count and no dead iterations (the kernels run once a tick and fetch
- * their instructions cold: code that is not there costs nothing). */
-template <int T>
-__device__ __forceinline__ uint32_t locate_team_t(const DevWorld& W, const int32_t* ls, const uint64_t* cp,
-                                                  int32_t n, uint64_t v, uint64_t base, bool active,
-                                                  uint32_t* word_out, float* risk_out) {
-  const Team tm = make_team(T);
-  int32_t lo = 0, hi = active ? n - 1 : 0;
-  uint64_t cp_lo = base;                    /* cp[lo - 1] (base while lo = 0) */
-  int32_t ls_hi = active ? ls[hi] : 0;      /* ls[hi] */
-  while (lo < hi) {
-    const int32_t m = hi - lo;
-    const int32_t p = team_probe<T>(lo, m, tm.l);
-    const uint64_t cpp = cp[p];
-    const int32_t lsp = ls[p];
-    const unsigned b = team_ballot(tm, cpp - base > v);
-    const int c = __ffs(b) - 1; /* first probe above v; probes ascend with the lane */
-    const uint64_t cp_below = __shfl_sync(tm.mask, cpp, c < 0 ? T - 1 : (c > 0 ? c - 1 : 0), T);
-    const int32_t ls_c = __shfl_sync(tm.mask, lsp, c < 0 ? 0 : c, T);
-    const int32_t lo0 = lo;
-    if (c < 0) {
-      lo = team_probe<T>(lo0, m, T - 1) + 1;
-      cp_lo = cp_below;
-    } else {
-      if (c > 0) {
-        lo = team_probe<T>(lo0, m, c - 1) + 1;
-        cp_lo = cp_below;
-      }
-      hi = team_probe<T>(lo0, m, c);
-      ls_hi = ls_c;
-    }
-  }
-  __syncwarp();
-  uint32_t hit = LPG_NONE;
-  int64_t cid = 0;
-  if (active) {
-    if (lo > 0) v -= cp_lo - base;
-    cid = ls_hi;
-  }
-  if constexpr (T < 4) {
-    if (active && tm.l == 0) hit = locate_in_chunk(W, cid, v);
-    __syncwarp();
-    hit = active ? __shfl_sync(tm.mask, hit, 0, T) : LPG_NONE;
-    if (word_out && hit != LPG_NONE) {
-      *word_out = __ldcg(reinterpret_cast<const uint32_t*>(W.ds + ((int64_t)hit & ~3LL)));
-      *risk_out = W.risk[hit];
-    }
-    return hit;
-  } else {
-    /* sub-block: lanes l < min(T, 16) hold 16 / min(T, 16) consecutive totals */
-    constexpr int TS = T < LPG_NSUB ? T : LPG_NSUB;
-    constexpr int PER = LPG_NSUB / TS;
-    int sb = -1;
-    uint64_t vl = 0;
-    if (active) {
-      uint64_t sw[PER];
-      uint64_t sum = 0;
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        sw[k] = tm.l < TS ? __ldcg(&W.sub_w[cid * LPG_NSUB + tm.l * PER + k]) : 0;
-        sum += sw[k];
-      }
-      const uint64_t incl = team_incl_scan(tm, sum);
-      const uint64_t excl = incl - sum;
-      const unsigned own = team_ballot(tm, sum > 0 && excl <= v && v < incl);
-      if (own != 0) {
-        const int ol = __ffs(own) - 1;
-        vl = v - excl;
-        if (tm.l == ol) {
-#pragma unroll
-          for (int k = 0; k < PER; ++k) {
-            if (sb < 0) {
-              if (sw[k] > vl) sb = tm.l * PER + k;
-              else vl -= sw[k];
-            }
-          }
-        }
-        sb = __shfl_sync(tm.mask, sb, ol, T);
-        vl = __shfl_sync(tm.mask, vl, ol, T);
-      }
-    }
-    __syncwarp();
-    /* slots: lane l holds L = 128 / T consecutive slots (L / 4 state words) */
-    constexpr int L = LPG_SUB / T;
-    const bool go = active && sb >= 0;
-    const int64_t s0 = go ? cid * LPG_CHUNK + (int64_t)sb * LPG_SUB + (int64_t)tm.l * L : 0;
-    uint32_t dw[L / 4];
-    float4 rv[L / 4];
-#pragma unroll
-    for (int k = 0; k < L / 4; ++k) {
-      if (go) {
-        dw[k] = __ldcg(reinterpret_cast<const uint32_t*>(W.ds + s0) + k);
-        rv[k] = reinterpret_cast<const float4*>(W.risk + s0)[k];
-      } else {
-        dw[k] = 0xffffffffu;
-        rv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    uint64_t wsum = 0;
-#pragma unroll
-    for (int k = 0; k < L; ++k)
-      if (sel_open((dw[k >> 2] >> (8 * (k & 3))) & 0xffu)) wsum += fix_risk(reinterpret_cast<const float*>(rv)[k]);
-    if (go) {
-      const uint64_t incl = team_incl_scan(tm, wsum);
-      const uint64_t excl = incl - wsum;
-      const unsigned own = team_ballot(tm, wsum > 0 && excl <= vl && vl < incl);
-      if (own != 0) {
-        const int ol = __ffs(own) - 1;
-        uint32_t word = 0;
-        float rk = 0.f;
-        if (tm.l == ol) {
-          uint64_t r = vl - excl;
-#pragma unroll
-          for (int k = 0; k < L; ++k) {
-            if (hit == LPG_NONE && sel_open((dw[k >> 2] >> (8 * (k & 3))) & 0xffu)) {
-              const uint64_t w = fix_risk(reinterpret_cast<const float*>(rv)[k]);
-              if (w > r) {
-                hit = (uint32_t)(s0 + k);
-                word = dw[k >> 2];
-                rk = reinterpret_cast<const float*>(rv)[k];
-              } else {
-                r -= w;
-              }
-            }
-          }
-        }
-        hit = __shfl_sync(tm.mask, hit, ol, T);
-        if (word_out) {
-          *word_out = __shfl_sync(tm.mask, word, ol, T);
-          *risk_out = __shfl_sync(tm.mask, rk, ol, T);
-        }
-      }
-    }
-    __syncwarp();
-    return hit;
-  }
-}
-
-/* locate_team_t for a team size known only at run time (uniform in the
- * warp). */
-__device__ __forceinline__ uint32_t locate_team(const DevWorld& W, const Team& tm, const int32_t* ls,
-                                                const uint64_t* cp, int32_t n, uint64_t v, uint64_t base,
-                                                bool active = true, uint32_t* word_out = nullptr,
-                                                float* risk_out = nullptr) {
-  switch (tm.T) {
-    case 32: return locate_team_t<32>(W, ls, cp, n, v, base, active, word_out, risk_out);
-    case 16: return locate_team_t<16>(W, ls, cp, n, v, base, active, word_out, risk_out);
-    case 8: return locate_team_t<8>(W, ls, cp, n, v, base, active, word_out, risk_out);
-    case 4: return locate_team_t<4>(W, ls, cp, n, v, base, active, word_out, risk_out);
-    case 2: return locate_team_t<2>(W, ls, cp, n, v, base, active, word_out, risk_out);
-    default: return locate_team_t<1>(W, ls, cp, n, v, base, active, word_out, risk_out);
-  }
-}
 
 /* The exposure of an agent that a target has claimed: strain by relative
- * FOI (model.py:1127-1145), its first step in E, and every susceptible total
- * but the sub-block's (sub_now: that one too).  Returns its weight. */
-__device__ __forceinline__ uint64_t expose_claimed(DevWorld& W, int64_t pos, int g, const SelInfo& N, uint64_t r53,
-                                                   int8_t et, float risk, bool sub_now) {
-  const int G = W.G;
+ * FOI (model.py:1127-1145; returned), its first step in E, and its weight w
+ * out of its chunk (sub_now: and its sub-block).  The node's totals are the
+ * caller's. */
+__device__ __forceinline__ int expose_claimed(DevWorld& W, int64_t pos, const SelInfo& N, uint64_t r53, int8_t et,
+                                              uint64_t w, bool sub_now) {
   const int64_t cid = pos / LPG_CHUNK;
   int s = 0;
   bool found = false;
@@ -2516,37 +2257,56 @@ __device__ __forceinline__ uint64_t expose_claimed(DevWorld& W, int64_t pos, int
     W.evt[pos] = e1;
     atomicMin(&W.sub_evt[pos >> 7], e1);
   }
-  const uint64_t w = fix_risk(risk);
-  atomicAdd(&W.tot[(int64_t)TT_S * G + g], -1);
-  atomicAdd(&W.tot[(int64_t)(TT_E0 + s) * G + g], 1);
-  atomicAdd(&W.ev[(int64_t)(EV_TXNEW0 + s) * G + g], 1);
-  atomicAdd((unsigned long long*)&W.uniq[g], 1ULL);
   if (w) {
-    atomicAdd((unsigned long long*)&W.sw[g], neg64(w));
     atomicAdd((unsigned long long*)&W.chunk_w[cid], neg64(w));
     if (sub_now) atomicAdd((unsigned long long*)&W.sub_w[cid * LPG_NSUB + (pos % LPG_CHUNK) / LPG_SUB], neg64(w));
   }
-  return w;
+  return s;
 }
 
-/* The first target to claim an agent (state 0 -> 1) exposes it (rounds
- * after the first, whose claims follow all of the round's locates).
- * Returns whether this target claimed it (and the weight it removed in
- * *w_out). */
-__device__ __forceinline__ bool claim(DevWorld& W, uint32_t hit, int g, const SelInfo& N, uint64_t* w_out = nullptr) {
-  const int64_t pos = hit;
-  /* the agent's fixed columns requested first, and its strain draw formed
-   * while the claim's atomic is in flight (a lost claim discards them) */
-  const uint32_t ref = W.ref[pos];
-  const int8_t et = W.et[pos];
-  const float risk = W.risk[pos];
+/* n agents of node g exposed by strain s, and n of all strains with weight w
+ * out of the node's totals. */
+__device__ __forceinline__ void node_strain(DevWorld& W, int g, int s, int n) {
+  atomicAdd(&W.tot[(int64_t)(TT_E0 + s) * W.G + g], n);
+  atomicAdd(&W.ev[(int64_t)(EV_TXNEW0 + s) * W.G + g], n);
+}
+__device__ __forceinline__ void node_exposed(DevWorld& W, int g, int n, uint64_t w) {
+  atomicAdd(&W.tot[(int64_t)TT_S * W.G + g], -n);
+  atomicAdd((unsigned long long*)&W.uniq[g], (unsigned long long)n);
+  if (w) atomicAdd((unsigned long long*)&W.sw[g], neg64(w));
+}
+/* The node totals of the warp's claims, one set of atomics per node of the
+ * warp (a warp's targets are neighbours, so mostly one node).  All lanes. */
+__device__ __forceinline__ void warp_node_exposed(DevWorld& W, int g, int ns, bool won, int s, uint64_t w) {
+  const unsigned all = __ballot_sync(FULLMASK, won);
+  if (!won) return;
+  const unsigned by = __match_any_sync(all, g);
+  const bool lead = (int)(threadIdx.x & 31) == __ffs(by) - 1;
+  const uint64_t wt = warp_sum_u64(by, w);
+  if (lead) node_exposed(W, g, __popc(by), wt);
+  for (int k = 0; k < ns; ++k) {
+    const int n = __popc(__ballot_sync(by, s == k));
+    if (lead && n) node_strain(W, g, k, n);
+  }
+}
+
+/* The first target to claim an agent (state 0 -> `mark`) exposes it.  With
+ * mark = 1 (the rounds of k_sel_rounds, whose claims follow all of the
+ * round's locates) it leaves its sub-block's weight at once; with
+ * LPG_DS_CLAIMED (a round of k_sel_round0, claimed as soon as the target is
+ * located) the round's other targets still see it and the claimer removes it
+ * after the round (claim0_finish).  Returns the strain, or -1 when
+ * another target has the agent. */
+__device__ __forceinline__ int claim(DevWorld& W, const Located& L, const SelInfo& N, uint32_t mark) {
+  const int64_t pos = L.hit;
+  uint32_t old = L.word;
   uint32_t* wp = reinterpret_cast<uint32_t*>(W.ds + (pos & ~3LL));
   const int sh = (int)(pos & 3) * 8;
-  uint32_t old = *(volatile uint32_t*)wp;
-  const uint64_t r53 = lpg_u53(N.seed, LPG_P_STRAIN, N.t, ref, 0, 0);
+  /* the strain draw, formed before the claim's atomic (a lost claim discards it) */
+  const uint64_t r53 = lpg_u53(N.seed, LPG_P_STRAIN, N.t, L.ref, 0, 0);
   bool won = false;
   while (((old >> sh) & 0xffu) == 0) {
-    const uint32_t nw = (old & ~(0xffu << sh)) | (1u << sh);
+    const uint32_t nw = (old & ~(0xffu << sh)) | (mark << sh);
     const uint32_t prev = atomicCAS(wp, old, nw);
     if (prev == old) {
       won = true;
@@ -2554,40 +2314,7 @@ __device__ __forceinline__ bool claim(DevWorld& W, uint32_t hit, int g, const Se
     }
     old = prev;
   }
-  if (!won) return false;
-  const uint64_t w = expose_claimed(W, pos, g, N, r53, et, risk, true);
-  if (w_out) *w_out = w;
-  return true;
-}
-
-/* A round-0 claim, made as soon as the target is located: state 0 ->
- * LPG_DS_CLAIMED (the round's other targets still see the agent's weight),
- * the exposure and every total but the sub-block weight, which the claimer
- * removes after the round (claim0_finish).  word and risk are the slot's
- * state word and risk as the locate read them (the word is the first guess
- * of the compare-and-swap). */
-__device__ __forceinline__ bool claim0(DevWorld& W, uint32_t hit, uint32_t word, float risk, int g,
-                                       const SelInfo& N, uint64_t* w_out) {
-  const int64_t pos = hit;
-  const uint32_t ref = W.ref[pos];
-  const int8_t et = W.et[pos];
-  uint32_t* wp = reinterpret_cast<uint32_t*>(W.ds + (pos & ~3LL));
-  const int sh = (int)(pos & 3) * 8;
-  uint32_t old = word;
-  const uint64_t r53 = lpg_u53(N.seed, LPG_P_STRAIN, N.t, ref, 0, 0);
-  bool won = false;
-  while (((old >> sh) & 0xffu) == 0) {
-    const uint32_t nw = (old & ~(0xffu << sh)) | (LPG_DS_CLAIMED << sh);
-    const uint32_t prev = atomicCAS(wp, old, nw);
-    if (prev == old) {
-      won = true;
-      break;
-    }
-    old = prev;
-  }
-  if (!won) return false;
-  *w_out = expose_claimed(W, pos, g, N, r53, et, risk, false);
-  return true;
+  return won ? expose_claimed(W, pos, N, r53, L.et, L.w, mark != LPG_DS_CLAIMED) : -1;
 }
 
 /* After round 0: the claimed agent becomes exposed (state 1) and leaves its
@@ -2637,25 +2364,6 @@ __device__ bool grid_sync(unsigned long long* ctr, long long limit, bool skip_ar
   return s_ok != 0;
 }
 
-/* First g in [lo, hi] with off[g] > q (the answer is known to be <= hi), by
- * a (T+1)-ary search of the team over off (shared memory). */
-template <int T>
-__device__ __forceinline__ int team_first_above(const Team& tm, const int64_t* off, int lo, int hi, int64_t q) {
-  while (lo < hi) {
-    const int m = hi - lo;
-    const unsigned b = team_ballot(tm, off[team_probe<T>(lo, m, tm.l)] > q);
-    const int c = __ffs(b) - 1;
-    const int lo0 = lo;
-    if (c < 0) {
-      lo = team_probe<T>(lo0, m, T - 1) + 1;
-    } else {
-      if (c > 0) lo = team_probe<T>(lo0, m, c - 1) + 1;
-      hi = team_probe<T>(lo0, m, c);
-    }
-  }
-  return lo;
-}
-
 /* Last g in [0, G) with off[g] <= q (off ascending from off[0] = 0, q below
  * off[G]), by one lane. */
 __device__ __forceinline__ int node_of_target(const int64_t* off, int G, int64_t q) {
@@ -2668,80 +2376,246 @@ __device__ __forceinline__ int node_of_target(const int64_t* off, int G, int64_t
   return lo;
 }
 
-/* Round 0's targets for a team size T.  A team takes its targets T at a
- * time: lane l of the team finds the node and forms the uniform of the
- * batch's l-th target (target q0 + (b T + l) nteams), the team then locates
- * the batch's targets one after another on the frozen CDF, and each lane
- * claims its own target's agent (claim0), so that the per-target work that
- * is not the search (node, uniform, claim, strain draw) runs once per lane
- * rather than once per team.  A lane keeps its first claim in registers and
+/* The 16 slots of a lane in stage 3 of a team of 8 (locate_batch). */
+struct Slots16 {
+  uint4 ds;
+  float4 r[4];
+};
+__device__ __forceinline__ Slots16 load_slots(const DevWorld& W, int64_t s0, bool go) {
+  Slots16 x;
+  x.ds = make_uint4(~0u, ~0u, ~0u, ~0u);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x.r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (go) {
+    x.ds = __ldcg(reinterpret_cast<const uint4*>(W.ds + s0));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x.r[k] = reinterpret_cast<const float4*>(W.risk + s0)[k];
+  }
+  return x;
+}
+
+/* Locates a team of 8's eight targets (lane l's target: v on the chunk list
+ * ls with prefix cp, n entries), stage by stage so that the loads of a stage
+ * are in flight for several targets at once: each lane searches its own
+ * chunk (a warp's targets are neighbours, their prefixes in L1); the team
+ * sums the sixteen sub-blocks of four targets at a time (two totals a lane);
+ * then the 128 slots of one target after another (sixteen a lane), the next
+ * target's requested before this one's are summed. Lane l gets its own
+ * target's agent.  A team's targets are on its first lanes (act).  All
+ * lanes of the warp. */
+template <bool FRESH>
+__device__ __forceinline__ void locate_batch(const DevWorld& W, const int32_t* ls, const uint64_t* cp, int32_t n,
+                                             uint64_t v, bool act, Located* out) {
+  const int l = threadIdx.x & 7, lane0 = threadIdx.x & 24; /* in its team; the team's first in its warp */
+  /* the largest number of targets of a team of the warp */
+  const int nk = __reduce_max_sync(FULLMASK, act ? l + 1 : 0);
+  out->hit = LPG_NONE;
+  if (nk == 0) return;
+  int32_t cid = 0;
+  if (act) {
+    int32_t lo = 0, hi = n - 1;
+    uint64_t below = 0; /* cp[lo - 1] */
+    while (lo < hi) {
+      const int32_t mid = (lo + hi) >> 1;
+      const uint64_t c = FRESH ? __ldcg(cp + mid) : cp[mid];
+      if (c > v) {
+        hi = mid;
+      } else {
+        lo = mid + 1;
+        below = c;
+      }
+    }
+    v -= below;
+    cid = ls[lo];
+  }
+  __syncwarp();
+  int sb = -1;
+#pragma unroll
+  for (int k0 = 0; k0 < 8; k0 += 4) {
+    if (k0 >= nk) break;
+    ulonglong2 x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t c = __shfl_sync(FULLMASK, cid, k0 + k, 8);
+      x[k] = __ldcg(reinterpret_cast<const ulonglong2*>(W.sub_w + c * LPG_NSUB) + l);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t vk = __shfl_sync(FULLMASK, v, k0 + k, 8);
+      const uint64_t sum = x[k].x + x[k].y;
+      uint64_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(FULLMASK, incl, o, 8);
+        if (l >= o) incl += y;
+      }
+      const uint64_t excl = incl - sum;
+      const unsigned own = (__ballot_sync(FULLMASK, excl <= vk && vk < incl) >> lane0) & 0xffu;
+      const int ol = own ? __ffs(own) - 1 : 0;
+      uint64_t r = vk - excl;
+      const bool second = r >= x[k].x;
+      if (second) r -= x[k].x;
+      r = __shfl_sync(FULLMASK, r, ol, 8);
+      const int b = __shfl_sync(FULLMASK, 2 * l + (second ? 1 : 0), ol, 8);
+      if (l == k0 + k && act && own) {
+        sb = b;
+        v = r;
+      }
+    }
+  }
+  const int64_t start = (int64_t)cid * LPG_CHUNK + (int64_t)(sb < 0 ? 0 : sb) * LPG_SUB;
+  int64_t s0 = __shfl_sync(FULLMASK, start, 0, 8) + l * 16;
+  bool go = __shfl_sync(FULLMASK, sb, 0, 8) >= 0;
+  Slots16 nx = load_slots(W, s0, go);
+#pragma unroll 1
+  for (int k = 0; k < nk; ++k) {
+    const Slots16 x = nx;
+    const int64_t at = s0;
+    const bool have = go;
+    if (k + 1 < nk) {
+      s0 = __shfl_sync(FULLMASK, start, k + 1, 8) + l * 16;
+      go = __shfl_sync(FULLMASK, sb, k + 1, 8) >= 0;
+      nx = load_slots(W, s0, go);
+    }
+    const uint64_t vk = __shfl_sync(FULLMASK, v, k, 8);
+    const uint32_t dw[4] = {x.ds.x, x.ds.y, x.ds.z, x.ds.w};
+    uint4 w[4]; /* the weights, 0 where a slot carries none */
+    uint64_t q[4], sum = 0;
+    uint32_t top = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t m = sel_open4(dw[j]);
+      w[j].x = sel_w32(x.r[j].x) & (uint32_t)((int32_t)(m << 24) >> 31);
+      w[j].y = sel_w32(x.r[j].y) & (uint32_t)((int32_t)(m << 16) >> 31);
+      w[j].z = sel_w32(x.r[j].z) & (uint32_t)((int32_t)(m << 8) >> 31);
+      w[j].w = sel_w32(x.r[j].w) & (uint32_t)((int32_t)m >> 31);
+      top = max(top, max(max(w[j].x, w[j].y), max(w[j].z, w[j].w)));
+      q[j] = ((uint64_t)w[j].x + w[j].y) + ((uint64_t)w[j].z + w[j].w);
+      sum += q[j];
+    }
+    if (__any_sync(FULLMASK, top == LPG_W32_BIG)) { /* a weight beyond 32 bits among the warp's slots */
+      sum = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t w4[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+        q[j] = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[j] += w4[i] != LPG_W32_BIG ? w4[i] : fix_risk(W.risk[at + 4 * j + i]);
+        sum += q[j];
+      }
+    }
+    uint64_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(FULLMASK, incl, o, 8);
+      if (l >= o) incl += y;
+    }
+    const uint64_t excl = incl - sum;
+    const bool own = have && excl <= vk && vk < incl;
+    uint32_t hit = LPG_NONE, word = 0;
+    uint64_t hw = 0;
+    if (own) {
+      /* the four slots, then the slot: the first whose running sum exceeds the target */
+      uint64_t r = vk - excl;
+      int kq = 0;
+      uint4 wq = w[0];
+      word = dw[0];
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        if (kq == j && r >= q[j]) {
+          r -= q[j];
+          kq = j + 1;
+          wq = w[j + 1];
+          word = dw[j + 1];
+        }
+      const uint32_t w4[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (hit == LPG_NONE) {
+          const uint64_t wi = w4[i] != LPG_W32_BIG ? w4[i] : fix_risk(W.risk[at + 4 * kq + i]);
+          if (r < wi) {
+            hit = (uint32_t)(at + 4 * kq + i);
+            hw = wi;
+          } else {
+            r -= wi;
+          }
+        }
+    }
+    const unsigned om = (__ballot_sync(FULLMASK, own) >> lane0) & 0xffu;
+    const int ol = om ? __ffs(om) - 1 : 0;
+    hit = __shfl_sync(FULLMASK, hit, ol, 8);
+    word = __shfl_sync(FULLMASK, word, ol, 8);
+    hw = __shfl_sync(FULLMASK, hw, ol, 8);
+    if (l == k) {
+      out->hit = hit;
+      out->word = word;
+      out->w = hw;
+      if (hit != LPG_NONE) { /* requested here, used at the claim */
+        out->ref = W.ref[hit];
+        out->et = W.et[hit];
+      }
+    }
+  }
+}
+
+/* The targets of a round made by the whole grid (round 0; FRESH: a later
+ * one, whose prefixes this kernel has rewritten).  A CTA has an equal run of
+ * consecutive targets, 256 of them at a time (target l * 32 + team of the
+ * 256 on lane l of a team of 8; 32 or fewer: one a team), so that its
+ * targets share nodes: their prefixes stay in L1 and the claims' node totals
+ * are added once a warp.  Each lane forms its own target's node and uniform,
+ * the team locates its targets (locate_batch), and each lane claims its own
+ * target's agent (claim).  A lane keeps its first claim in registers and
  * stores later ones' slots in hits[q]; then the grid barrier, after which
  * each lane settles its claims (state 1, sub-block weight).  Returns false
  * when the barrier's wait ran out. */
-template <int T>
-__device__ __forceinline__ bool round0_targets(DevWorld& W, const int64_t* offs, const SelInfo* info, int64_t K) {
+template <bool FRESH>
+__device__ __forceinline__ bool grid_targets(DevWorld& W, const int64_t* offs, const SelInfo* info, int64_t K,
+                                             int round) {
   const int G = W.G;
-  const Team tm = make_team(T);
-  const int64_t nteams = ((int64_t)gridDim.x * blockDim.x) / T;
-  const int64_t q0 = (int64_t)(threadIdx.x / T) * gridDim.x + blockIdx.x;
+  const int64_t qa = K * blockIdx.x / gridDim.x, qe = K * (blockIdx.x + 1) / gridDim.x;
+  const int64_t q0 = qa + (threadIdx.x & 7) * 32 + threadIdx.x / 8;
   uint32_t h0 = LPG_NONE;
   uint64_t w0 = 0;
-  /* warp-uniform trip count: every lane stays until no team of its warp has a target */
   int b = 0;
-  for (int64_t qb = q0; __any_sync(FULLMASK, qb < K); qb += (int64_t)T * nteams, ++b) {
-    /* this lane's target of the batch */
-    const int64_t q = qb + (int64_t)tm.l * nteams;
-    const bool act = q < K;
+  for (int64_t q = q0, qw = qa; qw < qe; q += 256, qw += 256, ++b) {
+    const bool act = q < qe;
     int g = 0;
     uint64_t v = 0;
-    int32_t la = 0, ln = 1, lcsr = 0;
+    int32_t la = 0, ln = 1, lcsr = 0, ns = 0;
     if (act) {
       g = node_of_target(offs, G, q);
       const SelInfo& N = info[g];
-      v = lpg_scale_target(lpg_u53(N.seed, LPG_P_SELECT, N.t, (uint64_t)N.i, 0, (uint64_t)(q - offs[g])), N.T);
       la = N.a;
       ln = N.n;
       lcsr = N.csr;
+      ns = N.ns;
+      const uint64_t total = FRESH ? __ldcg(W.cpref + la + ln - 1) : N.T;
+      v = lpg_scale_target(lpg_u53(N.seed, LPG_P_SELECT, N.t, (uint64_t)N.i, (uint64_t)round, (uint64_t)(q - offs[g])),
+                           total);
     }
-    /* the batch's targets are a prefix of the team's lanes (q ascends with l) */
-    const int nk = __reduce_max_sync(FULLMASK, (unsigned)__popc(team_ballot(tm, act)));
-    uint32_t my_hit = LPG_NONE, my_word = 0;
-    float my_rk = 0.f;
-    for (int k = 0; k < nk; ++k) {
-      const bool ak = __shfl_sync(FULLMASK, (int)act, k, T) != 0;
-      const uint64_t vk = __shfl_sync(FULLMASK, v, k, T);
-      const int32_t ak_a = __shfl_sync(FULLMASK, la, k, T);
-      const int32_t ak_n = __shfl_sync(FULLMASK, ln, k, T);
-      const int32_t ak_c = __shfl_sync(FULLMASK, lcsr, k, T);
-      const int32_t* ls = W.node_chunks[ak_c] + ak_a;
-      uint32_t word = 0;
-      float rk = 0.f;
-      const uint32_t hit = locate_team_t<T>(W, ls, W.cpref + ak_a, ak ? ak_n : 1, vk, 0, ak, &word, &rk);
-      if (tm.l == k) {
-        my_hit = hit;
-        my_word = word;
-        my_rk = rk;
-      }
-    }
+    Located L;
+    locate_batch<FRESH>(W, W.node_chunks[lcsr] + la, W.cpref + la, ln, v, act, &L);
+    int s = -1;
     if (act) {
-      uint32_t won_at = LPG_NONE;
-      uint64_t w = 0;
-      if (my_hit == LPG_NONE) W.reps[W.node_rep[g]].error = LPG_ERR_INTERNAL;
-      else if (claim0(W, my_hit, my_word, my_rk, g, info[g], &w)) won_at = my_hit;
+      if (L.hit == LPG_NONE) W.reps[W.node_rep[g]].error = LPG_ERR_INTERNAL;
+      else s = claim(W, L, info[g], LPG_DS_CLAIMED);
+      const uint32_t won_at = s >= 0 ? L.hit : LPG_NONE;
       if (b == 0) {
         h0 = won_at;
-        w0 = w;
+        w0 = L.w;
       } else {
         W.hits[q] = won_at;
       }
     }
+    __syncwarp();
+    warp_node_exposed(W, g, ns, s >= 0, s, L.w);
   }
   /* every target of the round located and claimed: the claimed agents
    * become exposed and leave their sub-blocks' weights */
   if (!grid_sync(W.grid_bar, W.wait_spin, W.test_bar_skip && blockIdx.x == 0)) return false;
   claim0_finish(W, h0, w0);
-  /* this lane's later claims: batches 1, 2, ... */
-  for (int64_t q = q0 + ((int64_t)T + tm.l) * nteams; q < K; q += (int64_t)T * nteams) {
+  for (int64_t q = q0 + 256; q < qe; q += 256) { /* this lane's later claims */
     const uint32_t h = W.hits[q];
     if (h != LPG_NONE) claim0_finish(W, h, fix_risk(W.risk[h]));
   }
@@ -2753,15 +2627,80 @@ __device__ __forceinline__ bool round0_targets(DevWorld& W, const int64_t* offs,
  * target count (ksel), its selection record and its node-local chunk
  * prefix.  Round 0 runs over all nodes at once in one cooperative launch
  * (k_sel_round0): every CTA forms the target offsets in its shared memory;
- * targets go round-robin over the CTAs, each located by a team of lanes on
- * the round's frozen CDF and claimed at once (claim0: the agent keeps its
- * weight for the round's other targets); after a grid barrier the claimers
- * settle the sub-block weights.  The few collisions left after round 0 are
- * redrawn per node by one CTA in later rounds (k_sel_rounds), with CTA
- * barriers only.  Round r of node n draws the (n, r, j) uniforms of the
- * oracle, so the CDF targets are the same whatever runs them, and which of
- * two targets on one agent claims it changes nothing (its strain draw is
- * keyed by the agent). */
+ * each CTA has a run of consecutive targets, located by teams of eight lanes
+ * on the round's frozen CDF and claimed at once (claim with
+ * LPG_DS_CLAIMED: the agent keeps its weight for the round's other
+ * targets); after a grid barrier the claimers settle the sub-block weights.
+ * While a node still lacks hundreds of agents, the grid makes the next round
+ * likewise.  The few collisions left are redrawn per node by one CTA
+ * (k_sel_rounds), with CTA barriers only.  Round r of node n draws the
+ * (n, r, j) uniforms of the oracle, so the CDF targets are the same whatever
+ * runs them, and which of two targets on one agent claims it changes nothing
+ * (its strain draw is keyed by the agent).
+ *
+ * Bound by the latency of a target's dependent reads (its chunk's sub-block
+ * totals, 128 states and risks, the agent's columns: 1 KB of lines), so the
+ * stages run for several targets at once and consecutive targets share a
+ * CTA.  774 nodes, 2.2e8 agents, 4.9e7 targets over 365 ticks: k_sel_round0
+ * 44 ms and k_sel_rounds 27 ms with targets dealt round-robin, searched one
+ * at a time by the whole team and added to the node totals one by one;
+ * 26 ms and 11 ms now (0.79 and 0.4 ns a target on the busiest ticks).
+ * Three CTAs an SM: with two, 27 ms.
+ *
+ * A round after the first is made by the whole grid while some node still
+ * lacks more agents than LPG_SEL_GRID_NODE: a round of one node costs its
+ * CTA about 10 us per 256 targets, a round of the grid two barriers, a scan
+ * over the nodes and their prefixes, about 12 us (both kernels together, 774
+ * nodes as above: lines at 64, 256 and 1024 give 38.3, 38.2 and 39.4 ms).
+ * Asked only on ticks with LPG_SEL_GRID_MIN targets, as the answer takes
+ * that scan. */
+#define LPG_SEL_GRID_MIN 16384
+#define LPG_SEL_GRID_NODE 256
+#define LPG_SEL_GRID_ROUNDS 8
+
+/* The round's target offsets over all nodes into off (shared memory, or
+ * global memory that every CTA writes alike); returns their number, the
+ * largest node's in *most.  All threads of the CTA. */
+__device__ int64_t sel_offsets(const DevWorld& W, int64_t* off, int round, int64_t* most) {
+  __shared__ int64_t s_total;
+  __shared__ unsigned long long s_most;
+  const int G = W.G;
+  if (threadIdx.x == 0) s_most = 0;
+  __syncthreads();
+  int64_t carry = 0, top = 0;
+  for (int base = 0; base < G; base += 4 * blockDim.x) {
+    /* 4 consecutive nodes a thread: one block scan per 4 * blockDim nodes */
+    const int g0 = base + 4 * threadIdx.x;
+    int64_t k[4], sum = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      k[u] = g0 + u < G ? __ldcg(&W.ksel[g0 + u]) : 0;
+      if (round > 0 && k[u] > 0) {
+        k[u] -= (int64_t)__ldcg((const unsigned long long*)&W.uniq[g0 + u]);
+        if (k[u] < 0 || __ldcg(&W.sw[g0 + u]) == 0) k[u] = 0;
+      }
+      sum += k[u];
+      top = k[u] > top ? k[u] : top;
+    }
+    int64_t tot;
+    int64_t run = carry + block_excl_scan(sum, &tot);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (g0 + u < G) off[g0 + u] = run;
+      run += k[u];
+    }
+    carry += tot;
+  }
+  if (round > 0 && top > 0) atomicMax(&s_most, (unsigned long long)top);
+  if (threadIdx.x == 0) {
+    off[G] = carry;
+    s_total = carry;
+  }
+  __syncthreads();
+  *most = (int64_t)s_most;
+  return s_total;
+}
+
 __global__ void __launch_bounds__(256, 3) k_sel_round0(DevWorld W) {
   pdl_begin();
   const int R = W.n_reps, G = W.G;
@@ -2771,65 +2710,42 @@ __global__ void __launch_bounds__(256, 3) k_sel_round0(DevWorld W) {
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   const SelInfo* info = reinterpret_cast<const SelInfo*>(W.sel_info);
-  __shared__ int64_t s_K;
-  __shared__ int64_t s_off[LPG_SEL_OFFS];
-  const bool offs_in_smem = G < LPG_SEL_OFFS;
-
-  /* target offsets of all nodes; every CTA computes the same values and
-   * keeps them in shared memory when they fit */
-  {
-    int64_t carry = 0;
-    for (int base = 0; base < G; base += 4 * blockDim.x) {
-      /* 4 consecutive nodes a thread: one block scan per 4 * blockDim nodes */
-      const int g0 = base + 4 * threadIdx.x;
-      int64_t k[4], sum = 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        k[u] = g0 + u < G ? __ldcg(&W.ksel[g0 + u]) : 0;
-        sum += k[u];
-      }
-      int64_t tot;
-      int64_t run = carry + block_excl_scan(sum, &tot);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (g0 + u < G) {
-          if (offs_in_smem) s_off[g0 + u] = run;
-          if (!offs_in_smem || blockIdx.x == 0) W.tgt_off[g0 + u] = run;
-        }
-        run += k[u];
-      }
-      carry += tot;
-    }
-    if (threadIdx.x == 0) {
-      if (offs_in_smem) s_off[G] = carry;
-      if (!offs_in_smem || blockIdx.x == 0) W.tgt_off[G] = carry;
-      s_K = carry;
-    }
-    __syncthreads();
-  }
-  const int64_t K = s_K;
+  extern __shared__ int64_t s_sel_off[];
+  const bool offs_in_smem = G < LPG_SEL_NODES;
+  /* every CTA forms the same offsets; when they do not fit in shared memory
+   * it writes them all itself and reads its own values back */
+  int64_t* offs = offs_in_smem ? s_sel_off : W.tgt_off;
+  int64_t most;
+  int64_t K = sel_offsets(W, offs, 0, &most);
   if (K > W.hits_cap) { /* the same in every CTA */
     if (gtid == 0) W.reps[0].error = LPG_ERR_INTERNAL;
     return;
   }
-  if (gtid == 0 && K) atomicAdd(&W.ctr[LPG_CTR_SEL_TARGETS], (unsigned long long)K);
-  /* (when the offsets do not fit in shared memory, every CTA has written
-   * all of them to tgt_off itself, so it reads its own values back) */
-  const int64_t* offs = offs_in_smem ? s_off : W.tgt_off;
-  /* Targets go round-robin over the CTAs (target q on CTA q mod grid), so
-   * that a few thousand of them still use every SM, each located by a team
-   * of T lanes: the largest power of two <= 32 with T * K <= threads, and
-   * at least 8 (more targets than teams: each team takes several in turn;
-   * smaller teams would hold more slots a lane than the registers of two
-   * CTAs an SM allow). */
-  int T = 8;
-  while (T < 32 && (int64_t)(2 * T) * K <= gsz) T *= 2;
+  const bool grid_rounds = offs_in_smem && K >= LPG_SEL_GRID_MIN;
+  int round = 0;
   bool ok;
-  switch (T) {
-    case 32: ok = round0_targets<32>(W, offs, info, K); break;
-    case 16: ok = round0_targets<16>(W, offs, info, K); break;
-    default: ok = round0_targets<8>(W, offs, info, K); break;
+  for (;;) {
+    if (gtid == 0 && K) atomicAdd(&W.ctr[LPG_CTR_SEL_TARGETS], (unsigned long long)K);
+    ok = round > 0 ? grid_targets<true>(W, offs, info, K, round) : grid_targets<false>(W, offs, info, K, 0);
+    ++round;
+    if (!ok || !grid_rounds || round >= LPG_SEL_GRID_ROUNDS) break; /* the same in every CTA (or a wait ran out) */
+    __syncthreads(); /* the offsets are read */
+    K = sel_offsets(W, offs, round, &most);
+    if (most <= LPG_SEL_GRID_NODE) break;
+    /* the new prefixes of the nodes that go on; the barrier also ends the
+     * settling of the claims (which changes neither the totals read above
+     * nor the chunks' weights) */
+    unsigned nodes = 0;
+    for (int g = (int)(gtid >> 5); g < G; g += (int)(gsz >> 5)) {
+      if (offs[g + 1] == offs[g]) continue;
+      const SelInfo& N = info[g];
+      warp_chunk_prefix(W, W.node_chunks[N.csr] + N.a, N.n, W.cpref + N.a);
+      ++nodes;
+    }
+    if ((threadIdx.x & 31) == 0 && nodes) atomicAdd(&W.ctr[LPG_CTR_SEL_NODE_ROUNDS], (unsigned long long)nodes);
+    if (!(ok = grid_sync(W.grid_bar, W.wait_spin))) break;
   }
+  if (gtid == 0) *W.sel_done = round;
   /* a CTA that never reached the barrier: the round is incomplete, and the
    * barrier's count is no longer to be trusted, so every replicate stops */
   if (!ok && threadIdx.x == 0)
@@ -2837,14 +2753,14 @@ __global__ void __launch_bounds__(256, 3) k_sel_round0(DevWorld W) {
       if (W.reps[r].active) W.reps[r].error = LPG_ERR_TIMEOUT;
 }
 
-/* Later rounds (after the round 0 claims): one CTA per node that still
+/* Later rounds (after k_sel_round0's): one CTA per node that still
  * lacks agents, rounds of its remaining target count over its current
  * weights until the node is served or has no susceptible weight left; then
  * the end of the tick (end_tick) for the CTA's nodes.  All threads of the
  * CTA run sel_rounds. */
 __device__ __noinline__ void sel_rounds(DevWorld& W);
 __device__ void end_tick(DevWorld& W, int64_t g0, int64_t gstride);
-__global__ void __launch_bounds__(256) k_sel_rounds(DevWorld W) {
+__global__ void __launch_bounds__(256, 2) k_sel_rounds(DevWorld W) {
   pdl_begin();
   const int R = W.n_reps;
   int any = 0;
@@ -2862,7 +2778,7 @@ __device__ __noinline__ void sel_rounds(DevWorld& W) {
 
   __shared__ int64_t s_k;
   __shared__ uint64_t s_T;
-  __shared__ unsigned int s_won;
+  __shared__ unsigned int s_won, s_strain[LPG_MAX_STRAINS];
   __shared__ unsigned long long s_wsum;
   __shared__ SelInfo s_N;
   __shared__ int32_t s_need[256];
@@ -2897,14 +2813,15 @@ __device__ __noinline__ void sel_rounds(DevWorld& W) {
     const bool local = n <= LPG_SEL_OFFS;
     /* this node's region of the target buffer: its own positions */
     uint32_t* hits = W.hits + (int64_t)(rp->chunk_base + a) * LPG_CHUNK;
-    for (int round = 1; round < LPG_MAX_ROUNDS; ++round) {
+    const int first = *W.sel_done; /* the rounds before were the grid's */
+    for (int round = first; round < LPG_MAX_ROUNDS; ++round) {
       if (threadIdx.x == 0) {
-        /* round 1 from the node's totals after round 0; later rounds from the
+        /* the first from the node's totals after the grid's rounds; later ones from the
          * previous round's claims, all made by this CTA (the totals equal
          * these values: size - uniq, and sw less the claimed weights) */
         int64_t k;
         uint64_t T;
-        if (round == 1) {
+        if (round == first) {
           k = __ldcg(&W.size[g]) - (int64_t)__ldcg((const unsigned long long*)&W.uniq[g]);
           T = __ldcg(&W.sw[g]);
         } else {
@@ -2915,15 +2832,13 @@ __device__ __noinline__ void sel_rounds(DevWorld& W) {
         s_k = (k > 0 && T > 0) ? k : 0;
         s_won = 0;
         s_wsum = 0;
+#pragma unroll
+        for (int s = 0; s < LPG_MAX_STRAINS; ++s) s_strain[s] = 0;
         if (s_k > 0) {
           atomicAdd(&W.ctr[LPG_CTR_SEL_TARGETS], (unsigned long long)s_k);
           atomicAdd(&W.ctr[LPG_CTR_SEL_NODE_ROUNDS], 1ULL);
-          if (round == 1) { /* the node's strain thresholds are the same every round */
-            s_N.seed = rp->seed;
-            s_N.t = rp->cur_t;
-            s_N.ns = rp->ns;
-            sel_strain_cum(W, rp, g, s_N.thr);
-          }
+          /* the node's strain thresholds are the same every round */
+          if (round == first) s_N = reinterpret_cast<const SelInfo*>(W.sel_info)[g];
         }
       }
       __syncthreads();
@@ -2955,29 +2870,48 @@ __device__ __noinline__ void sel_rounds(DevWorld& W) {
         carry += (uint64_t)tot;
       }
       __syncthreads();
-      int TT = 1;
-      while (TT < 32 && (int64_t)(2 * TT) * k <= (int64_t)blockDim.x) TT *= 2;
-      const Team tm = make_team(TT);
-      for (int64_t j = threadIdx.x / TT; __any_sync(FULLMASK, j < k); j += blockDim.x / TT) {
+      /* every target located, then claimed: the first 256 (target l * 32 +
+       * team on lane l of a team of 8) kept in registers in between, later
+       * ones' slots in hits */
+      Located L0;
+      const int64_t j0 = (threadIdx.x & 7) * 32 + threadIdx.x / 8;
+#pragma unroll 1
+      for (int64_t j = j0, jw = 0; jw < k; j += 256, jw += 256) {
         const bool act = j < k;
-        const uint64_t v = act ? lpg_scale_target(lpg_u53(rp->seed, LPG_P_SELECT, rp->cur_t, (uint64_t)i, (uint64_t)round, (uint64_t)j), T) : 0;
-        const uint32_t hit = locate_team(W, tm, ls, local ? s_cp : cp, n, v, 0, act);
-        if (act && tm.l == 0) {
-          if (hit == LPG_NONE) W.reps[W.node_rep[g]].error = LPG_ERR_INTERNAL;
-          hits[j] = hit;
-        }
+        const uint64_t v = act ? lpg_scale_target(lpg_u53(s_N.seed, LPG_P_SELECT, s_N.t, (uint64_t)i, (uint64_t)round, (uint64_t)j), T) : 0;
+        Located L;
+        locate_batch<false>(W, ls, local ? s_cp : cp, n, v, act, &L);
+        if (act && L.hit == LPG_NONE) W.reps[W.node_rep[g]].error = LPG_ERR_INTERNAL;
+        if (jw == 0) L0 = L;
+        else if (act) hits[j] = L.hit;
       }
       __syncthreads();
-      for (int64_t j = threadIdx.x; j < k; j += blockDim.x) {
-        const uint32_t hit = hits[j];
-        uint64_t w = 0;
-        if (hit != LPG_NONE && claim(W, hit, g, s_N, &w)) {
+#pragma unroll 1
+      for (int64_t j = j0; j < k; j += 256) {
+        if (j != j0) {
+          L0.hit = hits[j];
+          if (L0.hit != LPG_NONE) {
+            L0.word = *reinterpret_cast<volatile uint32_t*>(W.ds + ((int64_t)L0.hit & ~3LL));
+            L0.ref = W.ref[L0.hit];
+            L0.et = W.et[L0.hit];
+            L0.w = fix_risk(W.risk[L0.hit]);
+          }
+        }
+        if (L0.hit == LPG_NONE) continue;
+        const int s = claim(W, L0, s_N, 1);
+        if (s >= 0) {
           atomicAdd(&s_won, 1u);
-          if (w) atomicAdd(&s_wsum, (unsigned long long)w);
+          atomicAdd(&s_strain[s], 1u);
+          if (L0.w) atomicAdd(&s_wsum, (unsigned long long)L0.w);
         }
       }
       __threadfence_block();
       __syncthreads();
+      if (threadIdx.x == 0 && s_won) {
+        node_exposed(W, g, (int)s_won, s_wsum);
+        for (int s = 0; s < s_N.ns; ++s)
+          if (s_strain[s]) node_strain(W, g, s, (int)s_strain[s]);
+      }
     }
   }
 }
