@@ -293,13 +293,7 @@ __device__ __forceinline__ void scatter_one(const DevWorld& W, const ScatterArgs
   const int64_t rk = a.rank ? (int64_t)a.rank[i] : i - a.node_first[n];
   const int64_t pos = (int64_t)a.node_chunk0[n] * LPG_CHUNK + rk; /* a node's chunks are consecutive */
   W.ds[pos] = a.s.ds[i];
-  W.strain[pos] = a.s.strain[i];
-  W.et[pos] = a.s.et[i];
-  W.it[pos] = a.s.it[i];
-  W.pt[pos] = a.s.pt[i];
-  W.pp[pos] = a.s.pp[i];
-  W.par[pos] = a.s.par[i];
-  W.ipv[pos] = a.s.ipv[i];
+  rec_put(W.rec + pos, AgentRec{a.s.strain[i], a.s.et[i], a.s.it[i], a.s.pt[i], a.s.pp[i], a.s.par[i], a.s.ipv[i], 0});
   W.cm[pos] = a.s.cm[i];
   W.ri[pos] = a.s.ri[i];
   W.risk[pos] = a.s.risk[i];
@@ -312,13 +306,31 @@ __device__ __forceinline__ void scatter_one(const DevWorld& W, const ScatterArgs
 /* 16 slots of one column from 16 consecutive agents: element loads (the
  * source run may start anywhere), packed into 16-byte stores (the slots
  * start at a multiple of 16). */
+__device__ __forceinline__ uint32_t get4(const int8_t* __restrict__ src) {
+  return (uint32_t)(uint8_t)__ldg(src) | (uint32_t)(uint8_t)__ldg(src + 1) << 8 |
+         (uint32_t)(uint8_t)__ldg(src + 2) << 16 | (uint32_t)(uint8_t)__ldg(src + 3) << 24;
+}
 __device__ __forceinline__ void fill16(int8_t* __restrict__ dst, const int8_t* __restrict__ src) {
-  uint32_t w[4];
+  *reinterpret_cast<uint4*>(dst) = make_uint4(get4(src), get4(src + 4), get4(src + 8), get4(src + 12));
+}
+/* Byte k of a, b, c, d as word k (a 4 x 4 byte transpose). */
+__device__ __forceinline__ uint4 bytes4x4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  const uint32_t ab = __byte_perm(a, b, 0x5140), AB = __byte_perm(a, b, 0x7362);
+  const uint32_t cd = __byte_perm(c, d, 0x5140), CD = __byte_perm(c, d, 0x7362);
+  return make_uint4(__byte_perm(ab, cd, 0x5410), __byte_perm(ab, cd, 0x7632), __byte_perm(AB, CD, 0x5410),
+                    __byte_perm(AB, CD, 0x7632));
+}
+/* 16 agents' records from their seven byte columns. */
+__device__ __forceinline__ void fill_rec16(AgentRec* __restrict__ dst, const Staging& s, int64_t i0) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    w[j] = (uint32_t)(uint8_t)__ldg(src + 4 * j) | (uint32_t)(uint8_t)__ldg(src + 4 * j + 1) << 8 |
-           (uint32_t)(uint8_t)__ldg(src + 4 * j + 2) << 16 | (uint32_t)(uint8_t)__ldg(src + 4 * j + 3) << 24;
-  *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+  for (int j = 0; j < 4; ++j) {
+    const int64_t i = i0 + 4 * j;
+    const uint4 lo = bytes4x4(get4(s.strain + i), get4(s.et + i), get4(s.it + i), get4(s.pt + i));
+    const uint4 hi = bytes4x4(get4(s.pp + i), get4(s.par + i), get4(s.ipv + i), 0);
+    uint4* o = reinterpret_cast<uint4*>(dst + 4 * j);
+    o[0] = make_uint4(lo.x, hi.x, lo.y, hi.y);
+    o[1] = make_uint4(lo.z, hi.z, lo.w, hi.w);
+  }
 }
 __device__ __forceinline__ void fill16(uint8_t* dst, const uint8_t* src) {
   fill16(reinterpret_cast<int8_t*>(dst), reinterpret_cast<const int8_t*>(src));
@@ -358,13 +370,7 @@ __global__ void k_scatter_sorted(DevWorld W, ScatterArgs a, int32_t chunk_base, 
     const int64_t p0 = cid * LPG_CHUNK + o0;
     if (o0 + 16 <= meta.y) {
       fill16(W.ds + p0, a.s.ds + i0);
-      fill16(W.strain + p0, a.s.strain + i0);
-      fill16(W.et + p0, a.s.et + i0);
-      fill16(W.it + p0, a.s.it + i0);
-      fill16(W.pt + p0, a.s.pt + i0);
-      fill16(W.pp + p0, a.s.pp + i0);
-      fill16(W.par + p0, a.s.par + i0);
-      fill16(W.ipv + p0, a.s.ipv + i0);
+      fill_rec16(W.rec + p0, a.s, i0);
       fill16(W.cm + p0, a.s.cm + i0);
       fill16(W.ri + p0, a.s.ri + i0);
       fill16_32(W.risk + p0, a.s.risk + i0);
@@ -410,9 +416,10 @@ __global__ void k_gather(DevWorld W, Staging s, int32_t chunk_base, int32_t used
     if (o >= meta.y) continue;
     int64_t pos = cid * LPG_CHUNK + o;
     uint32_t i = W.ref[pos];
-    const int8_t ds = W.ds[pos], st = W.strain[pos], pp = W.pp[pos];
+    const AgentRec ar = rec_get(W.rec + pos);
+    const int8_t ds = W.ds[pos], st = ar.strain, pp = ar.pp;
     const uint8_t cm = W.cm[pos];
-    int8_t et = W.et[pos], it = W.it[pos], pt = W.pt[pos];
+    int8_t et = ar.et, it = ar.it, pt = ar.pt;
     if (ds_on && (ds == 1 || ds == 2)) /* the count-downs up to the step of tick tc */
       ev_advance(ds, st, et, it, pt, tc - W.evt[pos] + 1 + ev_pure(ds, st, et, it, pt, pp));
     put(s.ds, i, ds);
@@ -421,8 +428,8 @@ __global__ void k_gather(DevWorld W, Staging s, int32_t chunk_base, int32_t used
     put(s.it, i, it);
     put(s.pt, i, pt);
     put(s.pp, i, pp);
-    put(s.par, i, W.par[pos]);
-    put(s.ipv, i, W.ipv[pos]);
+    put(s.par, i, ar.par);
+    put(s.ipv, i, ar.ipv);
     put(s.cm, i, cm);
     put(s.node, i, (int16_t)(meta.x - node_base));
     int16_t ri = W.ri[pos];
@@ -821,13 +828,7 @@ extern "C" int lpg_start(lpg_handle* h) {
   const int64_t P = (int64_t)chunk_total * LPG_CHUNK;
   Carve carve;
   carve.add(&W.ds, P);
-  carve.add(&W.strain, P);
-  carve.add(&W.et, P);
-  carve.add(&W.it, P);
-  carve.add(&W.pt, P);
-  carve.add(&W.pp, P);
-  carve.add(&W.par, P);
-  carve.add(&W.ipv, P);
+  carve.add(&W.rec, P);
   carve.add(&W.cm, P);
   carve.add(&W.ri, P);
   carve.add(&W.risk, P);
@@ -870,11 +871,7 @@ extern "C" int lpg_start(lpg_handle* h) {
   carve.add(&W.tgt_off, G + 1);
   uint8_t* sel_info = nullptr;
   carve.add(&sel_info, (size_t)G * sizeof(SelInfo));
-  /* selection targets (at most the susceptibles) and the E/I queue slabs
-   * (at most one entry per position) share this buffer */
-  int64_t hits = (int64_t)chunk_total * LPG_CHUNK;
-  W.hits_cap = hits;
-  carve.add(&W.hits, hits);
+  W.hits_cap = (int64_t)chunk_total * LPG_CHUNK; /* one target per position (in the event queues' memory) */
   carve.add(&W.ctr, LPG_NUM_COUNTERS);
   carve.add(&W.end_done, 1);
   carve.add(&W.grid_bar, 1);
@@ -904,6 +901,7 @@ extern "C" int lpg_start(lpg_handle* h) {
     carve.add(&rp.pl_inf, np);
   }
   if (carve.commit(h)) return LPG_ERR_NOMEM;
+  W.hits = reinterpret_cast<uint32_t*>(W.evq);
   W.sel_info = sel_info;
   CK(cudaMemsetAsync(W.ds, 0xff, P, st));
   CK(cudaMemsetAsync(W.ref, 0xff, P * 4, st));

@@ -159,6 +159,27 @@ typedef struct {
   int32_t ei_sum;      /* k_end: nodes with E > 0 plus nodes with I > 0 (the next tick's stop rule) */
 } DevRep;
 
+/* What an agent's event touches beside its state: one 8-byte record, so that
+ * an event reads and writes one memory sector where seven byte columns cost
+ * seven. */
+struct __align__(8) AgentRec {
+  int8_t strain, et, it, pt, pp, par, ipv, unused;
+};
+#ifdef __CUDACC__
+/* The whole record in one 8-byte access. */
+__device__ __forceinline__ AgentRec rec_get(const AgentRec* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return AgentRec{(int8_t)u.x, (int8_t)(u.x >> 8), (int8_t)(u.x >> 16), (int8_t)(u.x >> 24),
+                  (int8_t)u.y, (int8_t)(u.y >> 8), (int8_t)(u.y >> 16), 0};
+}
+__device__ __forceinline__ void rec_put(AgentRec* p, const AgentRec& a) {
+  const uint32_t lo = (uint32_t)(uint8_t)a.strain | (uint32_t)(uint8_t)a.et << 8 | (uint32_t)(uint8_t)a.it << 16 |
+                      (uint32_t)(uint8_t)a.pt << 24;
+  const uint32_t hi = (uint32_t)(uint8_t)a.pp | (uint32_t)(uint8_t)a.par << 8 | (uint32_t)(uint8_t)a.ipv << 16;
+  *reinterpret_cast<uint2*>(p) = make_uint2(lo, hi);
+}
+#endif
+
 /* Global device state shared by the kernels of one handle. */
 typedef struct {
   int32_t n_reps, G; /* replicates, global nodes */
@@ -168,7 +189,8 @@ typedef struct {
   int64_t wait_spin;   /* iterations of the staged sweep's consumer waits before they give up */
   DevRep* reps;
   /* per position */
-  int8_t *ds, *strain, *et, *it, *pt, *pp, *par, *ipv;
+  int8_t* ds;
+  AgentRec* rec;
   uint8_t* cm;
   int16_t* ri; /* where RI runs: alive, not chronically-missed agents keep the timer before their
                   first RI tick (lpg_ri.h); the dead keep the value they died with */
@@ -208,7 +230,7 @@ typedef struct {
   int64_t* ksel;
   int64_t* tgt_off; /* [G + 1] */
   void* sel_info;     /* [G] SelInfo: per-node selection record of the tick */
-  uint32_t* hits; /* selection targets */
+  uint32_t* hits; /* selection targets: the event queues' memory, which the sweeps have finished with */
   int32_t* sel_done; /* rounds of the tick's selection that k_sel_round0 made */
   int64_t hits_cap;
   uint64_t* evq;     /* event queues of the sweeps: one slab per sweep CTA */

@@ -460,16 +460,10 @@ __global__ void __launch_bounds__(256) k_newborns(DevWorld W) {
       const int64_t pos = (int64_t)cid * LPG_CHUNK + off;
       const int64_t ref = rp->count_before + j;
       const int64_t q = ref - rp->count0;
-      W.et[pos] = rp->pl_et[q];
-      W.it[pos] = rp->pl_it[q];
-      W.pt[pos] = rp->pl_pt[q];
-      W.strain[pos] = rp->pl_strain[q];
       const int8_t pp = rp->pl_pp[q], par = rp->pl_par[q];
       const uint8_t cm = rp->pl_cm[q];
       const int16_t ri = rp->pl_ri[q];
-      W.pp[pos] = pp;
-      W.par[pos] = par;
-      W.ipv[pos] = rp->pl_ipv[q];
+      rec_put(W.rec + pos, AgentRec{rp->pl_strain[q], rp->pl_et[q], rp->pl_it[q], rp->pl_pt[q], pp, par, rp->pl_ipv[q], 0});
       W.cm[pos] = cm;
       W.ri[pos] = ri;
       const float risk = rp->pl_risk[q];
@@ -1265,6 +1259,7 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
     const int t = rp->cur_t;
     if (kind == QA_DEATH) {
       const int8_t s = (int8_t)(uint8_t)(e >> 48);
+      const AgentRec a = rec_get(W.rec + pos);
       nDead = 1;
       if (s == 0) {
         dS = -1;
@@ -1275,7 +1270,7 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
           atomicAdd((unsigned long long*)&W.sub_w[cid * LPG_NSUB + (pos % LPG_CHUNK) / LPG_SUB], neg64(w));
         }
       } else if (s == 1 || s == 2) {
-        st = W.strain[pos];
+        st = a.strain;
         if (s == 1) {
           dE = -1;
         } else {
@@ -1284,14 +1279,14 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
         }
         /* timers frozen at death: brought up to the step of t - 1 (they
          * count down only where disease states are stepped) */
-        int8_t et = W.et[pos], it = W.it[pos], pt = W.pt[pos];
-        const int k = (rp->comps & LPG_COMP_DS) ? t - W.evt[pos] + ev_pure(s, (int8_t)st, et, it, pt, W.pp[pos]) : 0;
+        int8_t et = a.et, it = a.it, pt = a.pt;
+        const int k = (rp->comps & LPG_COMP_DS) ? t - W.evt[pos] + ev_pure(s, (int8_t)st, et, it, pt, a.pp) : 0;
         if (k > 0) {
           ev_advance(s, (int8_t)st, et, it, pt, k);
-          if (s == 1) W.et[pos] = et;
+          if (s == 1) W.rec[pos].et = et;
           else {
-            W.it[pos] = it;
-            if (st == 0) W.pt[pos] = pt;
+            W.rec[pos].it = it;
+            if (st == 0) W.rec[pos].pt = pt;
           }
         }
       } else if (s == 3) {
@@ -1299,14 +1294,15 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
       }
       /* the RI timer stops at death: its value after the RI ticks before t */
       if (ri_runs(rp) && W.cm[pos] != 1) W.ri[pos] = ri_now(rp, W.ri[pos], W.ref[pos], W.dob[pos], t - 1);
-      if (W.pp[pos] == 1) dPP -= 1;
-      if (W.par[pos] == 1) dP -= 1;
+      if (a.pp == 1) dPP -= 1;
+      if (a.par == 1) dP -= 1;
     } else {
       /* an event step of an agent in E or I (its evt is t) */
       const int8_t s0 = W.ds[pos];
       int8_t s = s0;
-      st = W.strain[pos];
-      int8_t et = W.et[pos], it = W.it[pos], pt = W.pt[pos], pp = W.pp[pos];
+      AgentRec a = rec_get(W.rec + pos);
+      st = a.strain;
+      int8_t et = a.et, it = a.it, pt = a.pt, pp = a.pp;
       const float inf = W.inf[pos]; /* most events are a move; requested with the timers */
       /* the count-downs skipped since the timers were last brought up to date */
       ev_advance(s0, (int8_t)st, et, it, pt, t - W.evt[pos] + ev_pure(s0, (int8_t)st, et, it, pt, pp));
@@ -1317,7 +1313,7 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
           dI += 1;
         }
         et = dec_i8(et);
-        W.et[pos] = et;
+        a.et = et;
       }
       if (s == 2) {
         if (it <= 0) {
@@ -1326,29 +1322,28 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
           dR += 1;
         }
         it = dec_i8(it);
-        W.it[pos] = it;
+        a.it = it;
         if (st == 0) {
           if (pt <= 0 && pp == -1) {
-            const int8_t ipv = W.ipv[pos];
-            const uint32_t ref = W.ref[pos];
-            if (ipv == 0) {
+            if (a.ipv == 0) {
               pp = 1;
               dPP += 1;
               nPP += 1;
-              if (lpg_u53(rp->seed, LPG_P_PARALYSIS, t, ref, 0, 0) < rp->thr_par) {
-                W.par[pos] = 1;
+              if (lpg_u53(rp->seed, LPG_P_PARALYSIS, t, W.ref[pos], 0, 0) < rp->thr_par) {
+                a.par = 1;
                 dP += 1;
                 nP += 1;
               }
             } else {
               pp = 0;
             }
-            W.pp[pos] = pp;
+            a.pp = pp;
           }
           pt = dec_i8(pt);
-          W.pt[pos] = pt;
+          a.pt = pt;
         }
       }
+      if (s0 == 1 || s0 == 2) rec_put(W.rec + pos, a);
       if (s != s0) W.ds[pos] = s;
       if (dI != 0) { /* into I or out of it, not both */
         const uint64_t bw = fix_beta(inf, rp->strain_scal[st]);
@@ -1392,11 +1387,13 @@ __device__ __forceinline__ void ds_queue_step(DevWorld& W, uint64_t e, bool on) 
  * queued agents (ds_queue_step).  A CTA's queue slab starts at its first
  * item times 128 entries of evq.
  *
- * Bound by random DRAM sectors (640 B a sub-block, about six sectors read
- * and three written an event) and, where few nodes hold the outbreak, by
- * atomics on one address: infectivity is added once a warp and node, not
- * once an event.  774 nodes, 2.2e8 agents, 365 ticks: 39 to 34.5 ms; 70
- * nodes with 2.2e5 events in a tick: 99 to 59 us. */
+ * Bound by random DRAM sectors: 640 B a sub-block; an event reads its
+ * agent's record and infectivity and writes the record and the event tick
+ * (AgentRec: seven byte columns took six sectors more).  Where few nodes
+ * hold the outbreak the atomics on one address count as well: infectivity
+ * is added once a warp and node, not once an event.  774 nodes, 2.2e8
+ * agents, 365 ticks: 39 ms, 34.5 with the sums per warp, 30.4 with the
+ * records; 70 nodes with 2.2e5 events in a tick: 99, 59 and 49 us. */
 __global__ void __launch_bounds__(LPG_SWEEP_BLOCK) k_sweep_due(DevWorld W) {
   pdl_begin();
   __shared__ uint32_t s_qcnt;
@@ -1542,7 +1539,7 @@ __global__ void __launch_bounds__(256) k_evb(DevWorld W, int nslabs) {
           rivac = 1;
           if (s == 0) {
             s = 1;
-            W.strain[pos] = (int8_t)rp->ri_strain;
+            W.rec[pos].strain = (int8_t)rp->ri_strain;
             riprot = 1;
             dE[rp->ri_strain] += 1;
             exposed = true;
@@ -1550,7 +1547,7 @@ __global__ void __launch_bounds__(256) k_evb(DevWorld W, int nslabs) {
         }
         if (lpg_u53(rp->seed, LPG_P_RI, t, ref, 0, 1) < rp->thr_ipv[ni]) {
           ipvvac = 1;
-          W.ipv[pos] = 1;
+          W.rec[pos].ipv = 1;
         }
       }
       nsia = rp->sia_n;
@@ -1564,7 +1561,7 @@ __global__ void __launch_bounds__(256) k_evb(DevWorld W, int nslabs) {
           sv[k] = 1;
           if (s == 0 && r < ev.thr_pro[ni]) {
             s = 1;
-            W.strain[pos] = (int8_t)ev.strain;
+            W.rec[pos].strain = (int8_t)ev.strain;
             sp[k] = 1;
             dE[ev.strain] += 1;
             exposed = true;
@@ -1573,7 +1570,7 @@ __global__ void __launch_bounds__(256) k_evb(DevWorld W, int nslabs) {
       }
       if (exposed) {
         dS = -1;
-        const int8_t et = W.et[pos];
+        const int8_t et = W.rec[pos].et;
         ex_e1 = t + 1 + (et > 0 ? et : 0);
         W.evt[pos] = ex_e1;
         ex_w = fix_risk(W.risk[pos]);
@@ -1742,17 +1739,14 @@ __global__ void __launch_bounds__(1024) k_seed(DevWorld W) {
         pos = s_tie_pos[k];
       }
       int8_t s = W.ds[pos];
-      int sti = W.strain[pos];
+      AgentRec a = rec_get(W.rec + pos);
+      int sti = a.strain;
       const int64_t cid = pos / LPG_CHUNK;
       if (s == 1 || s == 2) {
         /* timers up to this tick's step, which has run */
-        int8_t et = W.et[pos], it = W.it[pos], pt = W.pt[pos];
-        const int k = t - W.evt[pos] + 1 + ev_pure(s, (int8_t)sti, et, it, pt, W.pp[pos]);
+        const int k = t - W.evt[pos] + 1 + ev_pure(s, (int8_t)sti, a.et, a.it, a.pt, a.pp);
         if (k > 0) {
-          ev_advance(s, (int8_t)sti, et, it, pt, k);
-          W.et[pos] = et;
-          W.it[pos] = it;
-          W.pt[pos] = pt;
+          ev_advance(s, (int8_t)sti, a.et, a.it, a.pt, k);
         }
       }
       if (s != 2) {
@@ -1774,13 +1768,14 @@ __global__ void __launch_bounds__(1024) k_seed(DevWorld W) {
         if (bw) atomicAdd((unsigned long long*)&W.bb[(int64_t)sti * G + g], (unsigned long long)bw);
         W.ds[pos] = 2;
       }
-      if (W.it[pos] <= 0) {
+      if (a.it <= 0) {
         lpg_stream sm;
         lpg_stream_init(&sm, rp->seed, LPG_P_SEEDTIMER, t, W.ref[pos], (uint64_t)ev.pad);
-        W.it[pos] = lpg_trunc_i8(lpg_dist_sample(&sm, rp->dur_kind, rp->dur_p1, rp->dur_p2));
+        a.it = lpg_trunc_i8(lpg_dist_sample(&sm, rp->dur_kind, rp->dur_p1, rp->dur_p2));
       }
+      rec_put(W.rec + pos, a);
       {
-        const int32_t e1 = t + 1 + ev_pure(2, (int8_t)sti, W.et[pos], W.it[pos], W.pt[pos], W.pp[pos]);
+        const int32_t e1 = t + 1 + ev_pure(2, (int8_t)sti, a.et, a.it, a.pt, a.pp);
         W.evt[pos] = e1;
         atomicMin(&W.sub_evt[pos >> 7], e1);
       }
@@ -2290,7 +2285,7 @@ __device__ __forceinline__ int expose_claimed(DevWorld& W, int64_t pos, const Se
       s = k;
       found = true;
     }
-  W.strain[pos] = (int8_t)s;
+  W.rec[pos].strain = (int8_t)s;
   {
     /* first step in E is at t + 1 (model.py:393-454) */
     const int32_t e1 = N.t + 1 + (et > 0 ? et : 0);
@@ -2592,7 +2587,7 @@ __device__ __forceinline__ void locate_batch(const DevWorld& W, const int32_t* l
       out->w = hw;
       if (hit != LPG_NONE) { /* requested here, used at the claim */
         out->ref = W.ref[hit];
-        out->et = W.et[hit];
+        out->et = W.rec[hit].et;
       }
     }
   }
@@ -2933,7 +2928,7 @@ __device__ __noinline__ void sel_rounds(DevWorld& W) {
           if (L0.hit != LPG_NONE) {
             L0.word = *reinterpret_cast<volatile uint32_t*>(W.ds + ((int64_t)L0.hit & ~3LL));
             L0.ref = W.ref[L0.hit];
-            L0.et = W.et[L0.hit];
+            L0.et = W.rec[L0.hit].et;
             L0.w = fix_risk(W.risk[L0.hit]);
           }
         }
@@ -3121,7 +3116,8 @@ __global__ void k_init_events(DevWorld W, int32_t* evt, int32_t* sub_evt, int tm
       const int64_t pos = (int64_t)rp->chunk_base * LPG_CHUNK + q;
       const int8_t ds = W.ds[pos];
       if (ds != 1 && ds != 2) continue;
-      const int32_t e = tm + 1 + ev_pure(ds, W.strain[pos], W.et[pos], W.it[pos], W.pt[pos], W.pp[pos]);
+      const AgentRec a = rec_get(W.rec + pos);
+      const int32_t e = tm + 1 + ev_pure(ds, a.strain, a.et, a.it, a.pt, a.pp);
       evt[pos] = e;
       atomicMin(&sub_evt[pos >> 7], e);
     }
@@ -3213,11 +3209,12 @@ __global__ void __launch_bounds__(LPG_SWEEP_THREADS) k_count(DevWorld W, int32_t
         const int64_t pos = cid * LPG_CHUNK + o;
         const int8_t s = o < fill ? W.ds[pos] : (int8_t)-1;
         const bool alive = s >= 0;
-        const int st = alive ? W.strain[pos] : 0;
+        const AgentRec a = alive ? rec_get(W.rec + pos) : AgentRec{};
+        const int st = a.strain;
         const int32_t dod = alive ? W.dod[pos] : LPG_NO_DOD;
         const uint64_t w = s == 0 ? fix_risk(W.risk[pos]) : 0;
         const uint64_t bw = s == 2 ? fix_beta(W.inf[pos], rp->strain_scal[st]) : 0;
-        const bool potp = alive && W.pp[pos] == 1, par = alive && W.par[pos] == 1;
+        const bool potp = a.pp == 1, par = a.par == 1;
         const int32_t dmin = __reduce_min_sync(FULLMASK, dod);
         const int nS = __popc(__ballot_sync(FULLMASK, s == 0)), nR = __popc(__ballot_sync(FULLMASK, s == 3));
         const int nPotp = __popc(__ballot_sync(FULLMASK, potp)), nPar = __popc(__ballot_sync(FULLMASK, par));
