@@ -105,10 +105,21 @@ __device__ __forceinline__ uint64_t fix_beta(float inf, double scal) {
 /* Three-word (192-bit) unsigned accumulators with the carry chain in PTX:
  * acc3_mul adds the 128-bit product x*y, acc3_add another accumulator. */
 __device__ __forceinline__ void acc3_mul(uint64_t& a0, uint64_t& a1, uint64_t& a2, uint64_t x, uint64_t y) {
-  const uint64_t lo = x * y, hi = __umul64hi(x, y);
-  asm("add.cc.u64 %0, %0, %3;\n\taddc.cc.u64 %1, %1, %4;\n\taddc.u64 %2, %2, 0;"
-      : "+l"(a0), "+l"(a1), "+l"(a2)
-      : "l"(lo), "l"(hi));
+  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), y0 = (uint32_t)y, y1 = (uint32_t)(y >> 32);
+  uint32_t w0 = (uint32_t)a0, w1 = (uint32_t)(a0 >> 32), w2 = (uint32_t)a1, w3 = (uint32_t)(a1 >> 32),
+           w4 = (uint32_t)a2, w5 = (uint32_t)(a2 >> 32);
+  asm("mad.lo.cc.u32 %0, %6, %8, %0;\n\tmadc.hi.cc.u32 %1, %6, %8, %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9, %2;\n\tmadc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+      "addc.cc.u32 %4, %4, 0;\n\taddc.u32 %5, %5, 0;\n\t"
+      "mad.lo.cc.u32 %1, %6, %9, %1;\n\tmadc.hi.cc.u32 %2, %6, %9, %2;\n\t"
+      "addc.cc.u32 %3, %3, 0;\n\taddc.cc.u32 %4, %4, 0;\n\taddc.u32 %5, %5, 0;\n\t"
+      "mad.lo.cc.u32 %1, %7, %8, %1;\n\tmadc.hi.cc.u32 %2, %7, %8, %2;\n\t"
+      "addc.cc.u32 %3, %3, 0;\n\taddc.cc.u32 %4, %4, 0;\n\taddc.u32 %5, %5, 0;"
+      : "+r"(w0), "+r"(w1), "+r"(w2), "+r"(w3), "+r"(w4), "+r"(w5)
+      : "r"(x0), "r"(x1), "r"(y0), "r"(y1));
+  a0 = w0 | (uint64_t)w1 << 32;
+  a1 = w2 | (uint64_t)w3 << 32;
+  a2 = w4 | (uint64_t)w5 << 32;
 }
 __device__ __forceinline__ void acc3_add(uint64_t& a0, uint64_t& a1, uint64_t& a2, uint64_t b0, uint64_t b1,
                                          uint64_t b2) {
@@ -1866,7 +1877,10 @@ __device__ __forceinline__ void warp_chunk_prefix(const DevWorld& W, const int32
  * in units of 2^-40 times the network weight in its two fixed-point parts
  * (lpg_net_split; transposed row, contiguous), the two products summed in
  * three-word accumulators, one conversion (lpg_mix_value) into inck; an
- * exact sum does not depend on how the threads split it.  The fifth warp
+ * exact sum does not depend on how the threads split it.  Bound by issuing
+ * the 64-bit products (4000 nodes: 59% of the issue slots, a quarter of the
+ * DRAM rate); with the 32-bit multiply-add carry chains and one reduction a
+ * strain and row 137 to 129 us there, 17.3 to 15.6 us at 774 nodes.  The fifth warp
  * forms the node-local chunk prefix (exact in integers) meanwhile. */
 template <int MW>
 __global__ void __launch_bounds__(32 * (MW + 1), MW == 4 ? LPG_NODE_MIX_MIN_BLOCKS : 16) k_node_mix(DevWorld W) {
@@ -1888,50 +1902,47 @@ __global__ void __launch_bounds__(32 * (MW + 1), MW == 4 ? LPG_NODE_MIX_MIN_BLOC
   const ulonglong2* qrow = reinterpret_cast<const ulonglong2*>(rp->netq_t) + (int64_t)i * n;
   constexpr int NT = 32 * MW;
   constexpr int PER = 6; /* source nodes a thread takes per pass: PER x NT nodes a pass */
-  if (lane == 0)
-    for (int k = 0; k < ns; ++k)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) s_mix[wid][k][q] = 0;
-  /* per strain: A = sum B hi and R = sum B lo, three words each, exact;
-   * one strain at a time (six accumulators live).  Sources without
+  /* per strain: A = sum B hi and R = sum B lo, three words each, exact; one
+   * strain at a time over the whole row (six accumulators live, reduced
+   * once), the next pass's B requested a pass ahead.  Sources without
    * infectivity add nothing to an exact sum, so a network entry is loaded
-   * only where some strain's B is nonzero, and a strain whose B is zero
-   * across the warp's sources of the pass is skipped: the sums, and so the
-   * results, are those of the full product. */
-  /* the same number of passes for every thread (the shuffles below need
-   * all 32 lanes), loads past the last node predicated off */
+   * only where the strain's B is nonzero, and a pass without any in the warp
+   * is skipped: the sums, and so the results, are those of the full product.
+   * The same number of passes for every thread (the shuffles below need all
+   * 32 lanes), loads past the last node predicated off. */
   const int npass = (n + PER * NT - 1) / (PER * NT);
-  for (int pass = 0; pass < npass; ++pass) {
-    const int ii0 = pass * PER * NT + threadIdx.x;
-    unsigned need = 0; /* bit u: source ii0 + u NT has infectivity of some strain */
-    for (int k = 0; k < ns; ++k) {
-#pragma unroll
-      for (int u = 0; u < PER; ++u) {
-        const int ii = ii0 + u * NT;
-        if (ii < n && W.bb[(int64_t)k * G + nb + ii] != 0) need |= 1u << u;
-      }
-    }
-    if (!__any_sync(FULLMASK, need != 0)) continue; /* warp-uniform */
-    ulonglong2 w[PER];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) w[u] = (need >> u) & 1 ? qrow[ii0 + u * NT] : make_ulonglong2(0, 0);
 #pragma unroll 1
-    for (int k = 0; k < ns; ++k) {
+  for (int k = 0; k < ns; ++k) {
+    const uint64_t* bb = W.bb + (int64_t)k * G + nb;
+    uint64_t a0 = 0, a1 = 0, a2 = 0, r0 = 0, r1 = 0, r2 = 0;
+    uint64_t nx[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int ii = threadIdx.x + u * NT;
+      nx[u] = ii < n ? bb[ii] : 0;
+    }
+    for (int pass = 0; pass < npass; ++pass) {
+      const int ii0 = pass * PER * NT + threadIdx.x;
       uint64_t b[PER];
       bool any = false;
 #pragma unroll
       for (int u = 0; u < PER; ++u) {
-        const int ii = ii0 + u * NT;
-        b[u] = (need >> u) & 1 ? W.bb[(int64_t)k * G + nb + ii] : 0;
+        b[u] = nx[u];
         any |= b[u] != 0;
+        const int ii = ii0 + (PER + u) * NT;
+        nx[u] = ii < n ? bb[ii] : 0;
       }
       if (!__any_sync(FULLMASK, any)) continue; /* warp-uniform */
-      uint64_t a0 = 0, a1 = 0, a2 = 0, r0 = 0, r1 = 0, r2 = 0;
+      ulonglong2 w[PER];
+#pragma unroll
+      for (int u = 0; u < PER; ++u) w[u] = b[u] ? qrow[ii0 + u * NT] : make_ulonglong2(0, 0);
 #pragma unroll
       for (int u = 0; u < PER; ++u) {
         acc3_mul(a0, a1, a2, b[u], w[u].x);
         acc3_mul(r0, r1, r2, b[u], w[u].y);
       }
+    }
+    if (__any_sync(FULLMASK, (a0 | a1 | a2 | r0 | r1 | r2) != 0)) {
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
         const uint64_t x0 = __shfl_down_sync(FULLMASK, a0, off), x1 = __shfl_down_sync(FULLMASK, a1, off),
@@ -1941,10 +1952,14 @@ __global__ void __launch_bounds__(32 * (MW + 1), MW == 4 ? LPG_NODE_MIX_MIN_BLOC
                        y2 = __shfl_down_sync(FULLMASK, r2, off);
         acc3_add(r0, r1, r2, y0, y1, y2);
       }
-      if (lane == 0) {
-        acc3_add(s_mix[wid][k][0], s_mix[wid][k][1], s_mix[wid][k][2], a0, a1, a2);
-        acc3_add(s_mix[wid][k][3], s_mix[wid][k][4], s_mix[wid][k][5], r0, r1, r2);
-      }
+    }
+    if (lane == 0) {
+      s_mix[wid][k][0] = a0;
+      s_mix[wid][k][1] = a1;
+      s_mix[wid][k][2] = a2;
+      s_mix[wid][k][3] = r0;
+      s_mix[wid][k][4] = r1;
+      s_mix[wid][k][5] = r2;
     }
   }
   /* the four mixing warps only (the fifth may have left) */
@@ -2070,8 +2085,7 @@ __global__ void __launch_bounds__(LPG_NODE_TX_THREADS, LPG_NODE_TX_MIN_BLOCKS) k
 #pragma unroll
   for (int k = 0; k < LPG_MAX_STRAINS; ++k)
     if (k < ns) total_p = total_p + p[k];
-  /* strain thresholds of the selection, the
-   * divisions on their own lanes */
+  /* strain thresholds of the selection, the divisions on their own lanes */
   const double qk = pk / total_p;
   uint64_t thr[LPG_MAX_STRAINS];
   {
