@@ -114,7 +114,7 @@ struct lpg_handle {
   int rounds_blocks = 0; /* k_sel_rounds */
   int evb_blocks = 0;
   int newborn_blocks = 0; /* per replicate */
-  bool node_batch_tx = false;  /* the draws one node a thread (k_node_tx_lanes) */
+  int tx_per = 1;              /* nodes a CTA of k_node_tx, at most 32 */
   bool node_batch_mix = false; /* the mixing one warp a node (k_node_mix<1>) */
 };
 
@@ -819,8 +819,11 @@ extern "C" int lpg_start(lpg_handle* h) {
   DevWorld& W = h->W;
   W.n_reps = R;
   W.G = G;
-  h->node_batch_tx = G > LPG_NODE_BATCH_MIN_PER_SM * h->sm_count;
-  h->node_batch_mix = h->node_batch_tx && maxn <= LPG_NODE_BATCH_MAX_NODES;
+  /* one CTA of k_node_tx per SM: with more, the CTAs of an SM share its FP64
+   * pipe (a batch of 12: 24.3 us a tick with one, 25.1, 28.0 and 32.5 with
+   * two, three and four; 4000 nodes 33.3, 33.4, 36.0 and 43.9) */
+  h->tx_per = std::min(32, (G + h->sm_count - 1) / h->sm_count);
+  h->node_batch_mix = G > LPG_NODE_BATCH_MIN_PER_SM * h->sm_count && maxn <= LPG_NODE_BATCH_MAX_NODES;
   W.total_chunks = chunk_total;
   W.stall_after = h->test_stall_after;
   W.wait_spin = h->test_wait_spin > 0 ? h->test_wait_spin : LPG_MBAR_SPIN;
@@ -1235,8 +1238,7 @@ static int launch_one(lpg_handle* h, int k, bool timed) {
       else CK(launch_pdl(k_node_mix<LPG_NODE_MIX_WARPS>, dim3(G), dim3(LPG_NODE_MIX_THREADS), 0, st, W));
       break;
     case 8:
-      if (h->node_batch_tx) CK(launch_pdl(k_node_tx_lanes, dim3((G + 127) / 128), dim3(128), 0, st, W));
-      else CK(launch_pdl(k_node_tx, dim3(G), dim3(LPG_NODE_TX_THREADS), 0, st, W));
+      CK(launch_pdl(k_node_tx, dim3((G + h->tx_per - 1) / h->tx_per), dim3(32 * LPG_NODE_TX_WARPS), 0, st, W, h->tx_per));
       break;
     case 9: {
       /* cooperative: its CTAs meet at a grid barrier, so all must be resident */

@@ -1800,10 +1800,6 @@ __global__ void __launch_bounds__(1024) k_seed(DevWorld W) {
  * target needs one load to find everything about its node. */
 #define LPG_SEL_OFFS 2048 /* chunk prefixes of a node that k_sel_rounds keeps in shared memory */
 #define LPG_SEL_NODES 8192 /* k_sel_round0 keeps its target offsets in shared memory when G < this */
-#define LPG_NODE_TX_THREADS 64
-/* six CTAs of the node step per SM (at most 170 registers a thread): one
- * wave covers 912 nodes, so a 774-node tick needs no second wave */
-#define LPG_NODE_TX_MIN_BLOCKS 6
 /* the mixing step: MW warps of products and sums, one warp for the node's
  * chunk prefix.  MW = 4 for a simulation of hundreds of nodes (six CTAs per
  * SM, at most 68 registers a thread: 774 nodes in one wave); MW = 1 for a
@@ -1812,10 +1808,9 @@ __global__ void __launch_bounds__(1024) k_seed(DevWorld W) {
 #define LPG_NODE_MIX_WARPS 4
 #define LPG_NODE_MIX_THREADS (32 * (LPG_NODE_MIX_WARPS + 1))
 #define LPG_NODE_MIX_MIN_BLOCKS 6
-/* the node steps switch to their batch forms above this many nodes (six
- * CTAs of the per-node kernels per SM: more would take a second wave); the
- * mixing only when no simulation has more than LPG_NODE_BATCH_MAX_NODES
- * nodes: one warp then sweeps each network row in a few passes, where rows
+/* the mixing switches to MW = 1 above this many nodes (six CTAs per SM: more
+ * would take a second wave), when no simulation has more than
+ * LPG_NODE_BATCH_MAX_NODES nodes: one warp then sweeps each network row in a few passes, where rows
  * of thousands of sources keep the per-node form's four mixing warps */
 #define LPG_NODE_BATCH_MIN_PER_SM 6
 #define LPG_NODE_BATCH_MAX_NODES 512
@@ -1977,290 +1972,159 @@ __global__ void __launch_bounds__(32 * (MW + 1), MW == 4 ? LPG_NODE_MIX_MIN_BLOC
 }
 
 /* Node-level force of infection and exposure counts (model.py:1327-1407);
- * the same arithmetic, in the same order, as the oracle's lpo_node_tx,
- * from the incoming infectivity k_node_mix formed.  One CTA per node. */
-/* Lane k < ns of the second warp: this node's infectivity total of strain k
- * (the first warp's pre_bb). */
-__device__ __forceinline__ uint64_t pre_bb_w1(const DevWorld& W, int g, int lane, int ns) {
-  return lane < ns ? W.bb[(int64_t)lane * W.G + g] : 0;
-}
-
-__global__ void __launch_bounds__(LPG_NODE_TX_THREADS, LPG_NODE_TX_MIN_BLOCKS) k_node_tx(DevWorld W) {
+ * the same arithmetic, in the same order, as the oracle's lpo_node_tx, from
+ * the incoming infectivity k_node_mix formed.
+ *
+ * Bound by chains of double-precision operations (65 cycles each, whether
+ * one lane of the warp works or 32).  So a CTA takes `per` nodes (at most
+ * 32), one a lane, and its warps take the parts that can run side by side:
+ * first strain k's
+ * probability on warp k, beside the gamma variate of the nodes without local
+ * infectivity on the fifth; then the exposure counts, each way to draw a
+ * Poisson variate (inversion from 0, inversion from the mode, transformed
+ * rejection) on a warp of its own, so that a warp's lanes do not wait for
+ * one another's branches, beside the strain thresholds on the fourth.  A
+ * batch of 12 (thousands of nodes): 40.4 us a tick with a node's work on one
+ * thread, 24.3 now; 4000 nodes 51 and 33 us; 14 nodes 17.7 us with a CTA of
+ * two warps a node, 16.9 now; 774 nodes 28.5 us in both. */
+#define LPG_NODE_TX_WARPS 5 /* LPG_MAX_STRAINS + 1 */
+__global__ void __launch_bounds__(32 * LPG_NODE_TX_WARPS) k_node_tx(DevWorld W, int per) {
   pdl_begin();
-  const int g = blockIdx.x;
+  __shared__ double s_p[LPG_MAX_STRAINS][32], s_gam[32];
+  __shared__ uint64_t s_gamk[32], s_thr[LPG_MAX_STRAINS][32];
+  __shared__ int64_t s_total[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __shared__ double s_gam;   /* the negative binomial's gamma variate, formed ahead by the second warp */
-  __shared__ uint64_t s_gamk; /* the exposure stream's position after it */
-  if (g >= W.G) return;
-  DevRep* rp = &W.reps[W.node_rep[g]];
-  if (threadIdx.x == 0) W.ksel[g] = 0;
-  if (!rp->active) return;
-  const int i = g - rp->node_base, n = rp->n_nodes, ns = rp->ns, t = rp->cur_t, G = W.G;
+  const int G = W.G;
+  const int g = lane < per && blockIdx.x * per + lane < G ? blockIdx.x * per + lane : G;
+  DevRep* rp = &W.reps[g < G ? W.node_rep[g] : 0];
+  const bool act = g < G && rp->active;
+  const bool tx = act && (rp->comps & LPG_COMP_TX);
+  const int i = act ? g - rp->node_base : 0, n = rp->n_nodes, ns = rp->ns, t = rp->cur_t;
+  if (g < G && wid == 0) W.ksel[g] = 0;
   int32_t pop_t = 0;
-  if (rp->comps & LPG_COMP_VD) {
-    const int32_t* pop1 = RES(rp, RS_POP, t - 1);
-    pop_t = pop1[i];
-    if (rp->vd_tick) pop_t = pop_t + W.ev[(int64_t)EV_BIRTHS * G + g] - W.ev[(int64_t)EV_DEATHS * G + g];
-    if (threadIdx.x == 0) RES(rp, RS_POP, t)[i] = pop_t;
-  } else {
-    pop_t = RES(rp, RS_POP, t)[i];
-  }
-  if (threadIdx.x == 0) {
-    W.size[g] = 0;
-    W.uniq[g] = 0;
-  }
-  if (!(rp->comps & LPG_COMP_TX)) return;
-  /* inputs of lane 0's draw, requested now so that they arrive during the
-   * mixing */
-  double pre_seas = 0.0, pre_r0s = 0.0, pre_rowsum = 0.0, pre_inck = 0.0;
-  uint64_t pre_bb = 0;
-  uint64_t pre_sw = 0;
-  int64_t pre_sc = 0;
-  /* lane k < ns of the first warp works on strain k after the mixing */
-  if (threadIdx.x < ns) {
-    pre_seas = rp->seas[t];
-    pre_r0s = rp->r0s[i];
-    pre_rowsum = rp->rowsum[i];
-    pre_bb = W.bb[(int64_t)threadIdx.x * G + g];
-    pre_inck = W.inck[(int64_t)threadIdx.x * G + g];
-  }
-  if (threadIdx.x == 0) {
-    pre_sw = W.sw[g];
-    pre_sc = W.tot[(int64_t)TT_S * G + g];
-  }
-  if (rp->rec) { /* the aggregates the expected-incidence map replays */
-    double* rr = rp->rec + ((int64_t)t * n + i) * (3 + ns);
-    if (threadIdx.x == 0) {
-      rr[0] = (double)pre_sw * 0x1.0p-24;
-      rr[1] = (double)pop_t;
-    }
-    if (threadIdx.x < ns) rr[3 + threadIdx.x] = (double)pre_bb * 0x1.0p-40;
-  }
-  if (wid == 1) {
-    /* the second warp: when the node has no local infectivity (the
-     * zero-inflated negative binomial, model.py:1383-1395), its gamma
-     * variate first: it uses the exposure stream from its second draw and
-     * not the tick's force of infection, so it is formed while the first
-     * warp works out the probabilities (a warp's double-precision operations
-     * do not overlap, another warp's do) */
-    const bool lz = __ballot_sync(FULLMASK, lane < ns && pre_bb_w1(W, g, lane, ns) != 0) == 0;
-    if (lane == 0 && lz && rp->zi < 1.0 && rp->nb_r >= 1) {
-      lpg_stream sg;
-      lpg_stream_init(&sg, rp->seed, LPG_P_TXCOUNT, t, (uint64_t)i, 0);
-      sg.k = 1; /* draw 0 is the zero-inflation test */
-      s_gam = lpg_gamma_mt(&sg, rp->nb_d, rp->nb_c, 1.0);
-      s_gamk = sg.k;
-    }
-    __syncwarp();
-    asm volatile("bar.sync 1, 64;" ::: "memory");
-    return;
-  }
-  if (wid != 0) return;
-  /* the first two blocks of lane 0's exposure-count stream, formed while
-   * the double-precision work below waits on its latencies */
+  uint64_t sw = 0, bb[LPG_MAX_STRAINS] = {0, 0, 0, 0};
+  bool local_zero = true;
+  double* rr = nullptr; /* the aggregates the expected-incidence map replays */
   lpg_stream sm;
-  lpg_stream_init(&sm, rp->seed, LPG_P_TXCOUNT, t, (uint64_t)i, 0);
-  lpg_stream_ahead(&sm);
-  /* Strain k on lane k (a double-precision warp instruction costs the same
-   * for one lane or 32): incoming infectivity, beta, rate, probability
-   * (model.py:1327-1363); then the sums over strains in strain order, as
-   * the oracle forms them. */
-  double pk = 0.0;
-  const double denom = (double)(pop_t > 1 ? pop_t : 1);
-  if (lane < ns) {
-    const double inck = pre_inck;
-    const double bpre = (double)pre_bb * 0x1.0p-40;
-    double beta = bpre + (inck - bpre * pre_rowsum);
-    beta = (beta * pre_seas) * pre_r0s;
-    const double rate = beta / denom;
-    pk = -lpg_expm1(-rate);
-    if (!(pk > 0.0)) pk = 0.0;
-    W.prob[(int64_t)lane * G + g] = pk;
+  if (act) {
+    if (rp->comps & LPG_COMP_VD) {
+      pop_t = RES(rp, RS_POP, t - 1)[i];
+      if (rp->vd_tick) pop_t = pop_t + W.ev[(int64_t)EV_BIRTHS * G + g] - W.ev[(int64_t)EV_DEATHS * G + g];
+      if (wid == 0) RES(rp, RS_POP, t)[i] = pop_t;
+    } else {
+      pop_t = RES(rp, RS_POP, t)[i];
+    }
+    if (wid == 0) {
+      W.size[g] = 0;
+      W.uniq[g] = 0;
+    }
   }
-  const int local_zero = __ballot_sync(FULLMASK, lane < ns && pre_bb != 0) == 0;
-  double p[LPG_MAX_STRAINS];
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) p[k] = __shfl_sync(FULLMASK, pk, k);
-  double total_p = 0.0;
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k)
-    if (k < ns) total_p = total_p + p[k];
-  /* strain thresholds of the selection, the divisions on their own lanes */
-  const double qk = pk / total_p;
-  uint64_t thr[LPG_MAX_STRAINS];
-  {
-    double c = 0.0;
+  if (tx) {
+    sw = W.sw[g];
 #pragma unroll
     for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-      const double q = __shfl_sync(FULLMASK, qk, k);
-      if (k < ns) c = c + q;
-      thr[k] = strain_threshold(c);
+      if (k < ns) bb[k] = W.bb[(int64_t)k * G + g];
+      if (bb[k] != 0) local_zero = false;
     }
-  }
-  __syncwarp();
-  asm volatile("bar.sync 1, 64;" ::: "memory"); /* the second warp's gamma variate is in s_gam */
-  if (lane != 0) return;
-  const double srisk = (double)pre_sw * 0x1.0p-24;
-  const double exposure = srisk * total_p;
-  if (rp->rec) rp->rec[((int64_t)t * n + i) * (3 + ns) + 2] = exposure;
-  int64_t total = 0;
-  if (!(exposure > 0.0)) {
-    total = 0;
-  } else if (local_zero) {
-    if (rp->zi >= 1.0) {
-      total = 0;
-    } else {
-      double mean = exposure / (1.0 - rp->zi);
-      double r = (double)rp->nb_r;
-      double pp = r / (r + mean);
-      double u = lpg_next(&sm);
-      if (u < rp->zi) {
-        total = 0;
-      } else if (rp->nb_r >= 1) {
-        /* lpg_negbinom_dc with its gamma variate from the second warp */
-        sm.k = s_gamk;
-        total = lpg_poisson(&sm, s_gam * ((1.0 - pp) / pp));
-      } else {
-        total = lpg_negbinom(&sm, r, pp);
+    if (rp->rec) rr = rp->rec + ((int64_t)t * n + i) * (3 + ns);
+    /* the first two blocks of the exposure-count stream, formed while the
+     * double-precision work waits on its latencies */
+    lpg_stream_init(&sm, rp->seed, LPG_P_TXCOUNT, t, (uint64_t)i, 0);
+    if (wid != 3) lpg_stream_ahead(&sm);
+    if (wid < LPG_MAX_STRAINS) {
+      /* strain wid: incoming infectivity, beta, rate, probability (model.py:1327-1363) */
+      double pk = 0.0;
+      if (wid < ns) {
+        uint64_t b = bb[0];
+#pragma unroll
+        for (int k = 1; k < LPG_MAX_STRAINS; ++k)
+          if (wid == k) b = bb[k];
+        const double bpre = (double)b * 0x1.0p-40;
+        const double denom = (double)(pop_t > 1 ? pop_t : 1);
+        if (rr) rr[3 + wid] = bpre;
+        double beta = bpre + (W.inck[(int64_t)wid * G + g] - bpre * rp->rowsum[i]);
+        beta = (beta * rp->seas[t]) * rp->r0s[i];
+        const double rate = beta / denom;
+        pk = -lpg_expm1(-rate);
+        if (!(pk > 0.0)) pk = 0.0;
+        W.prob[(int64_t)wid * G + g] = pk;
       }
+      s_p[wid][lane] = pk;
+    } else if (local_zero && rp->zi < 1.0 && rp->nb_r >= 1) {
+      /* no local infectivity (the zero-inflated negative binomial,
+       * model.py:1383-1395): the gamma variate uses the exposure stream from
+       * its second draw and not the tick's force of infection */
+      sm.k = 1; /* draw 0 is the zero-inflation test */
+      s_gam[lane] = lpg_gamma_mt(&sm, rp->nb_d, rp->nb_c, 1.0);
+      s_gamk[lane] = sm.k;
+      sm.k = 0;
     }
-  } else {
-    total = lpg_poisson(&sm, exposure);
   }
-  const int64_t sc = pre_sc;
+  __syncthreads();
+  if (tx) {
+    double p[LPG_MAX_STRAINS], total_p = 0.0; /* summed in strain order, as the oracle does */
+#pragma unroll
+    for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
+      p[k] = s_p[k][lane];
+      if (k < ns) total_p = total_p + p[k];
+    }
+    if (wid == 3) {
+      /* strain thresholds of the selection (model.py:1127-1135) */
+      double q[LPG_MAX_STRAINS], c = 0.0;
+#pragma unroll
+      for (int k = 0; k < LPG_MAX_STRAINS; ++k) q[k] = p[k] / total_p; /* independent divisions */
+#pragma unroll
+      for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
+        if (k < ns) c = c + q[k];
+        s_thr[k][lane] = strain_threshold(c);
+      }
+    } else {
+      const double exposure = ((double)sw * 0x1.0p-24) * total_p;
+      if (rr && wid == 0) {
+        rr[0] = (double)sw * 0x1.0p-24;
+        rr[1] = (double)pop_t;
+        rr[2] = exposure;
+      }
+      /* the warp that draws the count: 0-2 by the Poisson mean (as
+       * lpg_poisson chooses), 4 the negative binomial of r < 1 */
+      double lam = 0.0, pp = 0.0;
+      bool whole = false;
+      if (exposure > 0.0) {
+        if (!local_zero) {
+          lam = exposure;
+        } else if (rp->zi < 1.0) {
+          const double mean = exposure / (1.0 - rp->zi);
+          const double r = (double)rp->nb_r;
+          pp = r / (r + mean);
+          const double u = lpg_next(&sm);
+          if (u >= rp->zi) {
+            if (rp->nb_r >= 1) { /* lpg_negbinom_dc with its gamma variate from the fifth warp */
+              sm.k = s_gamk[lane];
+              lam = s_gam[lane] * ((1.0 - pp) / pp);
+            } else {
+              whole = true;
+            }
+          }
+        }
+      }
+      const int by = whole ? 4 : lam < 10.0 ? 0 : lam < 200.0 ? 1 : 2;
+      if (by == wid) s_total[lane] = whole ? lpg_negbinom(&sm, (double)rp->nb_r, pp) : lpg_poisson(&sm, lam);
+    }
+  }
+  __syncthreads();
+  if (wid != 0 || !tx) return;
+  const int64_t sc = W.tot[(int64_t)TT_S * G + g];
+  const int64_t total = s_total[lane];
   const int64_t size = total < sc ? total : sc;
   W.size[g] = size;
   /* the selection record of the node (round 0 targets: all of size) */
-  const uint64_t Tw = pre_sw;
-  if (size > 0 && Tw > 0) {
-    const int32_t* st = W.node_chunk_start[rp->csr_cur] + rp->csr_base;
-    SelInfo N;
-    N.seed = rp->seed;
-    N.T = Tw;
-#pragma unroll
-    for (int k = 0; k < LPG_MAX_STRAINS; ++k) N.thr[k] = thr[k];
-    N.a = rp->chunk_base + st[i];
-    N.n = st[i + 1] - st[i];
-    N.i = i;
-    N.t = t;
-    N.ns = ns;
-    N.csr = rp->csr_cur;
-    reinterpret_cast<SelInfo*>(W.sel_info)[g] = N;
-    W.ksel[g] = size;
-  }
-  if (size > 0) rp->any_demand = 1;
-}
-
-/* k_node_tx for a batch of thousands of small nodes: one node a thread,
- * the same operations in the same order (strains one after another; the
- * negative binomial's gamma variate drawn in line, from the same stream
- * positions).  A double-precision warp instruction costs the same for one
- * lane or 32, so here one serves 32 nodes: a batch's nodes take one wave
- * where a CTA a node takes ten. */
-__global__ void __launch_bounds__(128) k_node_tx_lanes(DevWorld W) {
-  pdl_begin();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= W.G) return;
-  DevRep* rp = &W.reps[W.node_rep[g]];
-  W.ksel[g] = 0;
-  if (!rp->active) return;
-  const int i = g - rp->node_base, n = rp->n_nodes, ns = rp->ns, t = rp->cur_t, G = W.G;
-  int32_t pop_t = 0;
-  if (rp->comps & LPG_COMP_VD) {
-    pop_t = RES(rp, RS_POP, t - 1)[i];
-    if (rp->vd_tick) pop_t = pop_t + W.ev[(int64_t)EV_BIRTHS * G + g] - W.ev[(int64_t)EV_DEATHS * G + g];
-    RES(rp, RS_POP, t)[i] = pop_t;
-  } else {
-    pop_t = RES(rp, RS_POP, t)[i];
-  }
-  W.size[g] = 0;
-  W.uniq[g] = 0;
-  if (!(rp->comps & LPG_COMP_TX)) return;
-  const double seas = rp->seas[t], r0s = rp->r0s[i], rowsum = rp->rowsum[i];
-  const uint64_t sw = W.sw[g];
-  const int64_t sc = W.tot[(int64_t)TT_S * G + g];
-  uint64_t bb[LPG_MAX_STRAINS];
-  double inc[LPG_MAX_STRAINS];
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-    bb[k] = k < ns ? W.bb[(int64_t)k * G + g] : 0;
-    inc[k] = k < ns ? W.inck[(int64_t)k * G + g] : 0.0;
-  }
-  double* rr = rp->rec ? rp->rec + ((int64_t)t * n + i) * (3 + ns) : nullptr;
-  if (rr) {
-    rr[0] = (double)sw * 0x1.0p-24;
-    rr[1] = (double)pop_t;
-  }
-  /* incoming infectivity, beta, rate and probability of each strain
-   * (model.py:1327-1363), and their sum in strain order */
-  const double denom = (double)(pop_t > 1 ? pop_t : 1);
-  double p[LPG_MAX_STRAINS];
-  double total_p = 0.0;
-  bool local_zero = true;
-#pragma unroll
-  for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-    p[k] = 0.0;
-    if (k < ns) {
-      const double bpre = (double)bb[k] * 0x1.0p-40;
-      if (rr) rr[3 + k] = bpre;
-      if (bb[k] != 0) local_zero = false;
-      double beta = bpre + (inc[k] - bpre * rowsum);
-      beta = (beta * seas) * r0s;
-      const double rate = beta / denom;
-      double pk = -lpg_expm1(-rate);
-      if (!(pk > 0.0)) pk = 0.0;
-      p[k] = pk;
-      W.prob[(int64_t)k * G + g] = pk;
-      total_p = total_p + pk;
-    }
-  }
-  /* strain thresholds of the selection */
-  uint64_t thr[LPG_MAX_STRAINS];
-  {
-    double c = 0.0;
-#pragma unroll
-    for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
-      if (k < ns) c = c + p[k] / total_p;
-      thr[k] = strain_threshold(c);
-    }
-  }
-  lpg_stream sm;
-  lpg_stream_init(&sm, rp->seed, LPG_P_TXCOUNT, t, (uint64_t)i, 0);
-  const double srisk = (double)sw * 0x1.0p-24;
-  const double exposure = srisk * total_p;
-  if (rr) rr[2] = exposure;
-  int64_t total = 0;
-  if (!(exposure > 0.0)) {
-    total = 0;
-  } else if (local_zero) {
-    if (rp->zi >= 1.0) {
-      total = 0;
-    } else {
-      double mean = exposure / (1.0 - rp->zi);
-      double r = (double)rp->nb_r;
-      double pp = r / (r + mean);
-      double u = lpg_next(&sm);
-      if (u < rp->zi) {
-        total = 0;
-      } else if (rp->nb_r >= 1) {
-        const double gam = lpg_gamma_mt(&sm, rp->nb_d, rp->nb_c, 1.0); /* lpg_negbinom_dc */
-        total = lpg_poisson(&sm, gam * ((1.0 - pp) / pp));
-      } else {
-        total = lpg_negbinom(&sm, r, pp);
-      }
-    }
-  } else {
-    total = lpg_poisson(&sm, exposure);
-  }
-  const int64_t size = total < sc ? total : sc;
-  W.size[g] = size;
   if (size > 0 && sw > 0) {
     const int32_t* st = W.node_chunk_start[rp->csr_cur] + rp->csr_base;
     SelInfo N;
     N.seed = rp->seed;
     N.T = sw;
 #pragma unroll
-    for (int k = 0; k < LPG_MAX_STRAINS; ++k) N.thr[k] = thr[k];
+    for (int k = 0; k < LPG_MAX_STRAINS; ++k) N.thr[k] = s_thr[k][lane];
     N.a = rp->chunk_base + st[i];
     N.n = st[i + 1] - st[i];
     N.i = i;
