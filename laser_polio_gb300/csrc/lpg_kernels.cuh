@@ -1207,13 +1207,17 @@ __global__ void __launch_bounds__(LPG_SWEEP_BLOCK) k_sweep_rs(DevWorld W) {
 /* Queue kernels: one thread per queued agent.  The queue is one slab per CTA
  * of the sweep; entries of a warp mostly belong to one node, so node counters
  * are summed across the lanes that share a node before the global atomics. */
+/* A lane that has its group to itself takes no reduction: groups are reduced
+ * one after another, and on a quiet tick a warp's agents are of 32 nodes. */
 __device__ __forceinline__ void warp_add(int32_t* p, unsigned peers, int32_t v) {
-  const int32_t tot = __reduce_add_sync(peers, v);
+  int32_t tot = v;
+  if (peers & (peers - 1)) tot = __reduce_add_sync(peers, v);
   if ((threadIdx.x & 31) == __ffs(peers) - 1 && tot) atomicAdd(p, tot);
 }
 /* Sum of 64-bit values over the lanes of peers, exact modulo 2^64 (four
  * 16-bit parts, each summed in 32 bits without overflow). */
 __device__ __forceinline__ uint64_t warp_sum_u64(unsigned peers, uint64_t w) {
+  if (!(peers & (peers - 1))) return w;
   uint64_t tot = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k)
@@ -2190,14 +2194,15 @@ __device__ __forceinline__ void node_exposed(DevWorld& W, int g, int n, uint64_t
 }
 /* The node totals of the warp's claims, one set of atomics per node of the
  * warp (a warp's targets are neighbours, so mostly one node).  All lanes. */
-__device__ __forceinline__ void warp_node_exposed(DevWorld& W, int g, int ns, bool won, int s, uint64_t w) {
+__device__ __forceinline__ void warp_node_exposed(DevWorld& W, int g, bool won, int s, uint64_t w) {
   const unsigned all = __ballot_sync(FULLMASK, won);
   if (!won) return;
   const unsigned by = __match_any_sync(all, g);
   const bool lead = (int)(threadIdx.x & 31) == __ffs(by) - 1;
   const uint64_t wt = warp_sum_u64(by, w);
   if (lead) node_exposed(W, g, __popc(by), wt);
-  for (int k = 0; k < ns; ++k) {
+#pragma unroll
+  for (int k = 0; k < LPG_MAX_STRAINS; ++k) {
     const int n = __popc(__ballot_sync(by, s == k));
     if (lead && n) node_strain(W, g, k, n);
   }
@@ -2325,7 +2330,36 @@ __device__ __forceinline__ void locate_batch(const DevWorld& W, const int32_t* l
   out->hit = LPG_NONE;
   if (nk == 0) return;
   int32_t cid = 0;
-  if (act) {
+  if (nk == 1) {
+    /* one target a team: its eight lanes search together, nine ways a step
+     * (the prefix is not in L1 yet: a step costs an L2 round trip) */
+    const bool on = __shfl_sync(FULLMASK, (int)act, 0, 8) != 0;
+    const uint64_t vt = __shfl_sync(FULLMASK, v, 0, 8);
+    const uint64_t* cpt = reinterpret_cast<const uint64_t*>(__shfl_sync(FULLMASK, (unsigned long long)cp, 0, 8));
+    int32_t lo = 0, hi = __shfl_sync(FULLMASK, n, 0, 8) - 1;
+    uint64_t below = 0; /* cp[lo - 1] */
+    while (__any_sync(FULLMASK, on && lo < hi)) {
+      const bool go = on && lo < hi;
+      /* probe l of [lo, hi): ascending with the lane */
+      const int32_t p = lo + (int32_t)(((uint32_t)(l + 1) * (uint32_t)(hi - lo)) / 9u);
+      const uint64_t c = go ? (FRESH ? __ldcg(cpt + p) : cpt[p]) : 0;
+      const unsigned up = (__ballot_sync(FULLMASK, go && c > vt) >> lane0) & 0xffu;
+      const int f = up ? __ffs(up) - 1 : 8; /* the first probe above the target */
+      const uint64_t cb = __shfl_sync(FULLMASK, c, f > 0 ? f - 1 : 0, 8);
+      const int32_t pb = __shfl_sync(FULLMASK, p, f > 0 ? f - 1 : 0, 8), pf = __shfl_sync(FULLMASK, p, f & 7, 8);
+      if (go) {
+        if (f > 0) {
+          lo = pb + 1;
+          below = cb;
+        }
+        if (f < 8) hi = pf;
+      }
+    }
+    if (act) { /* lane 0 */
+      v -= below;
+      cid = ls[lo];
+    }
+  } else if (act) {
     int32_t lo = 0, hi = n - 1;
     uint64_t below = 0; /* cp[lo - 1] */
     while (lo < hi) {
@@ -2349,11 +2383,13 @@ __device__ __forceinline__ void locate_batch(const DevWorld& W, const int32_t* l
     ulonglong2 x[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
+      if (k0 + k >= nk) break; /* the same for the warp */
       const int64_t c = __shfl_sync(FULLMASK, cid, k0 + k, 8);
       x[k] = __ldcg(reinterpret_cast<const ulonglong2*>(W.sub_w + c * LPG_NSUB) + l);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
+      if (k0 + k >= nk) break;
       const uint64_t vk = __shfl_sync(FULLMASK, v, k0 + k, 8);
       const uint64_t sum = x[k].x + x[k].y;
       uint64_t incl = sum;
@@ -2471,8 +2507,8 @@ __device__ __forceinline__ void locate_batch(const DevWorld& W, const int32_t* l
   }
 }
 
-/* The targets of a round made by the whole grid (round 0; FRESH: a later
- * one, whose prefixes this kernel has rewritten).  A CTA has an equal run of
+/* The targets of a round made by the whole grid (FRESH: a later one than
+ * round 0, which reads prefixes that this kernel has rewritten, past L1).  A CTA has an equal run of
  * consecutive targets, 256 of them at a time (target l * 32 + team of the
  * 256 on lane l of a team of 8; 32 or fewer: one a team), so that its
  * targets share nodes: their prefixes stay in L1 and the claims' node totals
@@ -2486,23 +2522,23 @@ template <bool FRESH>
 __device__ __forceinline__ bool grid_targets(DevWorld& W, const int64_t* offs, const SelInfo* info, int64_t K,
                                              int round) {
   const int G = W.G;
-  const int64_t qa = K * blockIdx.x / gridDim.x, qe = K * (blockIdx.x + 1) / gridDim.x;
-  const int64_t q0 = qa + (threadIdx.x & 7) * 32 + threadIdx.x / 8;
+  const int64_t qa = K * blockIdx.x / gridDim.x;
+  const uint32_t m = (uint32_t)(K * (blockIdx.x + 1) / gridDim.x - qa); /* this CTA's targets */
+  const uint32_t j0 = (threadIdx.x & 7) * 32 + threadIdx.x / 8;
   uint32_t h0 = LPG_NONE;
   uint64_t w0 = 0;
-  int b = 0;
-  for (int64_t q = q0, qw = qa; qw < qe; q += 256, qw += 256, ++b) {
-    const bool act = q < qe;
+  for (uint32_t jw = 0; jw < m; jw += 256) {
+    const int64_t q = qa + jw + j0;
+    const bool act = jw + j0 < m;
     int g = 0;
     uint64_t v = 0;
-    int32_t la = 0, ln = 1, lcsr = 0, ns = 0;
+    int32_t la = 0, ln = 1, lcsr = 0;
     if (act) {
       g = node_of_target(offs, G, q);
       const SelInfo& N = info[g];
       la = N.a;
       ln = N.n;
       lcsr = N.csr;
-      ns = N.ns;
       const uint64_t total = FRESH ? __ldcg(W.cpref + la + ln - 1) : N.T;
       v = lpg_scale_target(lpg_u53(N.seed, LPG_P_SELECT, N.t, (uint64_t)N.i, (uint64_t)round, (uint64_t)(q - offs[g])),
                            total);
@@ -2514,22 +2550,22 @@ __device__ __forceinline__ bool grid_targets(DevWorld& W, const int64_t* offs, c
       if (L.hit == LPG_NONE) W.reps[W.node_rep[g]].error = LPG_ERR_INTERNAL;
       else s = claim(W, L, info[g], LPG_DS_CLAIMED);
       const uint32_t won_at = s >= 0 ? L.hit : LPG_NONE;
-      if (b == 0) {
+      if (jw == 0) {
         h0 = won_at;
         w0 = L.w;
       } else {
-        W.hits[q] = won_at;
+        W.hits[qa + jw + j0] = won_at;
       }
     }
     __syncwarp();
-    warp_node_exposed(W, g, ns, s >= 0, s, L.w);
+    warp_node_exposed(W, g, s >= 0, s, L.w);
   }
   /* every target of the round located and claimed: the claimed agents
    * become exposed and leave their sub-blocks' weights */
   if (!grid_sync(W.grid_bar, W.wait_spin, W.test_bar_skip && blockIdx.x == 0)) return false;
   claim0_finish(W, h0, w0);
-  for (int64_t q = q0 + 256; q < qe; q += 256) { /* this lane's later claims */
-    const uint32_t h = W.hits[q];
+  for (uint32_t j = j0 + 256; j < m; j += 256) { /* this lane's later claims */
+    const uint32_t h = W.hits[qa + j];
     if (h != LPG_NONE) claim0_finish(W, h, fix_risk(W.risk[h]));
   }
   return true;
@@ -2558,7 +2594,9 @@ __device__ __forceinline__ bool grid_targets(DevWorld& W, const int64_t* offs, c
  * 44 ms and k_sel_rounds 27 ms with targets dealt round-robin, searched one
  * at a time by the whole team and added to the node totals one by one;
  * 26 ms and 11 ms now (0.79 and 0.4 ns a target on the busiest ticks).
- * Three CTAs an SM: with two, 27 ms.
+ * Three CTAs an SM: with two, 27 ms.  Quiet ticks (a thousand targets, one a
+ * team, the prefix search by its eight lanes): both kernels 30 us a tick at
+ * 774 nodes, as with teams of 32.
  *
  * A round after the first is made by the whole grid while some node still
  * lacks more agents than LPG_SEL_GRID_NODE: a round of one node costs its
