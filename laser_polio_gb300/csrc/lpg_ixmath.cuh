@@ -154,6 +154,30 @@ __device__ __forceinline__ double ix_log1p(const IxTables* T, double y) {
   return ix_double(sum << lz, 6 - lz);
 }
 
+/* ln m of m 2^-63 in [1, 2), with 63 fraction bits: r = m c_j - 1 as above. */
+__device__ __forceinline__ int64_t ix_log_mant(const IxTables* T, uint64_t m) {
+  const int j = (int)(m >> 56) & 127;
+  const uint64_t c = T->log_c[j];
+  const uint64_t hi = __umul64hi(m, c), lo = m * c;
+  const int64_t r = (int64_t)((hi - (1ULL << 62)) << 2 | lo >> 62); /* 64 fraction bits, |r| < 2^-7 */
+  const int64_t r2 = __mul64hi(r, r);
+  const int64_t r3 = __mul64hi(r2, r), r4 = __mul64hi(r2, r2);
+  const int64_t r5 = __mul64hi(r4, r);
+  int64_t s = r - (r2 >> 1) + __mul64hi(r3, 0x5555555555555555LL) - (r4 >> 2) + __mul64hi(r5, 0x3333333333333333LL);
+  s -= __mul64hi(__mul64hi(r3, r3), 0x2aaaaaaaaaaaaaaaLL);
+  s += __mul64hi(__mul64hi(r4, r3), 0x2492492492492492LL);
+  return (int64_t)T->log_v[j] + (s >> 1);
+}
+
+/* log2 x with 52 fraction bits of a positive normal x, rounded (within 2^-53). */
+__device__ __forceinline__ int64_t ix_log2(const IxTables* T, double x) {
+  const uint64_t b = (uint64_t)__double_as_longlong(x);
+  const int e = (int)(b >> 52) - 1023;
+  const int64_t v = ix_log_mant(T, ((b & 0xfffffffffffffULL) | 1ULL << 52) << 11);
+  const int64_t f = __mul64hi(v, 0x5c551d94ae0bf85eLL); /* times 1/(2 ln 2): log2 m with 61 fraction bits */
+  return ((int64_t)e << 52) + ((f + (1LL << 8)) >> 9);
+}
+
 /* The tables, formed once (0.1 ms where long double is done in software). */
 inline const IxTables* ix_tables() {
   static const IxTables tables = [] {
