@@ -70,3 +70,27 @@ def test_gpu_flows_equal_the_oracle_at_every_exponent(k, a, b, c):
     want = I.incidence(inp)[0]
     got = ops.expected_incidence(inp)[0]
     _close(got, want, "lam")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G", [30, 200])
+def test_gpu_distances_at_the_edges_of_the_logarithm(G):
+    """log2 of the distances in integers (normal ones) and in FP64: subnormal,
+    next to one, powers of two and their neighbours, infinite; the diagonal,
+    which is never read, may hold anything, and no other entry may be
+    negative or NaN."""
+    inp = I.random_inputs(12, G, 1, seed=4)
+    edges = [1e-310, 2.0**-1022, 0.5, 1 - 2.0**-53, 1.0, 1 + 2.0**-52, 2 - 2.0**-52, 2.0, 1e300, np.inf]
+    for j, d in enumerate(edges):
+        inp["dist"][0, j + 1] = inp["dist"][j + 1, 0] = d
+    inp.update(k=0.5, a=0.7, b=1.1, c=0.3, max_frac=1e-3)
+    _close(ops.expected_incidence(inp)[0], I.incidence(inp)[0], "lam")
+    lam = ops.expected_incidence(inp)[0]
+    odd = dict(inp, dist=inp["dist"].copy())
+    np.fill_diagonal(odd["dist"], [np.nan, -1.0] * (G // 2))
+    assert np.array_equal(ops.expected_incidence(odd)[0], lam)
+    for bad in (-1.0, np.nan):
+        odd = dict(inp, dist=inp["dist"].copy())
+        odd["dist"][3, G - 1] = bad
+        with pytest.raises(Exception):
+            ops.expected_incidence(odd)
