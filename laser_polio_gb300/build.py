@@ -20,7 +20,7 @@ OUT = PKG / "_build" / "liblpg.so"
 SOURCES = [CSRC / "lpg_engine.cu", CSRC / "lpg_ops.cu", CSRC / "lpg_adjoint.cu", CSRC / "lpg_init.cu",
            CSRC / "lpg_export.cpp", CSRC / "lpg_network.cpp"]
 DEPS = SOURCES + [CSRC / "lpg_kernels.cuh", CSRC / "lpg_engine.cuh", CSRC / "lpg_rng.h", CSRC / "lpg_detmath.h",
-                  CSRC / "lpg_ri.h", CSRC / "lpg_init.h", CSRC / "lpg_init_fast.cuh",
+                  CSRC / "lpg_ri.h", CSRC / "lpg_devmem.h", CSRC / "lpg_init.h", CSRC / "lpg_init_fast.cuh",
                   CSRC / "lpg_ixmath.cuh", CSRC / "lpg_ozaki.cuh",
                   ROOT / "include" / "lpg.h"]
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"

@@ -20,6 +20,7 @@
 #include "lpg.h"
 #include <utility>
 
+#include "lpg_devmem.h"
 #include "lpg_kernels.cuh"
 
 namespace {
@@ -43,6 +44,9 @@ const char* kKernelNames[] = {"k_begin", "k_newborns", "k_due", "k_sweep_a", "k_
                               "k_evb", "k_node_mix", "k_node_tx", "k_sel_round0", "k_sel_rounds"};
 constexpr int kNumTickKernels = 11; /* k_sel_rounds ends the tick (results rows, next tick's setup) */
 constexpr int kTicksPerGraph = 8;
+
+int dev_alloc(void** p, size_t bytes) { return (int)cudaMalloc(p, bytes); }
+void dev_release(void* p) { cudaFree(p); }
 
 /* Reference-ordered columns of one simulation on the device. */
 struct Staging {
@@ -80,16 +84,7 @@ struct lpg_handle {
   std::vector<SimHost> sims;
   std::vector<DevRep> hreps;
   DevWorld W{};
-  std::vector<void*> allocs;
-  /* small buffers are carved from slabs: one allocation, and for uploads one
-   * copy, for many */
-  struct Slab {
-    uint8_t* dev = nullptr;
-    std::vector<uint8_t> host; /* upload slabs: the bytes to copy */
-    size_t used = 0, sent = 0;
-  };
-  Slab plain;
-  std::vector<Slab> uploads;
+  DevMem mem{dev_alloc, dev_release};
   bool started = false;
   std::string err;
   bool use_graphs = true;
@@ -137,62 +132,40 @@ static int fail(lpg_handle* h, int code, const char* fmt, ...) {
                                        __FILE__, __LINE__);                                            \
   } while (0)
 
-constexpr size_t kSlabBytes = 1 << 20, kSlabItem = 1 << 17;
-static size_t pad256(size_t n) { return (n + 255) & ~(size_t)255; }
+static int no_memory(lpg_handle* h, size_t bytes, int e) {
+  return fail(h, LPG_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString((cudaError_t)e));
+}
 
 static int dalloc_bytes(lpg_handle* h, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) return fail(h, LPG_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-  h->allocs.push_back(*p);
-  return 0;
+  const int e = h->mem.own(p, bytes);
+  return e ? no_memory(h, bytes, e) : 0;
 }
 
 template <typename T>
 static int dalloc(lpg_handle* h, T** p, size_t n) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-  if (bytes > kSlabItem) return dalloc_bytes(h, (void**)p, bytes);
-  if (!h->plain.dev || h->plain.used + bytes > kSlabBytes) {
-    h->plain.used = 0;
-    const int rc = dalloc_bytes(h, (void**)&h->plain.dev, kSlabBytes);
-    if (rc) {
-      h->plain.dev = nullptr;
-      return rc;
-    }
-  }
-  *p = (T*)(h->plain.dev + h->plain.used);
-  h->plain.used += pad256(bytes);
-  return 0;
+  const int e = h->mem.part((void**)p, bytes);
+  return e ? no_memory(h, bytes, e) : 0;
 }
 
 /* A device copy of v; small ones arrive with the next flush_uploads. */
 template <typename T>
 static int dupload(lpg_handle* h, T** p, const std::vector<T>& v) {
   const size_t bytes = v.size() * sizeof(T);
-  if (bytes > kSlabItem) {
+  if (bytes > DevMem::kItemBytes) {
     int rc = dalloc(h, p, v.size());
     if (rc) return rc;
     CK(cudaMemcpyAsync(*p, v.data(), bytes, cudaMemcpyHostToDevice, h->stream));
     return 0;
   }
-  if (h->uploads.empty() || h->uploads.back().used + bytes > kSlabBytes) {
-    lpg_handle::Slab s;
-    const int rc = dalloc_bytes(h, (void**)&s.dev, kSlabBytes);
-    if (rc) return rc;
-    s.host.resize(kSlabBytes);
-    h->uploads.push_back(std::move(s));
-  }
-  lpg_handle::Slab& s = h->uploads.back();
-  *p = (T*)(s.dev + s.used);
-  if (bytes) memcpy(s.host.data() + s.used, v.data(), bytes);
-  s.used += pad256(std::max<size_t>(bytes, 1));
-  return 0;
+  const int e = h->mem.upload((void**)p, v.data(), bytes);
+  return e ? no_memory(h, bytes, e) : 0;
 }
 
 static int flush_uploads(lpg_handle* h) {
-  for (auto& s : h->uploads) {
+  for (auto& s : h->mem.uploads()) {
     if (s.used > s.sent)
-      CK(cudaMemcpyAsync(s.dev + s.sent, s.host.data() + s.sent, std::min(s.used, kSlabBytes) - s.sent,
-                         cudaMemcpyHostToDevice, h->stream));
+      CK(cudaMemcpyAsync(s.dev + s.sent, s.host.data() + s.sent, s.used - s.sent, cudaMemcpyHostToDevice, h->stream));
     s.sent = s.used;
   }
   return 0;
@@ -206,7 +179,7 @@ struct Carve {
   template <typename T>
   void add(T** p, size_t n) {
     items.emplace_back((void**)p, total);
-    total += pad256(std::max<size_t>(n, 1) * sizeof(T));
+    total += DevMem::pad(std::max<size_t>(n, 1) * sizeof(T));
   }
   int commit(lpg_handle* h) {
     uint8_t* base = nullptr;
@@ -218,13 +191,7 @@ struct Carve {
 };
 
 /* Frees an allocation of its own; a part of a slab stays until the end. */
-static void dfree_one(lpg_handle* h, void* p) {
-  if (!p) return;
-  auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
-  if (it == h->allocs.end()) return;
-  cudaFree(p);
-  h->allocs.erase(it);
-}
+static void dfree_one(lpg_handle* h, void* p) { h->mem.give_back(p); }
 
 /* The network in the two fixed-point parts of lpg_net_split, transposed:
  * q[2 (j n + i)], 32 x 32 tiles turned in shared memory. */
@@ -1728,7 +1695,7 @@ extern "C" void lpg_destroy(lpg_handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second.first);
   for (auto e : h->ev_pool) cudaEventDestroy(e);
-  for (void* p : h->allocs) cudaFree(p);
+  h->mem.clear();
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
