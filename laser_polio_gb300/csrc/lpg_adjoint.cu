@@ -34,7 +34,10 @@
  *   - The two contractions, u = beta N per (t, s) row and dL/dN = beta^T
  *     dL/du, both (T S) x G x G, run on the tensor cores by exact slicing
  *     (lpg_ozaki.cuh).  beta's slices are formed once per plan, N's and
- *     dL/du's each evaluation.
+ *     dL/du's each evaluation.  An element that is small beside its row's and
+ *     column's scales is formed again from the FP64 operands, so that each
+ *     element is good to 2^-45 of its own summed terms (four deviations; the
+ *     FP32 pairs used where many are small: rms).
  *   - Contractions too small for that are summed in FP64 where their results
  *     are used, with no launch of their own.
  *   - exp and log1p run in 64-bit integer arithmetic (lpg_ixmath.cuh).
@@ -43,6 +46,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -253,9 +257,9 @@ __device__ __forceinline__ double inc_recip(double d) {
 }
 
 struct IncStep {
-  int T, G, S, split; /* split: depth slices of the mixing product */
+  int T, G, S;
   const double *srisk, *beta, *rpop, *seas, *r0s, *rsN, *ltarget, *g_in;
-  const double* u; /* the mixing product's slabs, or */
+  const double* u; /* the mixing product, or */
   const double* N; /* the normalised network (small sums) */
   double R;
   double *lam, *loss; /* lam may be null */
@@ -279,7 +283,6 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
   __shared__ double s_loss[4];
   const int n = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * TC, lane = threadIdx.x & 31;
   const int T = A.T, G = A.G, S = A.S;
-  const size_t slab = (size_t)T * S * G;
   const bool in = n < G;
   const double keep = in ? 1.0 - A.rsN[n] : 0.0, r0 = in ? A.r0s[n] : 0.0;
   double loss = 0.0, acc_r0 = 0.0;
@@ -309,14 +312,7 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
       uu[s] = ex[s] = 0.0;
       if (s >= S) continue;
       const size_t k = ((size_t)t * S + s) * G + n;
-      double m;
-      if (SMALL) {
-        m = mix[s];
-      } else {
-        m = A.u[k];
-        for (int z = 1; z < A.split; ++z) m += A.u[z * slab + k];
-      }
-      uu[s] = __fma_rn(A.beta[k], keep, m);
+      uu[s] = __fma_rn(A.beta[k], keep, SMALL ? mix[s] : A.u[k]);
       ex[s] = inc_exp_neg(tab, uu[s] * q);
       l += 1.0 - ex[s];
     }
@@ -366,15 +362,15 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
 }
 
 /* The last block: dL/dR, dL/damp and dL/dpeak from w[t].  The others take
- * rows a in turn — C[a][b] = the sum of the flows product's nsplit depth
- * slices, or with SMALL the sum over (t, s) formed here, dL/dN[a][b] = C[a][b] - C[a][a] (zero on the diagonal), then dL/dG
+ * rows a in turn — C[a][b] of the flows product, or with SMALL the sum over
+ * (t, s) formed here, dL/dN[a][b] = C[a][b] - C[a][a] (zero on the diagonal), then dL/dG
  * through the row normalisation and the contributions to dL/dk, dL/da, dL/db,
  * dL/dc, kept per thread over the CTA's rows; dL/dN is written when asked
  * for.  Bound by FP64 issue: five operations an element and two a row and
  * thread (4000 nodes: 616 us with a reduction and two passes a row). */
 template <bool SMALL>
 __global__ void __launch_bounds__(INC_THREADS, SMALL ? 2 : 5)
-    k_inc_network_grad(int G, int T, int TS, int nsplit, const double* C, const double* beta, const double* gu, const double* Gm, const double* rs,
+    k_inc_network_grad(int G, int T, int TS, const double* C, const double* beta, const double* gu, const double* Gm, const double* rs,
                        const double* fac, const double* logp, const double* logd, double k, double logP,
                        double* gN, double* g_theta, const double* seas, const double* g_w, double R, double* g_seas) {
   __shared__ double s_part[INC_THREADS / 32];
@@ -397,7 +393,6 @@ __global__ void __launch_bounds__(INC_THREADS, SMALL ? 2 : 5)
     return;
   }
   extern __shared__ double s_flow[]; /* the small sums: partial rows [slices][G] */
-  const size_t GG = (size_t)G * G;
   auto nonzero = [](double x) { return ((uint64_t)__double_as_longlong(x) << 1) != 0; };
   double wk = 0.0, wa = 0.0, wb = 0.0, wc = 0.0;
   for (int a = blockIdx.x; a < G; a += rows) {
@@ -422,12 +417,7 @@ __global__ void __launch_bounds__(INC_THREADS, SMALL ? 2 : 5)
       }
       __syncthreads();
     }
-    auto flow = [&](int b) { /* the depth slices' sum */
-      if (SMALL) return s_flow[b];
-      double c = C[row + b];
-      for (int z = 1; z < nsplit; ++z) c += C[z * GG + row + b];
-      return c;
-    };
+    auto flow = [&](int b) { return SMALL ? s_flow[b] : C[row + b]; };
     const double diag = flow(a), f = fac[a];
     const bool cap = f != 1.0;
     double shift = 0.0; /* a capped row's coupling: sum of dL/dN G over the row, by its sum */
@@ -470,7 +460,7 @@ __global__ void __launch_bounds__(INC_THREADS, SMALL ? 2 : 5)
 
 }  // namespace
 
-enum { SC_LOSS = 0, SC_R = 1, SC_THETA = 4, SC_ERR = 8, SC_N = 16 };
+enum { SC_LOSS = 0, SC_R = 1, SC_THETA = 4, SC_ERR = 8, SC_LIST = 9, SC_N = 16 }; /* SC_LIST: two counts */
 
 struct lpg_incidence_plan {
   int T = 0, G = 0, S = 0;
@@ -488,14 +478,19 @@ struct lpg_incidence_plan {
   /* per evaluation */
   double *r0s = nullptr, *seas = nullptr, *Gm = nullptr, *rs = nullptr, *rsN = nullptr, *fac = nullptr,
          *u = nullptr, *lam = nullptr, *g = nullptr, *C = nullptr, *gN = nullptr;
-  /* cleared each evaluation, one block: sums [SC_N], gr0s [G], w [T], column maxima of N and dL/du [G] */
+  /* cleared each evaluation, one block: sums [SC_N], gr0s [G], w [T], column maxima of N and dL/du [G], their sums
+   * of squares [G] */
   double *sums = nullptr, *gr0s = nullptr, *gw = nullptr;
   unsigned long long *max_n = nullptr, *max_gu = nullptr;
+  uint32_t *sq_n = nullptr, *sq_gu = nullptr;
   size_t clear_bytes = 0;
   double *N = nullptr, *gu = nullptr;
-  /* the sliced products: digits, row and column maxima, tensor maps */
+  /* the sliced products: digits, row and column maxima and sums of squares, tensor maps */
   uint32_t *b_rows = nullptr, *b_cols = nullptr, *n_cols = nullptr, *gu_cols = nullptr;
   unsigned long long *max_br = nullptr, *max_bc = nullptr;
+  uint32_t *sq_br = nullptr, *sq_bc = nullptr;
+  unsigned long long* list_n = nullptr; /* two of the sums */
+  uint64_t* list = nullptr;
   CUtensorMap map_b{}, map_n{}, map_bt{}, map_gu{};
   double* host = nullptr; /* pinned: sums and gr0s [SC_N + G], then r0s [G] */
   /* profiling */
@@ -530,7 +525,8 @@ void plan_free(lpg_incidence_plan* p) {
   void* ps[] = {p->srisk, p->beta, p->rpop, p->doy,  p->year,    p->pops,   p->logp,   p->logd,    p->target,
                 p->lp2,   p->ld2,  p->tab,  p->r0s,  p->seas,    p->Gm,     p->rs,     p->rsN,     p->fac,
                 p->u,     p->lam,  p->g,    p->C,    p->gN,      p->sums,   p->N,
-                p->gu,    p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc};
+                p->gu,    p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc,
+                p->sq_br, p->sq_bc, p->list};
   for (void* q : ps)
     if (q) cudaFree(q);
   if (p->host) cudaFreeHost(p->host);
@@ -556,13 +552,16 @@ int plan_alloc(lpg_incidence_plan* p) {
       (rc = dalloc(&p->rsN, G)) || (rc = dalloc(&p->fac, G)) || (rc = dalloc(&p->lam, TG)) ||
       (rc = dalloc(&p->g, TG)) || (rc = dalloc(&p->gN, GG)))
     return rc;
-  const size_t clear = SC_N + G + T + 2 * G;
+  const size_t clear = SC_N + G + T + 3 * G; /* doubles; the sums of squares two to one */
   if ((rc = dalloc(&p->sums, clear))) return rc;
   p->clear_bytes = clear * sizeof(double);
+  p->list_n = reinterpret_cast<unsigned long long*>(p->sums + SC_LIST);
   p->gr0s = p->sums + SC_N;
   p->gw = p->gr0s + G;
   p->max_n = reinterpret_cast<unsigned long long*>(p->gw + T);
   p->max_gu = p->max_n + G;
+  p->sq_n = reinterpret_cast<uint32_t*>(p->max_gu + G);
+  p->sq_gu = p->sq_n + G;
   if ((rc = dalloc(&p->gu, TSG))) return rc;
   if (!p->small) {
     const size_t kg = depth_pad(p->G), kt = depth_pad((int)TS), half = OZ_SLICES / 2; /* two digits a word */
@@ -571,7 +570,9 @@ int plan_alloc(lpg_incidence_plan* p) {
     if ((rc = dalloc(&p->u, mix.split * TSG)) || (rc = dalloc(&p->C, flows.split * GG)) ||
         (rc = dalloc(&p->b_rows, half * TS * kg)) ||
         (rc = dalloc(&p->b_cols, half * G * kt)) || (rc = dalloc(&p->n_cols, half * G * kg)) ||
-        (rc = dalloc(&p->gu_cols, half * G * kt)) || (rc = dalloc(&p->max_br, TS)) || (rc = dalloc(&p->max_bc, G)))
+        (rc = dalloc(&p->gu_cols, half * G * kt)) || (rc = dalloc(&p->max_br, TS)) || (rc = dalloc(&p->max_bc, G)) ||
+        (rc = dalloc(&p->sq_br, TS)) || (rc = dalloc(&p->sq_bc, G)) ||
+        (rc = dalloc(&p->list, std::max(oz_list((int)TS, p->G), oz_list(p->G, p->G)))))
       return rc;
     if (!oz_map(&p->map_b, p->b_rows, (int)TS, (int)kg, OZ_BM) || !oz_map(&p->map_n, p->n_cols, p->G, (int)kg, OZ_BN) ||
         !oz_map(&p->map_bt, p->b_cols, p->G, (int)kt, OZ_BM) || !oz_map(&p->map_gu, p->gu_cols, p->G, (int)kt, OZ_BN))
@@ -652,16 +653,20 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
                                                           p->seas);
     k_oz_col_max<<<oz_col_grid(G, G), 256, 0, p->st>>>(G, G, p->Gm, p->fac, p->max_n);
     k_oz_slice_cols<<<dim3((G + 31) / 32, depth_pad(G) / 32), 256, 0, p->st>>>(G, G, depth_pad(G), p->Gm, p->fac,
-                                                                              p->max_n, p->n_cols);
+                                                                              p->max_n, p->n_cols, p->sq_n);
   }
-  mark(p, PH_MIX, 1); /* with small sums part of the step's launch, counted here too */
-  if (!p->small) PCK(oz_gemm(p->map_b, p->map_n, mix, p->nsm, p->st));
+  mark(p, PH_MIX, p->small ? 1 : 3); /* with small sums part of the step's launch, counted here too */
+  if (!p->small) {
+    PCK(oz_gemm(p->map_b, p->map_n, mix, p->nsm, p->st));
+    PCK(oz_refine<false>(OzRefine{TS, G, G, mix.split, p->beta, p->Gm, p->fac, p->max_br, p->max_n, p->sq_br, p->sq_n,
+                                  p->u, p->list_n, p->list},
+                         p->nsm, p->st));
+  }
   mark(p, PH_FORWARD, 1);
   IncStep A{};
   A.T = T;
   A.G = G;
   A.S = S;
-  A.split = mix.split;
   A.srisk = p->srisk;
   A.beta = p->beta;
   A.rpop = p->rpop;
@@ -689,16 +694,20 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
     mark(p, PH_NETWORK_GRAD, 1);
     const int smem = (int)sizeof(double) * (G > INC_THREADS ? G : INC_THREADS);
     k_inc_network_grad<true><<<G + 1, INC_THREADS, smem, p->st>>>(
-        G, T, TS, 1, nullptr, p->beta, p->gu, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
+        G, T, TS, nullptr, p->beta, p->gu, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
         p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
   } else {
     const int kt = depth_pad(TS);
-    k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->gu, nullptr, p->max_gu, p->gu_cols);
-    mark(p, PH_FLOWS, 1);
+    k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->gu, nullptr, p->max_gu, p->gu_cols,
+                                                                   p->sq_gu);
+    mark(p, PH_FLOWS, 3);
     PCK(oz_gemm(p->map_bt, p->map_gu, flows, p->nsm, p->st));
+    PCK(oz_refine<true>(OzRefine{G, G, TS, flows.split, p->beta, p->gu, nullptr, p->max_bc, p->max_gu, p->sq_bc, p->sq_gu,
+                                 p->C, p->list_n + 1, p->list},
+                        p->nsm, p->st));
     mark(p, PH_NETWORK_GRAD, 1);
     k_inc_network_grad<false><<<(G < 8 * p->nsm ? G : 8 * p->nsm) + 1, INC_THREADS, 0, p->st>>>(
-        G, T, TS, flows.split, p->C, nullptr, nullptr, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
+        G, T, TS, p->C, nullptr, nullptr, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
         p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
   }
   return plan_cuda(cudaGetLastError(), "gradient launch");
@@ -809,11 +818,14 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
       if (!p->small) {
         const int kg = depth_pad(G), kt = depth_pad(TS);
         rc = plan_cuda(cudaMemsetAsync(p->max_bc, 0, sizeof(unsigned long long) * G, p->st), "clear maxima");
+        if (rc == LPG_OK) rc = plan_cuda(cudaMemsetAsync(p->sq_bc, 0, sizeof(uint32_t) * G, p->st), "clear sums");
+        if (rc == LPG_OK) rc = plan_cuda(cudaMemsetAsync(p->sq_br, 0, sizeof(uint32_t) * TS, p->st), "clear sums");
         k_oz_row_max<<<(TS + 7) / 8, 256, 0, p->st>>>(TS, G, p->beta, p->max_br);
-        k_oz_slice_rows<<<dim3(TS, (kg / 2 + 255) / 256), 256, 0, p->st>>>(TS, G, kg, p->beta, p->max_br, p->b_rows);
+        k_oz_slice_rows<<<dim3(TS, (kg / 2 + 255) / 256), 256, 0, p->st>>>(TS, G, kg, p->beta, p->max_br, p->b_rows,
+                                                                              p->sq_br);
         k_oz_col_max<<<oz_col_grid(TS, G), 256, 0, p->st>>>(TS, G, p->beta, nullptr, p->max_bc);
         k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->beta, nullptr, p->max_bc,
-                                                                        p->b_cols);
+                                                                        p->b_cols, p->sq_bc);
       }
       if (rc == LPG_OK) rc = plan_cuda(cudaGetLastError(), "log launch");
     }

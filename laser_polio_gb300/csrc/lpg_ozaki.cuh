@@ -23,9 +23,9 @@
  * stage from 3.4 to 1.7 us; loads and products in warps of their own took
  * a stage from 2.9 us to those 1.7.  Measured: 1095 x 774 x 774 in 70 us,
  * 774 x 774 x 1095 in 61, 270 x 4000 x 4000 in 358, 4000 x 4000 x 270 in 307
- * (double-float on the FP32 pipe: 311, 355, 2015 and 1821); error 1e-16 of
- * the summed terms, rms.  An element's error is relative to its row's and
- * column's largest, not to itself.
+ * (double-float on the FP32 pipe: 311, 355, 2015 and 1821).  An element's
+ * error is relative to its row's and column's largest, not to itself, so
+ * k_oz_refine forms the elements again that are small beside those.
  *
  * Non-finite elements make their whole row or column scale NaN, and so
  * every element of C they take part in, as in a product that adds NaN.
@@ -95,6 +95,23 @@ __device__ __forceinline__ void oz_digits(double x, int e, uint16_t out[OZ_SLICE
   out[0] = (uint16_t)(__float_as_uint((float)(int)v) >> 16);
 }
 
+#define OZ_SQ_BITS 13       /* fraction bits of the sums of squares */
+
+/* |x| 2^-e as FP32, truncated; 0 below 2^-126 and for subnormal x. */
+__device__ __forceinline__ float oz_scaled_abs(double x, int e) {
+  const uint32_t h = (uint32_t)(oz_abs_bits(x) >> 32), l = (uint32_t)__double2loint(x);
+  const int ex = (int)(h >> 20) - 1023 - e + 127;
+  if (ex <= 0 || h < 0x100000u) return 0.0f;
+  if (ex >= 255) return __uint_as_float(0x7f7fffffu);
+  return __uint_as_float((uint32_t)ex << 23 | (h & 0xfffffu) << 3 | l >> 29);
+}
+
+/* The square of x 2^-e with OZ_SQ_BITS fraction bits, rounded up. */
+__device__ __forceinline__ uint32_t oz_square(double x, int e) {
+  const float f = oz_scaled_abs(x, e);
+  return e == OZ_NAN_EXP || f == 0.0f ? 0u : (uint32_t)(f * f * (float)(1 << OZ_SQ_BITS)) + 1u;
+}
+
 /* max |x| of every row / column of src [R][C] (bits; the caller clears max). */
 __global__ void __launch_bounds__(256) k_oz_row_max(int R, int C, const double* __restrict__ src, unsigned long long* max) {
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -131,16 +148,20 @@ __global__ void __launch_bounds__(256)
   atomicMax(&max[c], m);
 }
 
-/* dst [8][R][Kp] from src [R][K], scaled by rows; two depths a thread. */
+/* dst [8][R][Kp] from src [R][K], scaled by rows; two depths a thread.  The
+ * scaled rows' sums of squares are added to sq. */
 __global__ void __launch_bounds__(256)
     k_oz_slice_rows(int R, int K, int Kp, const double* __restrict__ src, const unsigned long long* __restrict__ max,
-                    uint32_t* __restrict__ dst) {
+                    uint32_t* __restrict__ dst, uint32_t* __restrict__ sq) {
   const int r = blockIdx.x, k = 2 * (blockIdx.y * 256 + threadIdx.x);
-  if (k >= Kp) return;
   const int e = oz_exp(max[r]);
+  const double x = k < K ? src[(size_t)r * K + k] : 0.0, y = k + 1 < K ? src[(size_t)r * K + k + 1] : 0.0;
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, oz_square(x, e) + oz_square(y, e));
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&sq[r], sum);
+  if (k >= Kp) return;
   uint16_t a[OZ_SLICES], b[OZ_SLICES];
-  oz_digits(k < K ? src[(size_t)r * K + k] : 0.0, e, a);
-  oz_digits(k + 1 < K ? src[(size_t)r * K + k + 1] : 0.0, e, b);
+  oz_digits(x, e, a);
+  oz_digits(y, e, b);
 #pragma unroll
   for (int s = 0; s < OZ_SLICES; ++s)
     dst[((size_t)s * R + r) * (Kp / 2) + k / 2] = (uint32_t)a[s] | (uint32_t)b[s] << 16;
@@ -148,10 +169,11 @@ __global__ void __launch_bounds__(256)
 
 /* dst [8][C][Kp] from src [K][C] (times fac[k], when given), scaled by columns: 32 x 32 tiles turned in
  * shared memory, then two depths a thread, so that sixteen threads write one
- * 64-byte run.  Bound by the integer digit extraction and the writes. */
+ * 64-byte run.  The scaled columns' sums of squares are added to sq.  Bound by
+ * the integer digit extraction and the writes. */
 __global__ void __launch_bounds__(256)
     k_oz_slice_cols(int K, int C, int Kp, const double* __restrict__ src, const double* __restrict__ fac,
-                    const unsigned long long* __restrict__ max, uint32_t* __restrict__ dst) {
+                    const unsigned long long* __restrict__ max, uint32_t* __restrict__ dst, uint32_t* __restrict__ sq) {
   __shared__ double s[32][33];
   const int c0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -170,6 +192,9 @@ __global__ void __launch_bounds__(256)
     uint16_t a[OZ_SLICES], b[OZ_SLICES];
     oz_digits(s[2 * kp][cl], e, a);
     oz_digits(s[2 * kp + 1][cl], e, b);
+    const uint32_t sum = __reduce_add_sync(0xffffu << (threadIdx.x & 16), oz_square(s[2 * kp][cl], e) +
+                                                                              oz_square(s[2 * kp + 1][cl], e));
+    if (kp == 0 && sum) atomicAdd(&sq[c], sum);
 #pragma unroll
     for (int i = 0; i < OZ_SLICES; ++i)
       dst[((size_t)i * C + c) * (Kp / 2) + k0 / 2 + kp] = (uint32_t)a[i] | (uint32_t)b[i] << 16;
@@ -472,6 +497,267 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+/* --- elements the digits cannot hold ------------------------------------------ */
+/* A digit product's element is off by about 2^-57 of its row's scale times
+ * its column's, and a sum over the depth by e = 2^-56.8 sqrt(sum a^2 + sum
+ * b^2) of them (a, b scaled to 1: a rounding of half of 2^-55 each, uniform).
+ * Where the element itself is small beside the two scales — a wave that has
+ * not reached the other's node, a flow across the map, one large node above
+ * a background — that is too much of it.  So an element is kept only where
+ * its summed terms are at least 2^45 e, so that it is off by at most 2^-45 of
+ * them (rms) as any element of a product of FP32 pairs is (rms 2^-45, 2^-42
+ * at worst, 774 terms).  |C| bounds the sum of the terms' magnitudes from
+ * below, and equals it where no signs differ. */
+#define OZ_KEEP 0x1.26p-12f /* 2^(45 - 56.8) */
+
+/* sqrt(sum a^2 + sum b^2) */
+__device__ __forceinline__ float oz_norm(uint32_t sa, uint32_t sb) {
+  return sqrtf(((float)sa + (float)sb) * (1.0f / (1 << OZ_SQ_BITS)));
+}
+
+/* Whether an element whose value is c cannot stay as the digits gave it. */
+__device__ __forceinline__ bool oz_small(double c, int ea, int eb, uint32_t sa, uint32_t sb) {
+  if (ea == OZ_NAN_EXP || eb == OZ_NAN_EXP || sa == 0 || sb == 0) return false; /* NaN, or exactly 0 */
+  return oz_scaled_abs(c, ea + eb) < OZ_KEEP * oz_norm(sa, sb);
+}
+
+/* x 2^(30 - e) as an FP32 pair: 24 bits cut off, the 29 below them rounded
+ * (30: room below for what is small beside the scale). */
+__device__ __forceinline__ float2 oz_pair(double x, int e) {
+  const uint64_t b = oz_abs_bits(x);
+  const int ex = (int)(b >> 52) - 1023 + 30 - e + 127;
+  if (e == OZ_NAN_EXP || ex <= 0 || b >> 52 == 0) return make_float2(0.f, 0.f);
+  const uint32_t sign = (uint32_t)(__double2hiint(x)) & 0x80000000u;
+  const float hi = __uint_as_float(sign | (uint32_t)ex << 23 | (uint32_t)(b >> 29 & 0x7fffffu));
+  const float low = (float)(uint32_t)(b & 0x1fffffffu); /* units of 2^(ex - 127 - 52) */
+  const float unit = ex > 52 ? __uint_as_float((uint32_t)(ex - 52) << 23) : 0.f;
+  return make_float2(hi, __uint_as_float(__float_as_uint(__fmul_rn(low, unit)) | sign));
+}
+
+/* (sh, sl) += a * b for FP32 pairs a, b: the exact product of the high
+ * parts (Dekker, by FMA) plus the cross terms, added by Knuth's TwoSum. */
+__device__ __forceinline__ void oz_pair_fma(float& sh, float& sl, float2 a, float2 b) {
+  const float ph = __fmul_rn(a.x, b.x);
+  float pl = __fmaf_rn(a.x, b.x, -ph);
+  pl = __fmaf_rn(a.x, b.y, pl);
+  pl = __fmaf_rn(a.y, b.x, pl);
+  const float s = __fadd_rn(sh, ph);
+  const float bp = __fsub_rn(s, sh);
+  const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bp)), __fsub_rn(ph, bp));
+  sl = __fadd_rn(sl, __fadd_rn(err, pl));
+  sh = s;
+}
+
+struct OzRefine {
+  int M, N, K, split;
+  const double *A, *B; /* A [M][K], or [K][M]; B [K][N], its row k times fac[k] where given */
+  const double* fac;
+  const unsigned long long *max_a, *max_b;
+  const uint32_t *sq_a, *sq_b;
+  double* C; /* [split][M][N] */
+  unsigned long long* count; /* entries of the list; cleared by the caller */
+  uint64_t* list;            /* elements m N + n; OZ_R_LIST for each tile */
+};
+
+#define OZ_R_THREADS 128
+#define OZ_R_BM 32
+#define OZ_R_BN 64
+#define OZ_R_BK 32
+#define OZ_R_LIST 128 /* elements of a tile formed one by one */
+
+/* Adds the depth slices into the first one, and finds the elements that
+ * oz_small names, a 32 x 64 tile a CTA.  Up to OZ_R_LIST of them go to the list (k_oz_fix); where there are more, they are
+ * formed here by a product of FP32 pairs over the whole tile (2048 elements
+ * of 774 terms: 75 us an SM in pairs, about 0.4 us an element in FP64, so the
+ * line lies near 128).  Bound by reading C where nothing is small; with
+ * k_oz_fix 17 and 18 us for the two products of 774 nodes, 365 ticks and 3
+ * strains (0.1% of the mixing's elements are small), 54 and 44 us of 4000
+ * nodes and 90 ticks. */
+template <bool TRANS_A>
+__global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
+  __shared__ int s_ea[OZ_R_BM], s_eb[OZ_R_BN], s_count, s_need;
+  __shared__ unsigned long long s_at;
+  __shared__ uint32_t s_sa[OZ_R_BM], s_sb[OZ_R_BN];
+  __shared__ uint16_t s_list[OZ_R_LIST];
+  const int tid = threadIdx.x, m0 = blockIdx.y * OZ_R_BM, n0 = blockIdx.x * OZ_R_BN;
+  if (tid < OZ_R_BN) {
+    const bool in = n0 + tid < R.N;
+    s_eb[tid] = in ? oz_exp(R.max_b[n0 + tid]) : 0;
+    s_sb[tid] = in ? R.sq_b[n0 + tid] : 0;
+  } else if (tid < OZ_R_BN + OZ_R_BM) {
+    const int r = tid - OZ_R_BN;
+    const bool in = m0 + r < R.M;
+    s_ea[r] = in ? oz_exp(R.max_a[m0 + r]) : 0;
+    s_sa[r] = in ? R.sq_a[m0 + r] : 0;
+  }
+  if (tid == 0) s_count = 0;
+  __syncthreads();
+  if (tid < 32) {
+    const uint32_t top = max(max(s_sa[tid], s_sb[tid]), s_sb[tid + 32]);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, top);
+    /* the biased exponent that an element scaled by 2^(ea + eb) needs at most */
+    if (tid == 0) s_need = (int)(__float_as_uint(OZ_KEEP * oz_norm(most, most)) >> 23) - 127 + 1023 + 1;
+  }
+  __syncthreads();
+  auto where = [&](int r, int c) { return (size_t)(m0 + r) * R.N + n0 + c; };
+  auto small = [&](int r, int c) {
+    return m0 + r < R.M && n0 + c < R.N && oz_small(R.C[where(r, c)], s_ea[r], s_eb[c], s_sa[r], s_sb[c]);
+  };
+  /* a thread's column is one, so that an element is first compared by its
+   * exponent with the most that any of the tile could need; only those below
+   * are looked at closely */
+  const int c = tid % OZ_R_BN, r0 = tid / OZ_R_BN;
+  const int need = s_need + (s_eb[c] == OZ_NAN_EXP ? 0 : s_eb[c]);
+  if (n0 + c < R.N) {
+    constexpr int PER = OZ_R_BM * OZ_R_BN / OZ_R_THREADS, STEP = OZ_R_THREADS / OZ_R_BN;
+    double v[PER]; /* a slice's loads in flight together */
+#pragma unroll
+    for (int i = 0; i < PER; ++i) v[i] = m0 + r0 + i * STEP < R.M ? R.C[where(r0 + i * STEP, c)] : 0.0;
+#pragma unroll 1
+    for (int z = 1; z < R.split; ++z) {
+      const double* Cz = R.C + z * ((size_t)R.M * R.N);
+      double w[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) w[i] = m0 + r0 + i * STEP < R.M ? Cz[where(r0 + i * STEP, c)] : 0.0;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) v[i] += w[i];
+    }
+    if (R.split > 1)
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (m0 + r0 + i * STEP < R.M) R.C[where(r0 + i * STEP, c)] = v[i];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int r = r0 + i * STEP;
+      if ((__double2hiint(v[i]) >> 20 & 0x7ff) - s_ea[r] >= need || m0 + r >= R.M) continue;
+      if (!oz_small(v[i], s_ea[r], s_eb[c], s_sa[r], s_sb[c])) continue;
+      const int at = atomicAdd(&s_count, 1);
+      if (at < OZ_R_LIST) s_list[at] = (uint16_t)(r * OZ_R_BN + c);
+    }
+  }
+  __syncthreads();
+  const int todo = s_count;
+  if (todo == 0) return;
+  if (todo <= OZ_R_LIST) {
+    if (tid == 0) s_at = atomicAdd(R.count, (unsigned long long)todo);
+    __syncthreads();
+    if (tid < todo) R.list[s_at + tid] = where(s_list[tid] / OZ_R_BN, s_list[tid] % OZ_R_BN);
+    return;
+  }
+  __shared__ float2 sA[OZ_R_BK][OZ_R_BM + 1]; /* [k][m] */
+  __shared__ float2 sB[OZ_R_BK][OZ_R_BN];     /* [k][n] */
+  const int tx = tid & 15, ty = tid >> 4;
+  float sh[4][4], sl[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sh[i][j] = sl[i][j] = 0.f;
+#pragma unroll 1
+  for (int k0 = 0; k0 < R.K; k0 += OZ_R_BK) {
+#pragma unroll
+    for (int q = 0; q < (OZ_R_BK * OZ_R_BM) / OZ_R_THREADS; ++q) {
+      const int e = tid + q * OZ_R_THREADS;
+      const int hi = e >> 5, lo = e & 31;
+      /* consecutive threads read consecutive m, or consecutive k */
+      const int k = TRANS_A ? hi : lo, m = TRANS_A ? lo : hi;
+      float2 v = make_float2(0.f, 0.f);
+      if (k0 + k < R.K && m0 + m < R.M)
+        v = oz_pair(R.A[TRANS_A ? (size_t)(k0 + k) * R.M + m0 + m : (size_t)(m0 + m) * R.K + k0 + k], s_ea[m]);
+      sA[k][m] = v;
+    }
+#pragma unroll
+    for (int q = 0; q < (OZ_R_BK * OZ_R_BN) / OZ_R_THREADS; ++q) {
+      const int e = tid + q * OZ_R_THREADS;
+      const int k = e >> 6, n = e & 63;
+      float2 v = make_float2(0.f, 0.f);
+      if (k0 + k < R.K && n0 + n < R.N)
+        v = oz_pair(oz_scaled(R.B[(size_t)(k0 + k) * R.N + n0 + n], R.fac, k0 + k), s_eb[n]);
+      sB[k][n] = v;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int q = 0; q < OZ_R_BK; ++q) {
+      float2 av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) av[i] = sA[q][ty + 8 * i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bv[j] = sB[q][tx + 16 * j];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) oz_pair_fma(sh[i][j], sl[i][j], av[i], bv[j]);
+    }
+    /* renormalise each pair (Fast2Sum: |sh| >= |sl|) so that sl stays small */
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float t = __fadd_rn(sh[i][j], sl[i][j]);
+        sl[i][j] = __fsub_rn(sl[i][j], __fsub_rn(t, sh[i][j]));
+        sh[i][j] = t;
+      }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = ty + 8 * i, c = tx + 16 * j;
+      if (small(r, c)) R.C[where(r, c)] = scalbn((double)sh[i][j] + (double)sl[i][j], s_ea[r] + s_eb[c] - 60);
+    }
+}
+
+/* The listed elements, a CTA each, in FP64.  Where terms may cancel
+ * (TRANS_A: dL/du has both signs) an element is given up as soon as the
+ * terms' magnitudes show that it is good.  Bound by the latency of the
+ * column's reads, a sector each. */
+template <bool TRANS_A>
+__global__ void __launch_bounds__(OZ_R_THREADS) k_oz_fix(OzRefine R) {
+  __shared__ double s_acc[OZ_R_THREADS / 32];
+  __shared__ float s_mag[OZ_R_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned long long todo = *R.count;
+  for (unsigned long long q = blockIdx.x; q < todo; q += gridDim.x) {
+    const size_t at = R.list[q], m = at / R.N, n = at % R.N;
+    const int ea = oz_exp(R.max_a[m]), eb = oz_exp(R.max_b[n]);
+    const float keep = OZ_KEEP * oz_norm(R.sq_a[m], R.sq_b[n]);
+    const double *a = R.A + (TRANS_A ? m : m * R.K), *b = R.B + n;
+    double acc = 0.0;
+    float mag = 0.f, all = 0.f;
+    for (int k0 = 0; k0 < R.K && !(all >= keep); k0 += 8 * OZ_R_THREADS) { /* all: the same in every thread */
+      double x[8], y[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = k0 + u * OZ_R_THREADS + threadIdx.x;
+        x[u] = k < R.K ? a[TRANS_A ? (size_t)k * R.M : (size_t)k] : 0.0;
+        y[u] = k < R.K ? b[(size_t)k * R.N] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = k0 + u * OZ_R_THREADS + threadIdx.x;
+        if (k >= R.K) break;
+        y[u] = oz_scaled(y[u], R.fac, k);
+        acc = __fma_rn(x[u], y[u], acc);
+        if (TRANS_A) mag += oz_scaled_abs(x[u], ea) * oz_scaled_abs(y[u], eb);
+      }
+      if (TRANS_A) {
+        float w = mag;
+        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if (lane == 0) s_mag[warp] = w;
+        __syncthreads();
+        all = (s_mag[0] + s_mag[1]) + (s_mag[2] + s_mag[3]);
+        __syncthreads();
+      }
+    }
+    if (all >= keep) continue;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __syncthreads();
+    if (lane == 0) s_acc[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) R.C[at] = (s_acc[0] + s_acc[1]) + (s_acc[2] + s_acc[3]);
+  }
+}
+
 /* --- host side -------------------------------------------------------------- */
 inline dim3 oz_col_grid(int R, int C) { return dim3((C + 255) / 256, (R + OZ_MAX_ROWS - 1) / OZ_MAX_ROWS); }
 
@@ -517,6 +803,18 @@ inline cudaError_t oz_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const O
   if (e != cudaSuccess) return e;
   const int units = G.tiles * G.split;
   k_oz_gemm<<<units < nsm ? units : nsm, OZ_THREADS, OZ_SMEM, st>>>(ta, tb, G);
+  return cudaGetLastError();
+}
+
+/* Entries of an M x N product's list. */
+inline size_t oz_list(int M, int N) {
+  return (size_t)OZ_R_LIST * ((N + OZ_R_BN - 1) / OZ_R_BN) * ((M + OZ_R_BM - 1) / OZ_R_BM);
+}
+
+template <bool TRANS_A>
+inline cudaError_t oz_refine(const OzRefine& R, int nsm, cudaStream_t st) {
+  k_oz_refine<TRANS_A><<<dim3((R.N + OZ_R_BN - 1) / OZ_R_BN, (R.M + OZ_R_BM - 1) / OZ_R_BM), OZ_R_THREADS, 0, st>>>(R);
+  k_oz_fix<TRANS_A><<<16 * nsm, OZ_R_THREADS, 0, st>>>(R);
   return cudaGetLastError();
 }
 
