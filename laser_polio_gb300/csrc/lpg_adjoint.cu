@@ -23,7 +23,7 @@
  * L = sum (log1p(lam) - log1p(target))^2 and its dL/dlam on the device.
  *
  * Layout in HBM: a plan keeps the aggregates resident — srisk and
- * 1/max(pop, 1) [T][G]; beta as [T][S][G] (strain-major per tick, so that the
+ * max(pop, 1) [T][G]; beta as [T][S][G] (strain-major per tick, so that the
  * (t, s) rows of the mixing product and every elementwise pass read G
  * consecutive doubles); u and dL/du the same way; log(dist), log2(dist) and
  * the flows and their gradients [G][G]; log(pops) [G].
@@ -108,13 +108,13 @@ __device__ __forceinline__ int64_t inc_log2(double x) {
 }
 
 /* log(pops), log2(pops) [G]; log(dist), log2(dist) [G][G] (the diagonal is
- * never read); 1/max(pop, 1) and log1p(target) [T][G]: once per plan.  The
+ * never read); max(pop, 1) and log1p(target) [T][G]: once per plan.  The
  * distances' log2 in integers: one FP64 logarithm a cell, not two (774 nodes:
  * 1.03 ms with both, about half now; ln in integers would be 0.9 ulp off
  * where CUDA's is 0.54). */
 __global__ void __launch_bounds__(INC_THREADS)
     k_inc_logs(const IxTables* tab, int G, size_t TG, const double* pops, const double* dist, double* logp,
-               double* logd, int64_t* lp2, int64_t* ld2, const double* pop, double* rpop, double* target) {
+               double* logd, int64_t* lp2, int64_t* ld2, const double* pop, double* popc, double* target) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < (size_t)G * G) {
     const double x = dist[idx];
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(INC_THREADS)
     lp2[idx] = inc_log2(pops[idx]);
   }
   if (idx < TG) {
-    rpop[idx] = 1.0 / fmax(pop[idx], 1.0);
+    popc[idx] = fmax(pop[idx], 1.0);
     if (target) target[idx] = log1p(target[idx]);
   }
 }
@@ -247,18 +247,9 @@ __device__ __forceinline__ double inc_log1p(const IxTables* tab, double y) {
   return ix_below(y, 0x1p60) && !ix_below(y, 0x1p-5) ? ix_log1p(tab, y) : log1p(y);
 }
 
-/* 1/d for d >= 1, to within an ulp: the hardware estimate, two Newton steps. */
-__device__ __forceinline__ double inc_recip(double d) {
-  if (!ix_below(d, 1e300) || ix_below(d, 1.0)) return 1.0 / d;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-  return __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-}
-
 struct IncStep {
   int T, G, S;
-  const double *srisk, *beta, *rpop, *seas, *r0s, *rsN, *ltarget, *g_in;
+  const double *srisk, *beta, *popc, *seas, *r0s, *rsN, *ltarget, *g_in;
   const double* u; /* the mixing product, or */
   const double* N; /* the normalised network (small sums) */
   double R;
@@ -294,8 +285,9 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
     const int t = t0 + i;
     if (!in || t >= T) continue;
     const size_t idx = (size_t)t * G + n;
-    const double st = A.seas[t], ip = A.rpop[idx];
-    const double q = st * A.R * r0 * ip;
+    const double st = A.seas[t];
+    const IxDivisor popc(A.popc[idx]);
+    const double q = popc.of(st * r0 * A.R);
     double uu[LPG_MAX_STRAINS], ex[LPG_MAX_STRAINS], l = 0.0, mix[LPG_MAX_STRAINS] = {0.0, 0.0, 0.0, 0.0};
     if (SMALL) {
       const double* b = A.beta + (size_t)t * S * G;
@@ -321,7 +313,7 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
     double g = 0.0;
     if (A.ltarget) {
       const double r = inc_log1p(tab, lv) - A.ltarget[idx];
-      g = 2.0 * r * inc_recip(1.0 + lv);
+      g = IxDivisor(1.0 + lv).of(2.0 * r);
       loss = __fma_rn(r, r, loss);
     }
     if (!A.grad) continue;
@@ -338,7 +330,7 @@ __global__ void __launch_bounds__(128, SMALL ? 4 : 6) k_inc_step(const IxTables*
       mx = b > mx ? b : mx;
       gq = __fma_rn(gr, uu[s], gq);
     }
-    const double gp = gq * ip;
+    const double gp = popc.of(gq);
     w[i] = gp * r0;
     acc_r0 = __fma_rn(gp * st, A.R, acc_r0);
   }
@@ -471,7 +463,7 @@ struct lpg_incidence_plan {
   double max_lp2 = 0.0, max_ld2 = 0.0; /* largest finite |log2 pops|, |log2 dist| */
   bool small = false;                  /* the contractions summed in FP64 where they are used */
   /* resident inputs */
-  double *srisk = nullptr, *beta = nullptr, *rpop = nullptr, *doy = nullptr, *year = nullptr, *pops = nullptr,
+  double *srisk = nullptr, *beta = nullptr, *popc = nullptr, *doy = nullptr, *year = nullptr, *pops = nullptr,
          *logp = nullptr, *logd = nullptr, *target = nullptr; /* target: its log1p */
   int64_t *lp2 = nullptr, *ld2 = nullptr;
   IxTables* tab = nullptr;
@@ -522,7 +514,7 @@ int dalloc(T** p, size_t n) {
 }
 
 void plan_free(lpg_incidence_plan* p) {
-  void* ps[] = {p->srisk, p->beta, p->rpop, p->doy,  p->year,    p->pops,   p->logp,   p->logd,    p->target,
+  void* ps[] = {p->srisk, p->beta, p->popc, p->doy,  p->year,    p->pops,   p->logp,   p->logd,    p->target,
                 p->lp2,   p->ld2,  p->tab,  p->r0s,  p->seas,    p->Gm,     p->rs,     p->rsN,     p->fac,
                 p->u,     p->lam,  p->g,    p->C,    p->gN,      p->sums,   p->N,
                 p->gu,    p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc,
@@ -544,7 +536,7 @@ int depth_pad(int k) { return (k + OZ_BK - 1) / OZ_BK * OZ_BK; }
 int plan_alloc(lpg_incidence_plan* p) {
   const size_t T = p->T, G = p->G, TG = T * G, TSG = TG * p->S, GG = G * G, TS = T * p->S;
   int rc;
-  if ((rc = dalloc(&p->srisk, TG)) || (rc = dalloc(&p->beta, TSG)) || (rc = dalloc(&p->rpop, TG)) ||
+  if ((rc = dalloc(&p->srisk, TG)) || (rc = dalloc(&p->beta, TSG)) || (rc = dalloc(&p->popc, TG)) ||
       (rc = dalloc(&p->doy, T)) || (rc = dalloc(&p->year, T)) || (rc = dalloc(&p->pops, G)) ||
       (rc = dalloc(&p->logp, G)) || (rc = dalloc(&p->logd, GG)) || (rc = dalloc(&p->r0s, G)) ||
       (rc = dalloc(&p->lp2, G)) || (rc = dalloc(&p->ld2, GG)) || (rc = dalloc(&p->tab, 1)) ||
@@ -669,7 +661,7 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   A.S = S;
   A.srisk = p->srisk;
   A.beta = p->beta;
-  A.rpop = p->rpop;
+  A.popc = p->popc;
   A.seas = p->seas;
   A.r0s = p->r0s;
   A.rsN = p->rsN;
@@ -794,7 +786,7 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
       double* dst;
       const double* src;
       size_t n;
-    } up[] = {{p->srisk, in->srisk, TG},       {p->beta, bt.data(), TG * S},        {p->rpop, in->pop, TG},
+    } up[] = {{p->srisk, in->srisk, TG},       {p->beta, bt.data(), TG * S},        {p->popc, in->pop, TG},
               {p->doy, in->doy, (size_t)T},    {p->year, in->year, (size_t)T},      {p->pops, in->pops, (size_t)G},
               {d_dist, in->dist, GG}};
     for (auto& c : up) {
@@ -813,7 +805,7 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
     if (rc == LPG_OK) {
       const size_t cells = GG > TG ? GG : TG;
       k_inc_logs<<<(unsigned)((cells + INC_THREADS - 1) / INC_THREADS), INC_THREADS, 0, p->st>>>(
-          p->tab, G, TG, p->pops, d_dist, p->logp, p->logd, p->lp2, p->ld2, p->rpop, p->rpop, p->target);
+          p->tab, G, TG, p->pops, d_dist, p->logp, p->logd, p->lp2, p->ld2, p->popc, p->popc, p->target);
       const int TS = T * S;
       if (!p->small) {
         const int kg = depth_pad(G), kt = depth_pad(TS);

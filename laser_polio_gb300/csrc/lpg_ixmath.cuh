@@ -64,6 +64,31 @@ __device__ __forceinline__ bool ix_below(double x, double hi) {
   return (uint64_t)__double_as_longlong(x) < (uint64_t)__double_as_longlong(hi);
 }
 
+/* Quotients by one divisor d: where d lies in [1, 2^500) the hardware's
+ * estimate of 1/d, one Newton step and Markstein's correction (P. Markstein,
+ * "Computation of elementary functions on the IBM RISC System/6000
+ * processor", IBM J. Res. Develop. 34, 1990): the quotient, its remainder by
+ * a fused multiply-add, and that times 1/d added.  The estimate's 20 bits
+ * become 76, so the quotient is the correctly rounded one but for one in
+ * millions, in five FP64 operations, three for a further dividend. */
+struct IxDivisor {
+  double d, y;
+  bool fast;
+  __device__ __forceinline__ explicit IxDivisor(double d_) : d(d_) {
+    const uint32_t e = (uint32_t)((uint64_t)__double_as_longlong(d) >> 52); /* sign and exponent */
+    fast = e - 1023u < 500u;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+  }
+  /* n / d */
+  __device__ __forceinline__ double of(double n) const {
+    const uint64_t b = (uint64_t)__double_as_longlong(n) << 1;
+    if (!fast || ((uint32_t)(b >> 53) - 523u >= 1000u && b != 0)) return n / d;
+    const double q = n * y;
+    return __fma_rn(__fma_rn(-q, d, n), y, q);
+  }
+};
+
 /* e^-x for 0 <= x < 2^-7: 1 - d, d = x - x^2 (1/2 - x (1/6 - x (1/24 - x
  * (1/120 - x (1/720 - x/5040))))) with 71 fraction bits, so that the result
  * is the correctly rounded one but for about one x in 1e5 at 2^-10 (1 - e^-x
