@@ -109,7 +109,7 @@ __device__ __forceinline__ double ix_exp_neg_small(double x) {
   return __longlong_as_double((long long)((1021ULL << 52) + (1ULL << 53) - ((D + (1ULL << 17)) >> 18)));
 }
 
-/* e^-x for 0 <= x < 700; below 1/2 from x / ln 2 with 64 fraction bits. */
+/* e^-x for 0 <= x < 700, from x / ln 2 with 64 fraction bits. */
 __device__ __forceinline__ double ix_exp_neg(const IxTables* T, double x) {
   if (ix_below(x, 0x1p-7)) return ix_exp_neg_small(x);
   int n;
@@ -122,10 +122,10 @@ __device__ __forceinline__ double ix_exp_neg(const IxTables* T, double x) {
     f = 0ULL - (__umul64hi(X, IX_LOG2E_63) << 2 | X * IX_LOG2E_63 >> 62);
     n = f ? -1 : 0;
   } else {
-    const uint64_t X = ix_fixed53(x);
-    const int64_t E = -(int64_t)(__umul64hi(X, IX_LOG2E_63) + (X * IX_LOG2E_63 >> 63)); /* 52 fraction bits */
-    n = (int)(E >> 52);
-    f = (uint64_t)E << 12;
+    const uint64_t X = ix_fixed53(x); /* exact: x has no lower bits */
+    const uint64_t hi = __umul64hi(X, IX_LOG2E_63), lo = X * IX_LOG2E_63; /* x / ln 2, 52 and 64 fraction bits */
+    f = 0ULL - (hi << 12 | lo >> 52);
+    n = -(int)(hi >> 52) - (f ? 1 : 0);
   }
   return ix_double(ix_exp2_frac(T, f), n);
 }
