@@ -25,16 +25,19 @@
  * Layout in HBM: a plan keeps the aggregates resident — srisk and
  * max(pop, 1) [T][G]; beta as [T][S][G] (strain-major per tick, so that the
  * (t, s) rows of the mixing product and every elementwise pass read G
- * consecutive doubles); u and dL/du the same way; log(dist), log2(dist) and
- * the flows and their gradients [G][G]; log(pops) [G].
+ * consecutive doubles); u the same way, and dL/du in its place; log(dist),
+ * log2(dist) and the flows and their gradients [G][G]; log(pops) [G].  The
+ * sliced products' digits take 48 bytes an element of beta up to INC_DIGITS
+ * elements, and no more than for those above: 200 MB.
  *
  * Arithmetic: double precision throughout, most of it without the FP64 unit.
  * GB300 issues about two FP64 FMAs per clock per SM, 128 FP32 or integer
  * operations, and 8192 bf16 tensor FMAs.
  *   - The two contractions, u = beta N per (t, s) row and dL/dN = beta^T
  *     dL/du, both (T S) x G x G, run on the tensor cores by exact slicing
- *     (lpg_ozaki.cuh).  beta's slices are formed once per plan, N's and
- *     dL/du's each evaluation.  An element that is small beside its row's and
+ *     (lpg_ozaki.cuh).  beta's slices are formed once per plan (by
+ *     columns with the target or at the first gradient), N's and dL/du's each
+ *     evaluation.  An element that is small beside its row's and
  *     column's scales is formed again from the FP64 operands, so that each
  *     element is good to 2^-45 of its own summed terms (four deviations; the
  *     FP32 pairs used where many are small: rms).
@@ -65,6 +68,7 @@ constexpr double kTwoPi = 6.283185307179586476925286766559;
 #define INC_MAX_ROWS (65535 * 32)
 #define INC_SMALL_NODES 128
 #define INC_SMALL_TERMS 4000000 /* T S G^2 */
+#define INC_DIGITS (1 << 22)    /* elements of beta whose digits a plan keeps (16 bytes each) */
 
 enum { PH_NETWORK, PH_MIX, PH_FORWARD, PH_BACKWARD, PH_FLOWS, PH_NETWORK_GRAD, PH_COUNT };
 const char* const kPhaseNames[PH_COUNT] = {"k_inc_network", "k_inc_gemm_mix", "k_inc_forward",
@@ -476,13 +480,17 @@ struct lpg_incidence_plan {
   unsigned long long *max_n = nullptr, *max_gu = nullptr;
   uint32_t *sq_n = nullptr, *sq_gu = nullptr;
   size_t clear_bytes = 0;
-  double *N = nullptr, *gu = nullptr;
-  /* the sliced products: digits, row and column maxima and sums of squares, tensor maps */
+  double *N = nullptr, *gu = nullptr; /* gu of the sliced products: in u's place */
+  /* the sliced products: digits, row and column maxima and sums of squares, tensor maps.  Digits of row_cap rows
+   * or dep_cap depths of beta at a time: all of them, kept, up to INC_DIGITS elements; above, a part after another in
+   * every evaluation.  n_cols and C share their memory (the
+   * mixing is done with the one before the flows write the other), gu_cols and the list theirs. */
+  int row_cap = 0, dep_cap = 0;
+  bool rows_ready = false, cols_ready = false, bc_ready = false;
   uint32_t *b_rows = nullptr, *b_cols = nullptr, *n_cols = nullptr, *gu_cols = nullptr;
   unsigned long long *max_br = nullptr, *max_bc = nullptr;
   uint32_t *sq_br = nullptr, *sq_bc = nullptr;
   unsigned long long* list_n = nullptr; /* two of the sums */
-  uint64_t* list = nullptr;
   CUtensorMap map_b{}, map_n{}, map_bt{}, map_gu{};
   double* host = nullptr; /* pinned: sums and gr0s [SC_N + G], then r0s [G] */
   /* profiling */
@@ -516,9 +524,9 @@ int dalloc(T** p, size_t n) {
 void plan_free(lpg_incidence_plan* p) {
   void* ps[] = {p->srisk, p->beta, p->popc, p->doy,  p->year,    p->pops,   p->logp,   p->logd,    p->target,
                 p->lp2,   p->ld2,  p->tab,  p->r0s,  p->seas,    p->Gm,     p->rs,     p->rsN,     p->fac,
-                p->u,     p->lam,  p->g,    p->C,    p->gN,      p->sums,   p->N,
-                p->gu,    p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc,
-                p->sq_br, p->sq_bc, p->list};
+                p->u,     p->lam,  p->g,    p->gN,   p->sums,    p->N,
+                p->small ? p->gu : nullptr, p->b_rows, p->b_cols, p->n_cols, p->gu_cols, p->max_br, p->max_bc,
+                p->sq_br, p->sq_bc};
   for (void* q : ps)
     if (q) cudaFree(q);
   if (p->host) cudaFreeHost(p->host);
@@ -554,22 +562,27 @@ int plan_alloc(lpg_incidence_plan* p) {
   p->max_gu = p->max_n + G;
   p->sq_n = reinterpret_cast<uint32_t*>(p->max_gu + G);
   p->sq_gu = p->sq_n + G;
-  if ((rc = dalloc(&p->gu, TSG))) return rc;
   if (!p->small) {
     const size_t kg = depth_pad(p->G), kt = depth_pad((int)TS), half = OZ_SLICES / 2; /* two digits a word */
+    const size_t tile = OZ_CHUNK * OZ_BK;
+    p->row_cap = (int)std::min(TS, TS * kg <= INC_DIGITS ? TS : std::max<size_t>(1, INC_DIGITS / kg / OZ_BM) * OZ_BM);
+    p->dep_cap = (int)std::min(kt, kt * G <= INC_DIGITS ? kt : std::max<size_t>(1, INC_DIGITS / G / tile) * tile);
     OzArgs mix{}, flows{};
     plan_products(p, &mix, &flows);
-    if ((rc = dalloc(&p->u, mix.split * TSG)) || (rc = dalloc(&p->C, flows.split * GG)) ||
-        (rc = dalloc(&p->b_rows, half * TS * kg)) ||
-        (rc = dalloc(&p->b_cols, half * G * kt)) || (rc = dalloc(&p->n_cols, half * G * kg)) ||
-        (rc = dalloc(&p->gu_cols, half * G * kt)) || (rc = dalloc(&p->max_br, TS)) || (rc = dalloc(&p->max_bc, G)) ||
-        (rc = dalloc(&p->sq_br, TS)) || (rc = dalloc(&p->sq_bc, G)) ||
-        (rc = dalloc(&p->list, std::max(oz_list((int)TS, p->G), oz_list(p->G, p->G)))))
+    const size_t words_n = std::max(half * G * kg, 2 * flows.split * GG);
+    const size_t words_gu =
+        std::max(half * G * p->dep_cap, 2 * std::max(oz_list((int)TS, p->G), oz_list(p->G, p->G)));
+    if ((rc = dalloc(&p->u, mix.split * TSG)) || (rc = dalloc(&p->b_rows, half * p->row_cap * kg)) ||
+        (rc = dalloc(&p->b_cols, half * G * p->dep_cap)) || (rc = dalloc(&p->n_cols, words_n)) ||
+        (rc = dalloc(&p->gu_cols, words_gu)) || (rc = dalloc(&p->max_br, TS)) || (rc = dalloc(&p->max_bc, G)) ||
+        (rc = dalloc(&p->sq_br, TS)) || (rc = dalloc(&p->sq_bc, G)))
       return rc;
-    if (!oz_map(&p->map_b, p->b_rows, (int)TS, (int)kg, OZ_BM) || !oz_map(&p->map_n, p->n_cols, p->G, (int)kg, OZ_BN) ||
-        !oz_map(&p->map_bt, p->b_cols, p->G, (int)kt, OZ_BM) || !oz_map(&p->map_gu, p->gu_cols, p->G, (int)kt, OZ_BN))
+    p->gu = p->u;
+    p->C = reinterpret_cast<double*>(p->n_cols);
+    if (!oz_map(&p->map_b, p->b_rows, p->row_cap, (int)kg, OZ_BM) || !oz_map(&p->map_n, p->n_cols, p->G, (int)kg, OZ_BN) ||
+        !oz_map(&p->map_bt, p->b_cols, p->G, p->dep_cap, OZ_BM) || !oz_map(&p->map_gu, p->gu_cols, p->G, p->dep_cap, OZ_BN))
       return lpg_ops_fail(LPG_ERR_CUDA, "incidence plan: a tensor map was refused");
-  } else if ((rc = dalloc(&p->N, GG))) {
+  } else if ((rc = dalloc(&p->N, GG)) || (rc = dalloc(&p->gu, TSG))) {
     return rc;
   }
   PCK(cudaMallocHost((void**)&p->host, (SC_N + 2 * G) * sizeof(double)));
@@ -584,23 +597,97 @@ inline void mark(lpg_incidence_plan* p, int ph, int n_launch) {
 }
 
 void plan_products(const lpg_incidence_plan* p, OzArgs* mix, OzArgs* flows) {
-  const int TS = p->T * p->S;
-  mix->M = TS;
+  mix->M = p->row_cap;
   mix->N = p->G;
   mix->k_stages = depth_pad(p->G) / OZ_BK;
-  oz_plan(mix, p->nsm, INC_MAX_SPLIT);
-  mix->max_a = p->max_br;
+  oz_plan(mix, p->nsm, p->row_cap < p->T * p->S ? 1 : INC_MAX_SPLIT); /* parts of u lie side by side: no slabs */
   mix->max_b = p->max_n;
-  mix->C = p->u;
   mix->err = p->sums + SC_ERR;
   flows->M = p->G;
   flows->N = p->G;
-  flows->k_stages = depth_pad(TS) / OZ_BK;
+  flows->k_stages = p->dep_cap / OZ_BK;
   oz_plan(flows, p->nsm, INC_MAX_SPLIT);
   flows->max_a = p->max_bc;
   flows->max_b = p->max_gu;
   flows->C = p->C;
   flows->err = p->sums + SC_ERR;
+}
+
+/* The digits of beta's rows [r0, r0 + n), and of depths [k0, k0 + n) by columns. */
+void slice_beta_rows(lpg_incidence_plan* p, int r0, int n) {
+  const int G = p->G, kg = depth_pad(G);
+  k_oz_slice_rows<<<dim3(n, (kg / 2 + 255) / 256), 256, 0, p->st>>>(p->row_cap, G, kg, p->beta + (size_t)r0 * G,
+                                                                   p->max_br + r0, p->b_rows, p->sq_br + r0);
+}
+void slice_beta_cols(lpg_incidence_plan* p, int k0, int n) {
+  k_oz_slice_cols<<<dim3((p->G + 31) / 32, depth_pad(n) / 32), 256, 0, p->st>>>(
+      n, p->G, p->dep_cap, p->beta + (size_t)k0 * p->G, nullptr, p->max_bc, p->b_cols, p->sq_bc);
+}
+
+/* What every evaluation (its gradient) needs of beta beside that: the
+ * digits, where a plan keeps them, and the columns' maxima. */
+int plan_rows(lpg_incidence_plan* p) {
+  const int TS = p->T * p->S;
+  if (p->rows_ready) return LPG_OK;
+  PCK(cudaMemsetAsync(p->sq_br, 0, sizeof(uint32_t) * TS, p->st));
+  if (p->row_cap < TS) return LPG_OK;
+  slice_beta_rows(p, 0, TS);
+  p->rows_ready = true;
+  return plan_cuda(cudaGetLastError(), "slicing");
+}
+int plan_cols(lpg_incidence_plan* p) {
+  const int G = p->G, TS = p->T * p->S;
+  if (!p->bc_ready) {
+    PCK(cudaMemsetAsync(p->max_bc, 0, sizeof(unsigned long long) * G, p->st));
+    k_oz_col_max<<<oz_col_grid(TS, G), 256, 0, p->st>>>(TS, G, p->beta, nullptr, p->max_bc);
+    p->bc_ready = true;
+  }
+  if (p->cols_ready) return LPG_OK;
+  PCK(cudaMemsetAsync(p->sq_bc, 0, sizeof(uint32_t) * G, p->st));
+  if (p->dep_cap < TS) return LPG_OK;
+  slice_beta_cols(p, 0, TS);
+  p->cols_ready = true;
+  return plan_cuda(cudaGetLastError(), "slicing");
+}
+
+/* u = beta N: row_cap rows at a time. */
+int plan_mix(lpg_incidence_plan* p, const OzArgs& mix) {
+  const int G = p->G, TS = p->T * p->S;
+  const int rc = plan_rows(p);
+  if (rc != LPG_OK) return rc;
+  for (int r0 = 0; r0 < TS; r0 += p->row_cap) {
+    OzArgs A = mix;
+    A.M = std::min(p->row_cap, TS - r0);
+    A.tiles = (A.M + OZ_BM - 1) / OZ_BM * A.tiles_n;
+    A.max_a = p->max_br + r0;
+    A.C = p->u + (size_t)r0 * G;
+    if (!p->rows_ready) slice_beta_rows(p, r0, A.M);
+    PCK(oz_gemm(p->map_b, p->map_n, A, p->nsm, p->st));
+  }
+  PCK(oz_refine<false>(OzRefine{TS, G, G, mix.split, p->beta, p->Gm, p->fac, p->max_br, p->max_n, p->sq_br, p->sq_n,
+                                p->u, p->list_n, reinterpret_cast<uint64_t*>(p->gu_cols)},
+                       p->nsm, p->st));
+  return LPG_OK;
+}
+
+/* C = beta^T dL/du: dep_cap depths at a time, added up in C. */
+int plan_flows(lpg_incidence_plan* p, const OzArgs& flows) {
+  const int G = p->G, TS = p->T * p->S;
+  for (int k0 = 0; k0 < TS; k0 += p->dep_cap) {
+    const int K = std::min(p->dep_cap, TS - k0), kd = depth_pad(K);
+    OzArgs A = flows;
+    A.k_stages = kd / OZ_BK;
+    A.per_split = (A.k_stages + A.split - 1) / A.split;
+    A.add = k0 > 0;
+    k_oz_slice_cols<<<dim3((G + 31) / 32, kd / 32), 256, 0, p->st>>>(K, G, p->dep_cap, p->gu + (size_t)k0 * G, nullptr,
+                                                                     p->max_gu, p->gu_cols, p->sq_gu);
+    if (!p->cols_ready) slice_beta_cols(p, k0, K);
+    PCK(oz_gemm(p->map_bt, p->map_gu, A, p->nsm, p->st));
+  }
+  PCK(oz_refine<true>(OzRefine{G, G, TS, flows.split, p->beta, p->gu, nullptr, p->max_bc, p->max_gu, p->sq_bc, p->sq_gu,
+                               p->C, p->list_n + 1, reinterpret_cast<uint64_t*>(p->gu_cols)},
+                      p->nsm, p->st));
+  return LPG_OK;
 }
 
 /* x with 56 fraction bits, |x| < 64. */
@@ -649,10 +736,8 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   }
   mark(p, PH_MIX, p->small ? 1 : 3); /* with small sums part of the step's launch, counted here too */
   if (!p->small) {
-    PCK(oz_gemm(p->map_b, p->map_n, mix, p->nsm, p->st));
-    PCK(oz_refine<false>(OzRefine{TS, G, G, mix.split, p->beta, p->Gm, p->fac, p->max_br, p->max_n, p->sq_br, p->sq_n,
-                                  p->u, p->list_n, p->list},
-                         p->nsm, p->st));
+    const int rc = plan_mix(p, mix);
+    if (rc != LPG_OK) return rc;
   }
   mark(p, PH_FORWARD, 1);
   IncStep A{};
@@ -689,14 +774,11 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
         G, T, TS, nullptr, p->beta, p->gu, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
         p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
   } else {
-    const int kt = depth_pad(TS);
-    k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->gu, nullptr, p->max_gu, p->gu_cols,
-                                                                   p->sq_gu);
+    int rc = plan_cols(p);
+    if (rc != LPG_OK) return rc;
     mark(p, PH_FLOWS, 3);
-    PCK(oz_gemm(p->map_bt, p->map_gu, flows, p->nsm, p->st));
-    PCK(oz_refine<true>(OzRefine{G, G, TS, flows.split, p->beta, p->gu, nullptr, p->max_bc, p->max_gu, p->sq_bc, p->sq_gu,
-                                 p->C, p->list_n + 1, p->list},
-                        p->nsm, p->st));
+    rc = plan_flows(p, flows);
+    if (rc != LPG_OK) return rc;
     mark(p, PH_NETWORK_GRAD, 1);
     k_inc_network_grad<false><<<(G < 8 * p->nsm ? G : 8 * p->nsm) + 1, INC_THREADS, 0, p->st>>>(
         G, T, TS, p->C, nullptr, nullptr, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
@@ -808,16 +890,9 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
           p->tab, G, TG, p->pops, d_dist, p->logp, p->logd, p->lp2, p->ld2, p->popc, p->popc, p->target);
       const int TS = T * S;
       if (!p->small) {
-        const int kg = depth_pad(G), kt = depth_pad(TS);
-        rc = plan_cuda(cudaMemsetAsync(p->max_bc, 0, sizeof(unsigned long long) * G, p->st), "clear maxima");
-        if (rc == LPG_OK) rc = plan_cuda(cudaMemsetAsync(p->sq_bc, 0, sizeof(uint32_t) * G, p->st), "clear sums");
-        if (rc == LPG_OK) rc = plan_cuda(cudaMemsetAsync(p->sq_br, 0, sizeof(uint32_t) * TS, p->st), "clear sums");
         k_oz_row_max<<<(TS + 7) / 8, 256, 0, p->st>>>(TS, G, p->beta, p->max_br);
-        k_oz_slice_rows<<<dim3(TS, (kg / 2 + 255) / 256), 256, 0, p->st>>>(TS, G, kg, p->beta, p->max_br, p->b_rows,
-                                                                              p->sq_br);
-        k_oz_col_max<<<oz_col_grid(TS, G), 256, 0, p->st>>>(TS, G, p->beta, nullptr, p->max_bc);
-        k_oz_slice_cols<<<dim3((G + 31) / 32, kt / 32), 256, 0, p->st>>>(TS, G, kt, p->beta, nullptr, p->max_bc,
-                                                                        p->b_cols, p->sq_bc);
+        rc = plan_rows(p);
+        if (rc == LPG_OK && target) rc = plan_cols(p); /* a target is given for its gradient */
       }
       if (rc == LPG_OK) rc = plan_cuda(cudaGetLastError(), "log launch");
     }

@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(256)
   atomicMax(&max[c], m);
 }
 
-/* dst [8][R][Kp] from src [R][K], scaled by rows; two depths a thread.  The
- * scaled rows' sums of squares are added to sq. */
+/* dst [8][R][Kp] from src [gridDim.x][K], scaled by rows; two depths a
+ * thread.  The scaled rows' sums of squares are added to sq. */
 __global__ void __launch_bounds__(256)
     k_oz_slice_rows(int R, int K, int Kp, const double* __restrict__ src, const unsigned long long* __restrict__ max,
                     uint32_t* __restrict__ dst, uint32_t* __restrict__ sq) {
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256)
     dst[((size_t)s * R + r) * (Kp / 2) + k / 2] = (uint32_t)a[s] | (uint32_t)b[s] << 16;
 }
 
-/* dst [8][C][Kp] from src [K][C] (times fac[k], when given), scaled by columns: 32 x 32 tiles turned in
+/* The first 32 gridDim.y depths of dst [8][C][Kp] from src [K][C] (times fac[k], when given), scaled by columns: 32 x 32 tiles turned in
  * shared memory, then two depths a thread, so that sixteen threads write one
  * 64-byte run.  The scaled columns' sums of squares are added to sq.  Bound by
  * the integer digit extraction and the writes. */
@@ -304,6 +304,7 @@ struct OzArgs {
   int M, N, k_stages;     /* depth in stages of OZ_BK */
   int split, per_split;   /* depth slices, stages a slice */
   int tiles_n, tiles;
+  int add;                /* to what C holds */
   const unsigned long long *max_a, *max_b;
   double* C; /* [split][M][N] */
   double* err;
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
               const int eb = col + c + q < G.N ? oz_exp(G.max_b[col + c + q]) : 0;
               w[q] = ea == OZ_NAN_EXP || eb == OZ_NAN_EXP ? __longlong_as_double(0x7ff8000000000000LL)
                                                           : oz_double(hi[c + q], lo[c + q], ea + eb);
-              if (kc != k0 && col + c + q < G.N) w[q] += out[c + q];
+              if ((kc != k0 || G.add) && col + c + q < G.N) w[q] += out[c + q];
             }
             if (col + c + 1 < G.N && even) {
               *reinterpret_cast<double2*>(out + c) = make_double2(w[0], w[1]);
