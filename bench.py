@@ -1104,7 +1104,9 @@ def incidence_arm(args):
         "e2e": {"value": K / (t_setup + t_eval), "unit": "evaluations/s", "setup_ms": t_setup * 1e3,
                 "ms_per_eval": t_eval / K * 1e3, "h2d_bytes_per_step": h2d_setup / K + 8 * G,
                 "d2h_bytes_per_step": 8 * (8 + G)},
-        "gpu_launches": 8 * K,  # per evaluation: network, column maxima, slicing, mix, step, slicing, flows, network_grad
+        # per evaluation: network, column maxima, slicing, mix and its two refining kernels, step, slicing, flows and
+        # their two, network_grad; with the small sums network, step, network_grad
+        "gpu_launches": (3 if G <= 128 and T * S * G * G <= 4_000_000 else 12) * K,
         "kernels": kernels,
         "roofline": roof,
         "cpu_baseline": cpu,

@@ -510,8 +510,10 @@ int lpg_incidence_plan_create(const lpg_incidence_in* in, const double* target, 
 int lpg_incidence_plan_eval(lpg_incidence_plan* p, const lpg_incidence_params* prm, const double* g_lam,
                             double* lam_out, double* loss_out, lpg_incidence_grad* grad);
 void* lpg_incidence_plan_stream(lpg_incidence_plan* p);
-/* Per-kernel device time (CUDA events on the plan's stream) of the
- * evaluations made while profiling is on; enabling resets the sums. */
+/* Device time (CUDA events on the plan's stream) of each phase of the
+ * evaluations made while profiling is on; enabling resets the sums.
+ * `launches` counts evaluations that had the phase, not kernels: a phase is
+ * several launches at large sizes and part of another's at small ones. */
 int lpg_incidence_plan_set_profiling(lpg_incidence_plan* p, int32_t enable);
 int lpg_incidence_plan_read_profile(lpg_incidence_plan* p, lpg_profile* out);
 void lpg_incidence_plan_destroy(lpg_incidence_plan* p);

@@ -497,7 +497,7 @@ struct lpg_incidence_plan {
   bool prof = false;
   cudaEvent_t ev[PH_COUNT + 1] = {};
   double ms[PH_COUNT] = {};
-  int64_t launches[PH_COUNT] = {};
+  int64_t evals[PH_COUNT] = {};
 };
 
 namespace {
@@ -590,10 +590,12 @@ int plan_alloc(lpg_incidence_plan* p) {
   return LPG_OK;
 }
 
-/* Marks the start of phase ph (and the end of the previous one). */
-inline void mark(lpg_incidence_plan* p, int ph, int n_launch) {
+/* Marks the start of phase ph of an evaluation (and the end of the previous
+ * one).  A phase may be several launches, or with the small sums part of
+ * another phase's. */
+inline void mark(lpg_incidence_plan* p, int ph) {
   if (p->prof) cudaEventRecord(p->ev[ph], p->st);
-  p->launches[ph] += n_launch;
+  p->evals[ph] += 1;
 }
 
 void plan_products(const lpg_incidence_plan* p, OzArgs* mix, OzArgs* flows) {
@@ -720,7 +722,7 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   }
   OzArgs mix{}, flows{};
   plan_products(p, &mix, &flows);
-  mark(p, PH_NETWORK, p->small ? 1 : 3);
+  mark(p, PH_NETWORK);
   const int nblk = G + (T + 31) / 32;
   if (p->small) {
     k_inc_network<true><<<nblk, INC_THREADS, 0, p->st>>>(G, T, p->tab, p->pops, p->logp, p->logd, p->lp2, p->ld2, V,
@@ -734,12 +736,12 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
     k_oz_slice_cols<<<dim3((G + 31) / 32, depth_pad(G) / 32), 256, 0, p->st>>>(G, G, depth_pad(G), p->Gm, p->fac,
                                                                               p->max_n, p->n_cols, p->sq_n);
   }
-  mark(p, PH_MIX, p->small ? 1 : 3); /* with small sums part of the step's launch, counted here too */
+  mark(p, PH_MIX);
   if (!p->small) {
     const int rc = plan_mix(p, mix);
     if (rc != LPG_OK) return rc;
   }
-  mark(p, PH_FORWARD, 1);
+  mark(p, PH_FORWARD);
   IncStep A{};
   A.T = T;
   A.G = G;
@@ -764,11 +766,11 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   A.grad = grad;
   const int rc = p->small ? launch_step<true>(p, A) : launch_step<false>(p, A);
   if (rc != LPG_OK || !grad) return rc;
-  mark(p, PH_BACKWARD, 1); /* its cells are part of the step's launch, counted here too; then the slicing */
+  mark(p, PH_BACKWARD); /* its cells are part of the step's launch; here the slicing */
   double* gN = want_network ? p->gN : nullptr;
   if (p->small) {
-    mark(p, PH_FLOWS, 1); /* part of the next launch */
-    mark(p, PH_NETWORK_GRAD, 1);
+    mark(p, PH_FLOWS);
+    mark(p, PH_NETWORK_GRAD);
     const int smem = (int)sizeof(double) * (G > INC_THREADS ? G : INC_THREADS);
     k_inc_network_grad<true><<<G + 1, INC_THREADS, smem, p->st>>>(
         G, T, TS, nullptr, p->beta, p->gu, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
@@ -776,10 +778,10 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   } else {
     int rc = plan_cols(p);
     if (rc != LPG_OK) return rc;
-    mark(p, PH_FLOWS, 3);
+    mark(p, PH_FLOWS);
     rc = plan_flows(p, flows);
     if (rc != LPG_OK) return rc;
-    mark(p, PH_NETWORK_GRAD, 1);
+    mark(p, PH_NETWORK_GRAD);
     k_inc_network_grad<false><<<(G < 8 * p->nsm ? G : 8 * p->nsm) + 1, INC_THREADS, 0, p->st>>>(
         G, T, TS, p->C, nullptr, nullptr, p->Gm, p->rs, p->fac, p->logp, p->logd, prm->k, p->logP, gN,
         p->sums + SC_THETA, p->seas, p->gw, sc.R, p->sums + SC_R);
@@ -963,7 +965,7 @@ extern "C" int lpg_incidence_plan_set_profiling(lpg_incidence_plan* p, int32_t e
   p->prof = enable != 0;
   for (int ph = 0; ph < PH_COUNT; ++ph) {
     p->ms[ph] = 0.0;
-    p->launches[ph] = 0;
+    p->evals[ph] = 0;
   }
   return LPG_OK;
 }
@@ -975,7 +977,7 @@ extern "C" int lpg_incidence_plan_read_profile(lpg_incidence_plan* p, lpg_profil
   for (int ph = 0; ph < PH_COUNT; ++ph) {
     out->names[ph] = kPhaseNames[ph];
     out->total_ms[ph] = p->ms[ph];
-    out->launches[ph] = p->launches[ph];
+    out->launches[ph] = p->evals[ph];
   }
   return LPG_OK;
 }

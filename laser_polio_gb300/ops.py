@@ -227,7 +227,7 @@ class IncidencePlan:
         self._lib.lpg_incidence_plan_set_profiling(self._h, int(enable))
 
     def profile(self) -> dict:
-        """{kernel: (total ms, launches)} of the evaluations since profiling was enabled."""
+        """{phase: (total ms, evaluations that had it)} since profiling was enabled."""
         pr = _abi.lpg_profile()
         rc = self._lib.lpg_incidence_plan_read_profile(self._h, C.byref(pr))
         if rc != 0:
