@@ -442,7 +442,10 @@ int lpg_count_seirp(const int16_t* node_id, const int8_t* disease_state, const i
 
 /* The same operation under the name of its form without device allocation
  * (lpg_count_seirp allocates nothing either).  No counterpart in the
- * reference, whose count_SEIRP allocates numpy tables on every call. */
+ * reference, whose count_SEIRP allocates numpy tables on every call.
+ * LPG_COUNT_SEIRP_STATIC_WORDS is the int32 words of the scratch that this
+ * form once had; no call needs it now, and callers that name it still build. */
+#define LPG_COUNT_SEIRP_STATIC_WORDS (1 << 20)
 int lpg_count_seirp_static(const int16_t* node_id, const int8_t* disease_state, const int8_t* strain,
                            const int8_t* potentially_paralyzed, const int8_t* paralyzed, int32_t n_nodes,
                            int32_t n_strains, int64_t n_people, int32_t* S, int32_t* E, int32_t* I, int32_t* R,
