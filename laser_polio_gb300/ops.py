@@ -59,9 +59,9 @@ def count_SEIRP(node_id, disease_state, strain, potentially_paralyzed, paralyzed
     device = cols[1].device
     with torch.cuda.device(device):
         G, ns = int(n_nodes), int(n_strains)
-        # one allocation for the eight results: the host side is most of a small call
-        S, E, I, R, potp, par, ebs, ibs = torch.empty(G * (6 + 2 * ns), dtype=torch.int32, device=device).split(
-            [G] * 6 + [G * ns] * 2)
+        # eight tensors of their own: a caller may keep or save one without the others
+        S, E, I, R, potp, par = [torch.empty(G, dtype=torch.int32, device=device) for _ in range(6)]
+        ebs, ibs = [torch.empty((G, ns), dtype=torch.int32, device=device) for _ in range(2)]
         bad = torch.empty(1, dtype=torch.int64, device=device) if n_invalid is not None else None
         lib = _lib.load()
         stream = torch.cuda.current_stream(device).cuda_stream
@@ -74,7 +74,7 @@ def count_SEIRP(node_id, disease_state, strain, potentially_paralyzed, paralyzed
             if rc == -1:
                 raise ValueError(msg)
             raise _lib.LpgError(rc, msg)
-    res = (S, E, I, R, ebs.view(G, ns), ibs.view(G, ns), potp, par)
+    res = (S, E, I, R, ebs, ibs, potp, par)
     if n_invalid is not None:
         n_invalid.append(int(bad.item()))
     if host:
