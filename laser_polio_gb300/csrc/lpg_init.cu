@@ -333,7 +333,9 @@ __global__ void __launch_bounds__(kThreads) k_rsel_mark(const uint32_t* __restri
  * allocation with its free costs 0.2 ms (the stream-ordered pool, which gives
  * its memory back at every synchronisation, the same).  4 MB at most a thread
  * and device, freed when the thread ends.  A call has its stream finish
- * before it returns, so the next one may use any stream. */
+ * before it returns, so the next one may use any stream.  All memory is
+ * allocated and freed in stream order: cudaFree would wait for every stream's
+ * kernels, of which a program may have a whole run queued. */
 constexpr size_t kWorkBytes = 4 << 20, kTableBytes = 1 << 18;
 struct Workspace {
   int device;
@@ -343,15 +345,19 @@ struct Workspace {
 struct Workspaces {
   std::vector<Workspace> all;
   ~Workspaces() {
-    for (auto& w : all) cudaFree(w.dev);
+    int device = 0;
+    const bool known = cudaGetDevice(&device) == cudaSuccess;
+    for (auto& w : all)
+      if (cudaSetDevice(w.device) == cudaSuccess) cudaFreeAsync(w.dev, nullptr);
+    if (known) cudaSetDevice(device);
   }
-  Workspace* get() {
+  Workspace* get(cudaStream_t st) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
     for (auto& w : all)
       if (w.device == device) return &w;
     Workspace w{device, nullptr, std::vector<uint8_t>(kTableBytes)};
-    if (cudaMalloc((void**)&w.dev, kWorkBytes) != cudaSuccess) {
+    if (cudaMallocAsync((void**)&w.dev, kWorkBytes, st) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
@@ -369,10 +375,10 @@ struct Scratch {
   std::vector<void*> ptrs;
   Workspace* w;
   size_t used = 0, sent = 0, taken = kTableBytes;
-  explicit Scratch(cudaStream_t s) : st(s), w(t_workspaces.get()) {}
+  explicit Scratch(cudaStream_t s) : st(s), w(t_workspaces.get(s)) {}
   ~Scratch() {
+    for (void* p : ptrs) cudaFreeAsync(p, st);
     cudaStreamSynchronize(st);
-    for (void* p : ptrs) cudaFree(p);
   }
   template <class T>
   int alloc(T** out, size_t n) {
@@ -382,7 +388,7 @@ struct Scratch {
       taken += room;
       return 0;
     }
-    if (cudaMalloc((void**)out, bytes) != cudaSuccess) {
+    if (cudaMallocAsync((void**)out, bytes, st) != cudaSuccess) {
       cudaGetLastError();
       return lpg_ops_fail(LPG_ERR_NOMEM, "init: device scratch of %zu bytes", bytes);
     }
