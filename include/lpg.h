@@ -521,6 +521,14 @@ int lpg_incidence_plan_set_profiling(lpg_incidence_plan* p, int32_t enable);
 int lpg_incidence_plan_read_profile(lpg_incidence_plan* p, lpg_profile* out);
 void lpg_incidence_plan_destroy(lpg_incidence_plan* p);
 
+/* Test hook of lpg_test_stall_sweep's kind for the plan's tensor-core
+ * products (plans large enough to have them): each CTA issues at most
+ * `stages` loads (negative: all) and its waits give up after `wait_polls`
+ * polls (0: the normal limit).  The evaluation then returns LPG_ERR_TIMEOUT;
+ * the kernel has waited for the loads and products that it did issue, and
+ * the plan stays usable.  No counterpart in the reference. */
+int lpg_test_stall_products(lpg_incidence_plan* p, int32_t stages, int64_t wait_polls);
+
 /* One-shot: a plan on `stream`, one evaluation at in's parameters, freed.
  * lam_out [T][G] (host) receives lam.  With g_lam non-NULL ([T][G], host:
  * dL/dlam), *grad receives the gradients of L = sum g_lam * lam.

@@ -65,6 +65,7 @@ SIGNATURES = {
     "lpg_init_mean_infectivity": (C.c_double, [C.c_uint64, C.c_double, _abi.lpg_dist]),
     "lpg_test_stall_sweep": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64]),
     "lpg_test_stall_round0": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64]),
+    "lpg_test_stall_products": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64]),
     "lpg_set_launch": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
     "lpg_get_launch": (C.c_int, [C.c_void_p, C.c_int32]),
 }

@@ -487,6 +487,7 @@ struct lpg_incidence_plan {
    * mixing is done with the one before the flows write the other), gu_cols and the list theirs. */
   int row_cap = 0, dep_cap = 0;
   bool rows_ready = false, cols_ready = false, bc_ready = false;
+  int polls = OZ_WAIT_POLLS, stall = -1; /* lpg_test_stall_products */
   uint32_t *b_rows = nullptr, *b_cols = nullptr, *n_cols = nullptr, *gu_cols = nullptr;
   unsigned long long *max_br = nullptr, *max_bc = nullptr;
   uint32_t *sq_br = nullptr, *sq_bc = nullptr;
@@ -605,6 +606,8 @@ void plan_products(const lpg_incidence_plan* p, OzArgs* mix, OzArgs* flows) {
   oz_plan(mix, p->nsm, p->row_cap < p->T * p->S ? 1 : INC_MAX_SPLIT); /* parts of u lie side by side: no slabs */
   mix->max_b = p->max_n;
   mix->err = p->sums + SC_ERR;
+  mix->polls = flows->polls = p->polls;
+  mix->stall = flows->stall = p->stall;
   flows->M = p->G;
   flows->N = p->G;
   flows->k_stages = p->dep_cap / OZ_BK;
@@ -959,6 +962,15 @@ extern "C" int lpg_incidence_plan_eval(lpg_incidence_plan* p, const lpg_incidenc
 }
 
 extern "C" void* lpg_incidence_plan_stream(lpg_incidence_plan* p) { return p ? (void*)p->st : nullptr; }
+
+extern "C" int lpg_test_stall_products(lpg_incidence_plan* p, int32_t stages, int64_t wait_polls) {
+  if (!p) return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: null argument");
+  if (wait_polls < 0 || wait_polls > OZ_WAIT_POLLS)
+    return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: wait_polls %lld out of range", (long long)wait_polls);
+  p->stall = stages < 0 ? -1 : stages;
+  p->polls = wait_polls > 0 ? (int)wait_polls : OZ_WAIT_POLLS;
+  return LPG_OK;
+}
 
 extern "C" int lpg_incidence_plan_set_profiling(lpg_incidence_plan* p, int32_t enable) {
   if (!p) return lpg_ops_fail(LPG_ERR_ARG, "incidence plan: null argument");

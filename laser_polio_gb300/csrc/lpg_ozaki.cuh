@@ -49,7 +49,7 @@
 #define OZ_B_BYTES (OZ_SLICES * OZ_BN * OZ_BK * 2)
 #define OZ_STAGE_BYTES (OZ_A_BYTES + OZ_B_BYTES)
 #define OZ_SMEM (OZ_STAGES * OZ_STAGE_BYTES + 1024)
-#define OZ_WAIT_NS 1000000000ULL /* a wait gives up after a second */
+#define OZ_WAIT_POLLS (1 << 24) /* a wait gives up after so many polls, about 2.2 s (0.13 us each, measured) */
 #define OZ_NAN_EXP 0x7fffffff
 
 /* --- slicing --------------------------------------------------------------- */
@@ -203,9 +203,10 @@ __global__ void __launch_bounds__(256)
 
 /* --- the product ------------------------------------------------------------ */
 __device__ __forceinline__ uint32_t oz_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool oz_wait(uint64_t* bar, uint32_t parity, const volatile int* fail) {
-  uint64_t t0 = 0;
-  for (;;) {
+/* Counted in polls, not in time: those do not go on while the context is
+ * switched out or held by a debugger. */
+__device__ __forceinline__ bool oz_wait(uint64_t* bar, uint32_t parity, const volatile int* fail, int polls) {
+  for (int it = 0; it < polls; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -213,11 +214,9 @@ __device__ __forceinline__ bool oz_wait(uint64_t* bar, uint32_t parity, const vo
         : "r"(oz_smem(bar)), "r"(parity)
         : "memory");
     if (ok) return true;
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    if (t0 == 0) t0 = t;
-    else if (t - t0 > OZ_WAIT_NS || *fail) return false;
+    if (fail && *fail) return false;
   }
+  return false;
 }
 
 __device__ __forceinline__ void oz_load(uint32_t dst, const CUtensorMap* map, int k, int row, uint64_t* bar) {
@@ -305,6 +304,7 @@ struct OzArgs {
   int split, per_split;   /* depth slices, stages a slice */
   int tiles_n, tiles;
   int add;                /* to what C holds */
+  int polls, stall;       /* a wait's limit; the load after which no more are issued (a test's; negative: none) */
   const unsigned long long *max_a, *max_b;
   double* C; /* [split][M][N] */
   double* err;
@@ -315,12 +315,12 @@ struct OzArgs {
  * loads ahead, a product warp issues each stage's digit products (the queue
  * of issued products is short, so a thread that did both would load late),
  * and sixteen warps drain the accumulators.  Every wait is bounded and gives
- * up once another has: then *err is set, the loads in flight are waited for
- * (bounded) and the CTA gives its TMEM back and leaves. */
+ * up once another has: then *err is set, the products and loads in flight are
+ * waited for (bounded) and the CTA gives its TMEM back and leaves. */
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, OzArgs G) {
   extern __shared__ uint8_t oz_raw[];
-  __shared__ uint64_t full[OZ_STAGES], empty[OZ_STAGES], done, drained;
+  __shared__ uint64_t full[OZ_STAGES], empty[OZ_STAGES], done, drained, quiet;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_fail;
   const uint32_t base = (oz_smem(oz_raw) + 1023u) & ~1023u;
@@ -331,6 +331,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(oz_smem(&empty[s])) : "memory");
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(oz_smem(&done)) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(oz_smem(&quiet)) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(oz_smem(&drained)), "r"(OZ_DRAIN_WARPS) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_fail = 0;
@@ -346,17 +347,21 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
   const int units = G.tiles * G.split;
+  int loads = 0; /* issued, by the load warp's first lane */
 
   if (warp == OZ_DRAIN_WARPS) { /* loads */
     if (lane == 0) {
-      int n = 0;
       bool ok = true;
       for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
         const int z = unit / G.tiles, tile = unit % G.tiles;
         const int k0 = z * G.per_split, k1 = min(G.k_stages, k0 + G.per_split);
-        for (int k = k0; k < k1; ++k, ++n) {
-          const int s = n % OZ_STAGES;
-          if (n >= OZ_STAGES && !oz_wait(&empty[s], (uint32_t)(n / OZ_STAGES - 1) & 1u, &s_fail)) {
+        for (int k = k0; k < k1; ++k, ++loads) {
+          const int s = loads % OZ_STAGES;
+          if (loads == G.stall) {
+            ok = false;
+            break;
+          }
+          if (loads >= OZ_STAGES && !oz_wait(&empty[s], (uint32_t)(loads / OZ_STAGES - 1) & 1u, &s_fail, G.polls)) {
             s_fail = 1;
             ok = false;
             break;
@@ -369,12 +374,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           oz_load(dst + OZ_A_BYTES, &tb, k * OZ_BK, (tile % G.tiles_n) * OZ_BN, &full[s]);
         }
       }
-      /* nothing may land after the CTA has left (in a good run the products have waited for every load) */
-      if (!ok) {
-        const int never = 0;
-        for (int q = n > OZ_STAGES ? n - OZ_STAGES : 0; q < n; ++q)
-          oz_wait(&full[q % OZ_STAGES], (uint32_t)(q / OZ_STAGES) & 1u, &never);
-      }
     }
   } else if (warp == OZ_DRAIN_WARPS + 1) { /* products */
     if (lane == 0) {
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int z = unit / G.tiles;
         const int k0 = z * G.per_split, k1 = min(G.k_stages, k0 + G.per_split);
         for (int kc = k0; ok && kc < k1; kc += OZ_CHUNK, ++drains) {
-          if (drains > 0 && !oz_wait(&drained, (uint32_t)(drains - 1) & 1u, &s_fail)) {
+          if (drains > 0 && !oz_wait(&drained, (uint32_t)(drains - 1) & 1u, &s_fail, G.polls)) {
             ok = false;
             break;
           }
@@ -392,7 +391,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           const int ke = min(k1, kc + OZ_CHUNK);
           for (int k = kc; k < ke; ++k, ++n) {
             const int s = n % OZ_STAGES;
-            if (!oz_wait(&full[s], (uint32_t)(n / OZ_STAGES) & 1u, &s_fail)) {
+            if (!oz_wait(&full[s], (uint32_t)(n / OZ_STAGES) & 1u, &s_fail, G.polls)) {
               ok = false;
               break;
             }
@@ -435,7 +434,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const int col0 = (tile % G.tiles_n) * OZ_BN + (warp >> 2) * 16;
       double* Cz = G.C + (size_t)z * G.M * G.N;
       for (int kc = k0; ok && kc < k1; kc += OZ_CHUNK, ++drains) {
-        ok = oz_wait(&done, (uint32_t)drains & 1u, &s_fail);
+        ok = oz_wait(&done, (uint32_t)drains & 1u, &s_fail, G.polls);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
           s_fail = 1;
@@ -493,7 +492,17 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid == 0 && s_fail) *G.err = 1.0;
+  if (s_fail) { /* in a good run the drains have waited for every product, and the products for every load */
+    if (tid == 0) *G.err = 1.0;
+    if (warp == OZ_DRAIN_WARPS && lane == 0)
+      for (int q = loads > OZ_STAGES ? loads - OZ_STAGES : 0; q < loads; ++q)
+        oz_wait(&full[q % OZ_STAGES], (uint32_t)(q / OZ_STAGES) & 1u, nullptr, OZ_WAIT_POLLS);
+    if (warp == OZ_DRAIN_WARPS + 1 && lane == 0) { /* the thread that issued the products */
+      oz_commit(&quiet);
+      oz_wait(&quiet, 0, nullptr, OZ_WAIT_POLLS);
+    }
+    __syncthreads();
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
@@ -800,6 +809,7 @@ inline void oz_plan(OzArgs* G, int nsm, int max_split) {
 }
 
 inline cudaError_t oz_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const OzArgs& G, int nsm, cudaStream_t st) {
+  if (G.polls <= 0) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
   if (e != cudaSuccess) return e;
   const int units = G.tiles * G.split;

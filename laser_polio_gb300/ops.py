@@ -234,6 +234,13 @@ class IncidencePlan:
             _raise(self._lib, rc)
         return {pr.names[i].decode(): (pr.total_ms[i], pr.launches[i]) for i in range(pr.n_kernels)}
 
+    def test_stall_products(self, stages: int, wait_polls: int = 0):
+        """Test hook (lpg_test_stall_products): the products' CTAs issue at
+        most `stages` loads and give up a wait after `wait_polls` polls."""
+        rc = self._lib.lpg_test_stall_products(self._h, int(stages), int(wait_polls))
+        if rc != 0:
+            _raise(self._lib, rc)
+
     def close(self):
         if getattr(self, "_h", None):
             self._lib.lpg_incidence_plan_destroy(self._h)
