@@ -878,7 +878,6 @@ extern "C" int lpg_start(lpg_handle* h) {
   carve.add(&W.bb, (size_t)LPG_MAX_STRAINS * G);
   carve.add(&W.nb_end, G);
   carve.add(&W.nb_li0, G);
-  carve.add(&W.prob, (size_t)LPG_MAX_STRAINS * G);
   carve.add(&W.inck, (size_t)LPG_MAX_STRAINS * G);
   carve.add(&W.size, G);
   carve.add(&W.uniq, G);

@@ -2051,7 +2051,6 @@ __global__ void __launch_bounds__(32 * LPG_NODE_TX_WARPS) k_node_tx(DevWorld W, 
         const double rate = beta / denom;
         pk = -lpg_expm1(-rate);
         if (!(pk > 0.0)) pk = 0.0;
-        W.prob[(int64_t)wid * G + g] = pk;
       }
       s_p[wid][lane] = pk;
     } else if (local_zero && rp->zi < 1.0 && rp->nb_r >= 1) {
