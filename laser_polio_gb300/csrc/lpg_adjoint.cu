@@ -769,7 +769,7 @@ int plan_run(lpg_incidence_plan* p, const lpg_incidence_params* prm, IncScalars 
   A.grad = grad;
   const int rc = p->small ? launch_step<true>(p, A) : launch_step<false>(p, A);
   if (rc != LPG_OK || !grad) return rc;
-  mark(p, PH_BACKWARD); /* its cells are part of the step's launch; here the slicing */
+  mark(p, PH_BACKWARD); /* its cells are part of the step's launch */
   double* gN = want_network ? p->gN : nullptr;
   if (p->small) {
     mark(p, PH_FLOWS);

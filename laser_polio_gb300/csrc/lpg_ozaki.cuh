@@ -571,23 +571,27 @@ struct OzRefine {
 
 #define OZ_R_THREADS 128
 #define OZ_R_BM 32
-#define OZ_R_BN 64
+#define OZ_R_BN 32
 #define OZ_R_BK 32
-#define OZ_R_LIST 128 /* elements of a tile formed one by one */
+#define OZ_R_LIST 64 /* elements of a tile formed one by one */
 
 /* Adds the depth slices into the first one, and finds the elements that
- * oz_small names, a 32 x 64 tile a CTA.  Up to OZ_R_LIST of them go to the list (k_oz_fix); where there are more, they are
- * formed here by a product of FP32 pairs over the whole tile (2048 elements
- * of 774 terms: 75 us an SM in pairs, about 0.4 us an element in FP64, so the
- * line lies near 128).  Bound by reading C where nothing is small; with
- * k_oz_fix 17 and 18 us for the two products of 774 nodes, 365 ticks and 3
- * strains (0.1% of the mixing's elements are small), 54 and 44 us of 4000
- * nodes and 90 ticks. */
+ * oz_small names, a 32 x 32 tile a CTA.  Up to OZ_R_LIST of them go to the
+ * list (k_oz_fix); where there are more, they are formed here by a product of
+ * FP32 pairs over the tile's rows that have some, and over the depths at
+ * which those rows have terms (a row of few infected nodes has few).  Bound
+ * by reading C where nothing is small; by FP32 issue where all is: 774 nodes,
+ * 365 ticks, 3 strains, waves that hardly overlap: 547 us for the flows (a
+ * 32 x 64 tile: 677).  With k_oz_fix 16 and 17 us for the two products of
+ * that size where 0.1% of the mixing's elements are small, 49 and 47 us of
+ * 4000 nodes and 90 ticks; 133 us for the mixing of a recorded run's
+ * aggregates, 5% of whose elements are small.  The list's line: a tile of 774
+ * terms in pairs takes an SM about 20 us, an element in FP64 0.4 us. */
 template <bool TRANS_A>
 __global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
   __shared__ int s_ea[OZ_R_BM], s_eb[OZ_R_BN], s_count, s_need;
   __shared__ unsigned long long s_at;
-  __shared__ uint32_t s_sa[OZ_R_BM], s_sb[OZ_R_BN];
+  __shared__ uint32_t s_sa[OZ_R_BM], s_sb[OZ_R_BN], s_rows, s_some;
   __shared__ uint16_t s_list[OZ_R_LIST];
   const int tid = threadIdx.x, m0 = blockIdx.y * OZ_R_BM, n0 = blockIdx.x * OZ_R_BN;
   if (tid < OZ_R_BN) {
@@ -600,10 +604,10 @@ __global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
     s_ea[r] = in ? oz_exp(R.max_a[m0 + r]) : 0;
     s_sa[r] = in ? R.sq_a[m0 + r] : 0;
   }
-  if (tid == 0) s_count = 0;
+  if (tid == 0) s_count = s_rows = 0;
   __syncthreads();
   if (tid < 32) {
-    const uint32_t top = max(max(s_sa[tid], s_sb[tid]), s_sb[tid + 32]);
+    const uint32_t top = max(s_sa[tid], s_sb[tid]);
     const uint32_t most = __reduce_max_sync(0xffffffffu, top);
     /* the biased exponent that an element scaled by 2^(ea + eb) needs at most */
     if (tid == 0) s_need = (int)(__float_as_uint(OZ_KEEP * oz_norm(most, most)) >> 23) - 127 + 1023 + 1;
@@ -642,6 +646,7 @@ __global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
       if ((__double2hiint(v[i]) >> 20 & 0x7ff) - s_ea[r] >= need || m0 + r >= R.M) continue;
       if (!oz_small(v[i], s_ea[r], s_eb[c], s_sa[r], s_sb[c])) continue;
       const int at = atomicAdd(&s_count, 1);
+      atomicOr(&s_rows, 1u << r);
       if (at < OZ_R_LIST) s_list[at] = (uint16_t)(r * OZ_R_BN + c);
     }
   }
@@ -657,13 +662,17 @@ __global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
   __shared__ float2 sA[OZ_R_BK][OZ_R_BM + 1]; /* [k][m] */
   __shared__ float2 sB[OZ_R_BK][OZ_R_BN];     /* [k][n] */
   const int tx = tid & 15, ty = tid >> 4;
-  float sh[4][4], sl[4][4];
+  float sh[4][2], sl[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sh[i][j] = sl[i][j] = 0.f;
+    for (int j = 0; j < 2; ++j) sh[i][j] = sl[i][j] = 0.f;
+  const uint32_t rows = s_rows; /* the others' elements stay */
 #pragma unroll 1
   for (int k0 = 0; k0 < R.K; k0 += OZ_R_BK) {
+    __syncthreads();
+    if (tid == 0) s_some = 0;
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < (OZ_R_BK * OZ_R_BM) / OZ_R_THREADS; ++q) {
       const int e = tid + q * OZ_R_THREADS;
@@ -671,100 +680,141 @@ __global__ void __launch_bounds__(OZ_R_THREADS) k_oz_refine(OzRefine R) {
       /* consecutive threads read consecutive m, or consecutive k */
       const int k = TRANS_A ? hi : lo, m = TRANS_A ? lo : hi;
       float2 v = make_float2(0.f, 0.f);
-      if (k0 + k < R.K && m0 + m < R.M)
+      if (k0 + k < R.K && (rows >> m & 1u))
         v = oz_pair(R.A[TRANS_A ? (size_t)(k0 + k) * R.M + m0 + m : (size_t)(m0 + m) * R.K + k0 + k], s_ea[m]);
       sA[k][m] = v;
+      const uint32_t some = __ballot_sync(0xffffffffu, v.x != 0.0f);
+      if (lo == 0 && some) atomicOr(&s_some, TRANS_A ? 1u << k : some);
     }
+    __syncthreads();
+    const uint32_t some = s_some; /* the depths at which some row has a term: few where few nodes are infected */
+    if (some == 0) continue;
 #pragma unroll
     for (int q = 0; q < (OZ_R_BK * OZ_R_BN) / OZ_R_THREADS; ++q) {
       const int e = tid + q * OZ_R_THREADS;
-      const int k = e >> 6, n = e & 63;
+      const int k = e >> 5, n = e & 31;
       float2 v = make_float2(0.f, 0.f);
-      if (k0 + k < R.K && n0 + n < R.N)
+      if ((some >> k & 1u) && n0 + n < R.N)
         v = oz_pair(oz_scaled(R.B[(size_t)(k0 + k) * R.N + n0 + n], R.fac, k0 + k), s_eb[n]);
       sB[k][n] = v;
     }
     __syncthreads();
-#pragma unroll 4
-    for (int q = 0; q < OZ_R_BK; ++q) {
-      float2 av[4], bv[4];
+    auto add = [&](int q) {
+      float2 av[4], bv[2];
 #pragma unroll
       for (int i = 0; i < 4; ++i) av[i] = sA[q][ty + 8 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = sB[q][tx + 16 * j];
+      for (int j = 0; j < 2; ++j) bv[j] = sB[q][tx + 16 * j];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) oz_pair_fma(sh[i][j], sl[i][j], av[i], bv[j]);
+        for (int j = 0; j < 2; ++j) oz_pair_fma(sh[i][j], sl[i][j], av[i], bv[j]);
+    };
+    if (some == 0xffffffffu) {
+#pragma unroll 4
+      for (int q = 0; q < OZ_R_BK; ++q) add(q);
+    } else {
+#pragma unroll 1
+      for (uint32_t left = some; left; left &= left - 1) add(__ffs(left) - 1);
     }
     /* renormalise each pair (Fast2Sum: |sh| >= |sl|) so that sl stays small */
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < 2; ++j) {
         const float t = __fadd_rn(sh[i][j], sl[i][j]);
         sl[i][j] = __fsub_rn(sl[i][j], __fsub_rn(t, sh[i][j]));
         sh[i][j] = t;
       }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
       const int r = ty + 8 * i, c = tx + 16 * j;
       if (small(r, c)) R.C[where(r, c)] = scalbn((double)sh[i][j] + (double)sl[i][j], s_ea[r] + s_eb[c] - 60);
     }
 }
 
-/* The listed elements, a CTA each, in FP64.  Where terms may cancel
- * (TRANS_A: dL/du has both signs) an element is given up as soon as the
- * terms' magnitudes show that it is good.  Bound by the latency of the
- * column's reads, a sector each. */
-template <bool TRANS_A>
-__global__ void __launch_bounds__(OZ_R_THREADS) k_oz_fix(OzRefine R) {
-  __shared__ double s_acc[OZ_R_THREADS / 32];
-  __shared__ float s_mag[OZ_R_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned long long todo = *R.count;
-  for (unsigned long long q = blockIdx.x; q < todo; q += gridDim.x) {
-    const size_t at = R.list[q], m = at / R.N, n = at % R.N;
-    const int ea = oz_exp(R.max_a[m]), eb = oz_exp(R.max_b[n]);
-    const float keep = OZ_KEEP * oz_norm(R.sq_a[m], R.sq_b[n]);
-    const double *a = R.A + (TRANS_A ? m : m * R.K), *b = R.B + n;
-    double acc = 0.0;
-    float mag = 0.f, all = 0.f;
-    for (int k0 = 0; k0 < R.K && !(all >= keep); k0 += 8 * OZ_R_THREADS) { /* all: the same in every thread */
-      double x[8], y[8];
+/* The listed elements in FP64, a CTA each; a warp each where there are more
+ * than OZ_F_WARPS a CTA.  Where terms may cancel (TRANS_A: dL/du has both
+ * signs) an element is given up as soon as the terms' magnitudes show that it
+ * is good.  Bound by the latency of the column's reads, a sector each, and
+ * with many elements by their number: then a warp reads B only where A is not
+ * 0 (few nodes infected is what makes many elements small). */
+#define OZ_F_WARPS 2
+template <bool TRANS_A, int THREADS>
+__device__ __forceinline__ void oz_fix_one(const OzRefine& R, size_t at, double* s_acc, float* s_mag) {
+  constexpr bool CTA = THREADS > 32;
+  const int t = threadIdx.x % THREADS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t m = at / R.N, n = at % R.N;
+  const int ea = oz_exp(R.max_a[m]), eb = oz_exp(R.max_b[n]);
+  const float keep = OZ_KEEP * oz_norm(R.sq_a[m], R.sq_b[n]);
+  const double *a = R.A + (TRANS_A ? m : m * R.K), *b = R.B + n;
+  double acc = 0.0;
+  float mag = 0.f, all = 0.f;
+  for (int k0 = 0; k0 < R.K && !(all >= keep); k0 += 8 * THREADS) { /* all: the same in every thread */
+    double x[8], y[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = k0 + u * OZ_R_THREADS + threadIdx.x;
-        x[u] = k < R.K ? a[TRANS_A ? (size_t)k * R.M : (size_t)k] : 0.0;
-        y[u] = k < R.K ? b[(size_t)k * R.N] : 0.0;
-      }
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + u * THREADS + t;
+      x[u] = k < R.K ? a[TRANS_A ? (size_t)k * R.M : (size_t)k] : 0.0;
+    }
+    unsigned some = 0xffu; /* bit u: a term of some lane */
+    if (!CTA) {
+      some = 0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = k0 + u * OZ_R_THREADS + threadIdx.x;
-        if (k >= R.K) break;
-        y[u] = oz_scaled(y[u], R.fac, k);
-        acc = __fma_rn(x[u], y[u], acc);
-        if (TRANS_A) mag += oz_scaled_abs(x[u], ea) * oz_scaled_abs(y[u], eb);
-      }
-      if (TRANS_A) {
-        float w = mag;
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        if (lane == 0) s_mag[warp] = w;
+      for (int u = 0; u < 8; ++u) some |= (unsigned)__any_sync(0xffffffffu, oz_abs_bits(x[u]) != 0) << u;
+    }
+    if (some == 0) continue;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + u * THREADS + t;
+      y[u] = (some >> u & 1u) && k < R.K ? b[(size_t)k * R.N] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + u * THREADS + t;
+      if (!(some >> u & 1u)) continue;
+      if (k < R.K) y[u] = oz_scaled(y[u], R.fac, k);
+      acc = __fma_rn(x[u], y[u], acc);
+      if (TRANS_A) mag += oz_scaled_abs(x[u], ea) * oz_scaled_abs(y[u], eb);
+    }
+    if (TRANS_A) {
+      all = mag;
+      for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+      if (CTA) {
+        if (lane == 0) s_mag[warp] = all;
         __syncthreads();
         all = (s_mag[0] + s_mag[1]) + (s_mag[2] + s_mag[3]);
         __syncthreads();
       }
     }
-    if (all >= keep) continue;
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  }
+  if (all >= keep) return;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (CTA) {
     __syncthreads();
     if (lane == 0) s_acc[warp] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) R.C[at] = (s_acc[0] + s_acc[1]) + (s_acc[2] + s_acc[3]);
+    acc = (s_acc[0] + s_acc[1]) + (s_acc[2] + s_acc[3]);
+  }
+  if (t == 0) R.C[at] = acc;
+}
+
+template <bool TRANS_A>
+__global__ void __launch_bounds__(OZ_R_THREADS) k_oz_fix(OzRefine R) {
+  __shared__ double s_acc[OZ_R_THREADS / 32];
+  __shared__ float s_mag[OZ_R_THREADS / 32];
+  constexpr int WARPS = OZ_R_THREADS / 32;
+  const unsigned long long todo = *R.count;
+  if (todo <= (unsigned long long)OZ_F_WARPS * gridDim.x) {
+    for (unsigned long long q = blockIdx.x; q < todo; q += gridDim.x)
+      oz_fix_one<TRANS_A, OZ_R_THREADS>(R, R.list[q], s_acc, s_mag);
+  } else {
+    for (unsigned long long q = (unsigned long long)blockIdx.x * WARPS + (threadIdx.x >> 5); q < todo;
+         q += (unsigned long long)gridDim.x * WARPS)
+      oz_fix_one<TRANS_A, 32>(R, R.list[q], s_acc, s_mag);
   }
 }
 
@@ -825,7 +875,7 @@ inline size_t oz_list(int M, int N) {
 template <bool TRANS_A>
 inline cudaError_t oz_refine(const OzRefine& R, int nsm, cudaStream_t st) {
   k_oz_refine<TRANS_A><<<dim3((R.N + OZ_R_BN - 1) / OZ_R_BN, (R.M + OZ_R_BM - 1) / OZ_R_BM), OZ_R_THREADS, 0, st>>>(R);
-  k_oz_fix<TRANS_A><<<16 * nsm, OZ_R_THREADS, 0, st>>>(R);
+  k_oz_fix<TRANS_A><<<8 * nsm, OZ_R_THREADS, 0, st>>>(R);
   return cudaGetLastError();
 }
 
