@@ -159,7 +159,7 @@ def sweep_b_bytes(params, t):
 
 # DRAM bytes ncu measured per unit of counted work, by kernel: (counter,
 # bytes per unit, bytes per launch besides), and where they were measured.
-NCU_TRAFFIC_PER_UNIT = {"k_select": ("sel_targets", 950.0, 0.0)}
+NCU_TRAFFIC_PER_UNIT = {"k_select": ("sel_targets", 980.0, 0.0)}
 NCU_TRAFFIC_SOURCE = {
     "k_select": "ncu DRAM read+write of k_sel_round0 + k_sel_rounds per target located, "
                 "on tick 151 of the 5e7-agent Nigeria-like case, times the targets of the timed ticks",
@@ -195,9 +195,8 @@ NCU_TRAFFIC_SOURCE = {
 #   k_node_tx: per node its population inputs (last row, births, deaths:
 #     12 B), seasonality, R0 scalar and row sum (24 B), per strain the
 #     infectivity total and incoming infectivity (16 B x 3), susceptible
-#     weight and count (12 B) read; population, per-strain probability
-#     (4 + 8 x 3 B), count, target totals (24 B) and the selection record
-#     (96 B) written: 248 B.
+#     weight and count (12 B) read; population (4 B), count, target totals
+#     (24 B) and the selection record (96 B) written: 224 B.
 SWEEP_INDEX_B, SWEEP_DUE_B, SWEEP_EVT_B, SWEEP_DOD_B, QUEUE_ENTRY_B = 4.0, 128.0, 516.0, 516.0, 8.0
 DUE_ITEM_B = 8.0
 DSQ_ENTRY_B = 8.0 + 9.0 + 8.0
@@ -206,7 +205,7 @@ SEL_TARGET_B = 12.0 + 128.0 + 128.0 + 512.0
 SEL_CLAIM_B = 15.0
 NODE_TX_CHUNK_B = 20.0
 NODE_TX_NET_B = 16.0  # a network entry in its two fixed-point parts
-NODE_TX_NODE_B = 248.0
+NODE_TX_NODE_B = 224.0
 RI_INDEX_B, RI_DUE_B = 4.0, 128.0 * 12.0 + 4.0
 
 
@@ -1002,8 +1001,9 @@ def incidence_arm(args):
     loss and gradients down).  value: K evaluations between CUDA events on
     the plan's stream.  e2e: wall time from host arrays, the plan's one-time
     upload of the aggregates and target included, over the same K
-    evaluations.  roofline: the slower product's FP32 instructions over its
-    mean launch time (profiling pass) against the nominal FP32 issue rate."""
+    evaluations.  roofline: the slower product's digit products over its
+    phase's mean time (profiling pass; the refining of small elements
+    included) against the measured bf16 rate."""
     import torch
 
     from laser_polio_gb300 import ops, synthetic
@@ -1058,7 +1058,7 @@ def incidence_arm(args):
     kernels = {name: {"launches": n, "ms_per_eval": ms / K, "share": ms / tot if tot else None}
                for name, (ms, n) in prof.items()}
     # the products run by exact slicing on the tensor cores: 43 products of bf16 digit slices
-    # (diagonals 0 to 8 of eight slices each), T S G G terms a product and launch
+    # (diagonals 0 to 8 of eight slices each), T S G G terms a product and evaluation
     terms = float(T * S * G * G)
     top = max(prof, key=lambda n: prof[n][0])
     gemm = max(("k_inc_gemm_mix", "k_inc_gemm_flows"), key=lambda n: prof[n][0])
@@ -1100,7 +1100,7 @@ def incidence_arm(args):
                  "forward runs of the engine" if replay else "synthetic (seeded numpy, replayed-aggregate shapes)"),
         "config": {"workload": f"adjoint of expected incidence, {G} nodes, {T} ticks, {S} strains",
                    "loss": "sum (log1p(lam) - log1p(target))^2",
-                   "l2": "working set (~40 MB) L2-resident by design; no flush"},
+                   "l2": "working set (~75 MB) L2-resident by design; no flush"},
         "e2e": {"value": K / (t_setup + t_eval), "unit": "evaluations/s", "setup_ms": t_setup * 1e3,
                 "ms_per_eval": t_eval / K * 1e3, "h2d_bytes_per_step": h2d_setup / K + 8 * G,
                 "d2h_bytes_per_step": 8 * (8 + G)},

@@ -844,9 +844,10 @@ extern "C" int lpg_incidence_plan_create(const lpg_incidence_in* in, const doubl
   widest(dlo, &p->max_ld2);
   widest(dhi, &p->max_ld2);
   /* the FP64 sums are one chain of G terms a thread; the sliced products take
-   * about 60 us with their operands' slicing, whatever their size (181
-   * ticks, 100 nodes, 2 strains: 71 us in three kernels against 91 in eight;
-   * 21 ticks, 333 nodes, 3 strains: 131 against about 100) */
+   * about 80 us with their operands' slicing and refining, whatever their
+   * size (an evaluation of 181 ticks, 100 nodes, 2 strains: 100 us in three
+   * kernels against 137 in twelve; 244 ticks, 128 nodes: 101 and 143; 21
+   * ticks, 333 nodes, 3 strains: 155 and 152) */
   p->small = G <= INC_SMALL_NODES && (int64_t)T * S * G * G <= INC_SMALL_TERMS;
   int rc = LPG_OK;
   int dev = 0;

@@ -4,8 +4,11 @@
  * The reference builds its agent table on the host with numpy
  * (model.py:101-175, 561-713, 816-866, 1548-1611, 1887-1894), minutes at
  * Nigeria scale.  Here:
- *   - k_init_slots fills every per-slot column in one grid-stride pass over
- *     the capacity (lpg_init.h holds the arithmetic, shared with the oracle);
+ *   - the per-slot columns are filled in grid-stride passes over the capacity
+ *     (lpg_init.h holds the arithmetic, shared with the oracle): constants and
+ *     node ids by k_init_base, dates by k_init_dates, timers and heterogeneity
+ *     by lpg_init_fast.cuh's kernels, or by k_init_slots in FP64 where the
+ *     parameters have no fast form;
  *   - the choices without replacement (chronically missed, immune and
  *     initially infected agents) take, in each group, the k agents with the
  *     smallest counter-based 64-bit keys, ties by slot.  Keys are uniform, so

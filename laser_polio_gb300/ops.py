@@ -169,7 +169,12 @@ class IncidencePlan:
     """The replayed aggregates (and an optional target curve [T, G]) kept
     resident on the current CUDA device (lpg_incidence_plan_* in
     include/lpg.h); ``evaluate`` runs the expected-incidence map and its
-    reverse pass at new parameters without re-uploading them."""
+    reverse pass at new parameters without re-uploading them.
+
+    Device memory: 64 bytes an element of beta beside the [T, G] and [G, G]
+    arrays, from 2^22 elements on 16 bytes an element and 200 MB.  The two
+    products are good to about 2^-45 of each element's own summed terms; all
+    else is FP64."""
 
     def __init__(self, inp: dict, target=None):
         desc, keep, (T, G, S) = _incidence_desc(inp, need_r0s=False)
